@@ -57,7 +57,7 @@ def build(quiet: bool = True) -> None:
     out = subprocess.DEVNULL if quiet else None
     subprocess.run(["make", "-C", HERE, "restate"], check=True, stdout=out)
     ref = reference_dir()
-    if ref and os.path.isdir(ref):
+    if ref and os.path.isfile(os.path.join(ref, "main.cpp")):
         subprocess.run(["make", "-C", HERE, "-j8", f"REF={ref}", "ref"], check=True, stdout=out)
 
 
