@@ -120,10 +120,21 @@ struct SweepArgs {
     const int32_t *__restrict__ vjob = nullptr;
     const double *__restrict__ jconst = nullptr;
     const uint8_t *__restrict__ jdone = nullptr;
+
+    // loads of the per-vertex and per-community arrays (curr, vdeg, cdeg, csize,
+    // noprune, active, frozen): no sweep launch writes what it reads, so the read-only
+    // path serves them
+    template <class T> static __device__ __forceinline__ T ld(const T *p) { return __ldg(p); }
+};
+
+// The same for a kernel that runs many sweeps: those arrays change between its
+// barriers, so the loads go to L2, past the caches that may hold older values.
+struct LiveArgs : SweepArgs {
+    template <class T> static __device__ __forceinline__ T ld(const T *p) { return __ldcg(p); }
 };
 
 // the constant of v's graph; false when v belongs to a graph whose phase has ended
-__device__ __forceinline__ bool vertex_live(const SweepArgs &a, int32_t v, double &cst) {
+template <class A> __device__ __forceinline__ bool vertex_live(const A &a, int32_t v, double &cst) {
     cst = a.constant;
     if (!a.vjob) return true;
     const int32_t j = __ldg(a.vjob + v);
@@ -155,8 +166,9 @@ __device__ __forceinline__ bool better(bool ok_a, double g_a, int32_t c_a, bool 
 // step of gain_of is monotone, a larger ay gives a larger (ay - ax), a larger second
 // term and a smaller difference. A candidate whose bound is below the best gain found
 // so far cannot win (nor tie), so its community degree is never read.
-__device__ __forceinline__ bool can_prune(const SweepArgs &a, double vd, double cst) {
-    return a.noprune && !__ldg(a.noprune) && vd >= 0.0 && isfinite(vd) && cst >= 0.0 &&
+template <class A>
+__device__ __forceinline__ bool can_prune(const A &a, double vd, double cst) {
+    return a.noprune && !A::ld(a.noprune) && vd >= 0.0 && isfinite(vd) && cst >= 0.0 &&
            isfinite(cst);
 }
 
@@ -170,8 +182,8 @@ __device__ __forceinline__ bool can_prune(const SweepArgs &a, double vd, double 
 // largest bounds are equal (integral weights give many equal counters, and every
 // tied candidate must be read anyway), every candidate, eight community-degree loads
 // at a time.
-template <int T>
-__device__ __forceinline__ void best_of_row(const SweepArgs &a, const int32_t (&c)[T],
+template <int T, class A>
+__device__ __forceinline__ void best_of_row(const A &a, const int32_t (&c)[T],
                                             uint32_t first, int32_t cc, const double *cnt,
                                             int stride, double eix, double vd, double ax,
                                             double cst, int dmax, bool &ok, double &bg,
@@ -201,7 +213,7 @@ __device__ __forceinline__ void best_of_row(const SweepArgs &a, const int32_t (&
         if (!(ub > 0.0)) return; // no candidate has a positive bound: no move
         const double u2 = e2 == -INFINITY ? -INFINITY : gain_of(e2, eix, vd, 0.0, ax, cst);
         if (u2 < ub) {
-            const double g = gain_of(e1, eix, vd, __ldg(a.cdeg + uc), ax, cst);
+            const double g = gain_of(e1, eix, vd, A::ld(a.cdeg + uc), ax, cst);
             if (g > 0.0) {
                 ok = true;
                 bg = g;
@@ -215,7 +227,7 @@ __device__ __forceinline__ void best_of_row(const SweepArgs &a, const int32_t (&
                     const double w = cnt[j * stride];
                     const double u = gain_of(w, eix, vd, 0.0, ax, cst);
                     if (u > 0.0 && (!ok || u >= bg)) {
-                        const double g2 = gain_of(w, eix, vd, __ldg(a.cdeg + c[j]), ax, cst);
+                        const double g2 = gain_of(w, eix, vd, A::ld(a.cdeg + c[j]), ax, cst);
                         if (g2 > 0.0 && better(true, g2, c[j], ok, bg, bc, a.ref)) {
                             bg = g2;
                             bc = c[j];
@@ -236,7 +248,7 @@ __device__ __forceinline__ void best_of_row(const SweepArgs &a, const int32_t (&
         for (int q = 0; q < 8; q++) {
             const int j = b + q;
             ay[q] = 0.0;
-            if (j < T && ((first >> j) & 1u) && c[j] != cc) ay[q] = __ldg(a.cdeg + c[j]);
+            if (j < T && ((first >> j) & 1u) && c[j] != cc) ay[q] = A::ld(a.cdeg + c[j]);
         }
 #pragma unroll
         for (int q = 0; q < 8; q++) {
@@ -259,7 +271,8 @@ __device__ __forceinline__ void best_of_row(const SweepArgs &a, const int32_t (&
 // only when their bound reaches the best gain; without, or when the largest bound is
 // shared by two slots, every slot, four community-degree loads per lane at a time. The
 // (gain, id) order makes the result independent of the visiting order.
-__device__ __forceinline__ void warp_best(const SweepArgs &a, const int32_t *keys,
+template <class A>
+__device__ __forceinline__ void warp_best(const A &a, const int32_t *keys,
                                           const double *vals, int64_t base, int64_t step,
                                           int64_t nk, double eix, double vd, double ax, double cst,
                                           bool &ok, double &gain, int32_t &cand) {
@@ -299,7 +312,7 @@ __device__ __forceinline__ void warp_best(const SweepArgs &a, const int32_t *key
                 goto full_scan;
             }
             double g = 0.0;
-            if (lane == wl) g = gain_of(uw, eix, vd, __ldg(a.cdeg + uc), ax, cst);
+            if (lane == wl) g = gain_of(uw, eix, vd, A::ld(a.cdeg + uc), ax, cst);
             g = __shfl_sync(full, g, wl);
             const int32_t c0 = __shfl_sync(full, uc, wl);
             if (g > 0.0) {
@@ -314,7 +327,7 @@ __device__ __forceinline__ void warp_best(const SweepArgs &a, const int32_t *key
                     const double w = vals[i];
                     const double u = gain_of(w, eix, vd, 0.0, ax, cst);
                     if (u > 0.0 && (!ok || u >= gain)) {
-                        const double gg = gain_of(w, eix, vd, __ldg(a.cdeg + k), ax, cst);
+                        const double gg = gain_of(w, eix, vd, A::ld(a.cdeg + k), ax, cst);
                         if (gg > 0.0 && better(true, gg, k, ok, gain, cand, a.ref)) {
                             gain = gg;
                             cand = k;
@@ -341,7 +354,7 @@ full_scan:
                 kq[j] = i < nk ? keys[i] : EMPTY;
             }
 #pragma unroll
-            for (int j = 0; j < 4; j++) aq[j] = kq[j] != EMPTY ? __ldg(a.cdeg + kq[j]) : 0.0;
+            for (int j = 0; j < 4; j++) aq[j] = kq[j] != EMPTY ? A::ld(a.cdeg + kq[j]) : 0.0;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 if (kq[j] == EMPTY) continue;
@@ -369,23 +382,26 @@ full_scan:
 
 // the community sizes the singleton rule (louvain.cpp:2275-2276) reads: needed only
 // when the chosen community's id is larger than the current one's
-__device__ __forceinline__ void sizes_for_rule(const SweepArgs &a, bool ok, int32_t cand, int32_t cc,
+template <class A>
+__device__ __forceinline__ void sizes_for_rule(const A &a, bool ok, int32_t cand, int32_t cc,
                                                int32_t &ccSize, int32_t &csz) {
     ccSize = 0;
     csz = 0;
     if (ok && vg_rid(a.ref, cand) > vg_rid(a.ref, cc)) {
-        ccSize = __ldg(a.csize + cc);
-        csz = __ldg(a.csize + cand);
+        ccSize = A::ld(a.csize + cc);
+        csz = A::ld(a.csize + cand);
     }
 }
 
 // decision + bookkeeping shared by all kernels (louvain.cpp:2275-2416)
-__device__ __forceinline__ void load_comm(const SweepArgs &a, int32_t c, double &deg, int32_t &size) {
-    deg = __ldg(a.cdeg + c);
-    size = __ldg(a.csize + c);
+template <class A>
+__device__ __forceinline__ void load_comm(const A &a, int32_t c, double &deg, int32_t &size) {
+    deg = A::ld(a.cdeg + c);
+    size = A::ld(a.csize + c);
 }
 
-__device__ __forceinline__ void commit_vertex(const SweepArgs &a, int32_t v, int32_t cc,
+template <class A>
+__device__ __forceinline__ void commit_vertex(const A &a, int32_t v, int32_t cc,
                                               int32_t ccSize, double vd, bool has_edges,
                                               double counter0, bool ok, int32_t cand, int32_t csz) {
     int32_t tgt = cc;
@@ -436,6 +452,90 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // accumulated in an interleaved shared-memory slot of the community's first
 // occurrence. Candidate degrees are gathered eight at a time.
 
+// vertex v (row a.rowptr[v] = e0, degree d <= T) by one thread; slots: the thread's T
+// shared-memory doubles, NT apart
+template <int T, int NT, class A>
+__device__ __forceinline__ void thread_vertex(const A &a, int32_t v, int64_t e0, int d, double cst,
+                                              double *slots) {
+    if (a.active && !A::ld(a.active + v)) {
+        a.cw[v] = A::ld(a.frozen + v);
+        return;
+    }
+    const int32_t cc = A::ld(a.curr + v);
+    const double vd = A::ld(a.vdeg + v);
+    const double ccDeg = A::ld(a.cdeg + cc);
+    // the 32-slot kernel's loops end at the largest degree among the lanes here (at
+    // least each lane's own): they take the same vertex class in position order
+    const int dmax = T > 16 ? (int)__reduce_max_sync(__activemask(), (unsigned)d) : T;
+    int32_t c[T];
+    uint32_t selfm = 0; // bit j: edge j is a self loop
+    {
+        // weights go straight to the thread's shared-memory slots (asynchronous
+        // copies); tails are loaded up front, then their communities gathered
+        int32_t t[T];
+#pragma unroll
+        for (int j = 0; j < T; j++) {
+            if (j >= dmax) break;
+            t[j] = -1;
+            if (j < d) {
+                t[j] = __ldcs(a.tail + e0 + j);
+                cp_async8(slots + j * NT, a.weight + e0 + j);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < T; j++) {
+            if (j >= dmax) break;
+            c[j] = -1;
+            if (j < d) {
+                c[j] = A::ld(a.curr + t[j]);
+                if (t[j] == v) selfm |= 1u << j;
+            }
+        }
+    }
+    cp_async_wait_all();
+    double selfLoop = 0.0;
+    if (selfm) {
+#pragma unroll
+        for (int j = 0; j < T; j++) {
+            if (j >= dmax) break;
+            if ((selfm >> j) & 1u) selfLoop = __dadd_rn(selfLoop, slots[j * NT]);
+        }
+    }
+    // counters fold in place at the slot of each community's first occurrence,
+    // in CSR order (slot j still holds w_j when edge j is folded: only first
+    // occurrences receive additions)
+    uint32_t first = 0; // bit j: edge j is the first occurrence of its community
+    int j0 = -1;        // first occurrence of the current community
+#pragma unroll
+    for (int j = 0; j < T; j++) {
+        if (j >= dmax) break;
+        if (j < d) {
+            int fj = j;
+#pragma unroll
+            for (int k = j - 1; k >= 0; k--)
+                if (c[k] == c[j]) fj = k;
+            if (fj == j) {
+                first |= 1u << j;
+                if (c[j] == cc) j0 = j;
+            } else {
+                slots[fj * NT] = __dadd_rn(slots[fj * NT], slots[j * NT]);
+            }
+        }
+    }
+    const double counter0 = j0 >= 0 ? slots[j0 * NT] : 0.0;
+    const double eix = __dsub_rn(counter0, selfLoop);
+    const double ax = __dsub_rn(ccDeg, vd);
+    double bg;
+    int32_t bc;
+    bool ok;
+    best_of_row<T>(a, c, first, cc, slots, NT, eix, vd, ax, cst, dmax, ok, bg, bc);
+    // the singleton rule (louvain.cpp:2275-2276) needs the sizes only when
+    // the winner's id is larger than the current community's
+    int32_t ccSize, bs;
+    sizes_for_rule(a, ok, bc, cc, ccSize, bs);
+    commit_vertex(a, v, cc, ccSize, vd, d > 0, counter0, ok, bc, bs);
+}
+
 template <bool LIST, int T, int NT>
 __global__ void __launch_bounds__(NT, (T <= 16 ? VG_T16_MINB : VG_T32_MINB)) k_sweep_thread(
     SweepArgs a, const int32_t *__restrict__ list, int64_t count) {
@@ -448,86 +548,7 @@ __global__ void __launch_bounds__(NT, (T <= 16 ? VG_T16_MINB : VG_T32_MINB)) k_s
         if (!LIST && d > T) continue; // the list kernels take the larger degrees
         double cst;
         if (!vertex_live(a, v, cst)) continue;
-        if (a.active && !a.active[v]) {
-            a.cw[v] = a.frozen[v];
-            continue;
-        }
-        const int32_t cc = __ldg(a.curr + v);
-        const double vd = a.vdeg[v];
-        const double ccDeg = __ldg(a.cdeg + cc);
-        // the 32-slot kernel's loops end at the largest degree among the lanes here (at
-        // least each lane's own): they take the same vertex class in position order
-        const int dmax = T > 16 ? (int)__reduce_max_sync(__activemask(), (unsigned)d) : T;
-        int32_t c[T];
-        uint32_t selfm = 0; // bit j: edge j is a self loop
-        {
-            // weights go straight to the thread's shared-memory slots (asynchronous
-            // copies); tails are loaded up front, then their communities gathered
-            int32_t t[T];
-#pragma unroll
-            for (int j = 0; j < T; j++) {
-                if (j >= dmax) break;
-                t[j] = -1;
-                if (j < d) {
-                    t[j] = __ldcs(a.tail + e0 + j);
-                    cp_async8(&ssum[j][tid], a.weight + e0 + j);
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < T; j++) {
-                if (j >= dmax) break;
-                c[j] = -1;
-                if (j < d) {
-                    c[j] = __ldg(a.curr + t[j]);
-                    if (t[j] == v) selfm |= 1u << j;
-                }
-            }
-        }
-        cp_async_wait_all();
-        double selfLoop = 0.0;
-        if (selfm) {
-#pragma unroll
-            for (int j = 0; j < T; j++) {
-                if (j >= dmax) break;
-                if ((selfm >> j) & 1u) selfLoop = __dadd_rn(selfLoop, ssum[j][tid]);
-            }
-        }
-        // counters fold in place at the slot of each community's first occurrence,
-        // in CSR order (slot j still holds w_j when edge j is folded: only first
-        // occurrences receive additions)
-        uint32_t first = 0; // bit j: edge j is the first occurrence of its community
-        int j0 = -1;        // first occurrence of the current community
-#pragma unroll
-        for (int j = 0; j < T; j++) {
-            if (j >= dmax) break;
-            if (j < d) {
-                int fj = j;
-#pragma unroll
-                for (int k = j - 1; k >= 0; k--)
-                    if (c[k] == c[j]) fj = k;
-                if (fj == j) {
-                    first |= 1u << j;
-                    if (c[j] == cc) j0 = j;
-                } else {
-                    ssum[fj][tid] = __dadd_rn(ssum[fj][tid], ssum[j][tid]);
-                }
-            }
-        }
-        const double counter0 = j0 >= 0 ? ssum[j0][tid] : 0.0;
-        const double eix = __dsub_rn(counter0, selfLoop);
-        const double ax = __dsub_rn(ccDeg, vd);
-        double bg;
-        int32_t bc;
-        bool ok;
-        best_of_row<T>(a, c, first, cc, &ssum[0][tid], NT, eix, vd, ax, cst, dmax, ok, bg, bc);
-        // the singleton rule (louvain.cpp:2275-2276) needs the sizes only when
-        // the winner's id is larger than the current community's
-        int32_t ccSize = 0, bs = 0;
-        if (ok && vg_rid(a.ref, bc) > vg_rid(a.ref, cc)) {
-            ccSize = __ldg(a.csize + cc);
-            bs = __ldg(a.csize + bc);
-        }
-        commit_vertex(a, v, cc, ccSize, vd, d > 0, counter0, ok, bc, bs);
+        thread_vertex<T, NT>(a, v, e0, d, cst, &ssum[0][tid]);
     }
 }
 
@@ -710,11 +731,132 @@ template <int CAP, int WARPS> constexpr size_t warp_smem_bytes() {
     return (size_t)WARPS * CAP * (sizeof(double) + sizeof(int32_t)) + (size_t)WARPS * 32 * sizeof(double);
 }
 
+// vertex v by one warp; keys/vals: a table of at least twice its degree (rounded up to
+// a power of two), stage: 32 doubles, all the warp's own
+template <class A>
+__device__ __forceinline__ void warp_vertex(const A &a, int32_t v, double cst, int32_t *keys,
+                                            double *vals, double *stage) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int32_t cc = A::ld(a.curr + v);
+    if (a.active && !A::ld(a.active + v)) {
+        if (lane == 0) a.cw[v] = A::ld(a.frozen + v);
+        return;
+    }
+    const int64_t e0 = a.rowptr[v];
+    const int d = (int)(a.rowptr[v + 1] - e0);
+    int logcap = 5;
+    while ((1 << logcap) < 2 * d) logcap++;
+    const int cap = 1 << logcap;
+    for (int s = lane; s < cap; s += 32) keys[s] = EMPTY;
+    __syncwarp();
+    double selfLoop = 0.0;
+    // groups of four 32-edge chunks: the group's tails and weights are loaded
+    // together, then their communities, so a group costs two round trips
+    for (int g0 = 0; g0 < d; g0 += 4 * 32) {
+        int32_t tt[4], cg[4];
+        double ww[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int k = g0 + j * 32 + lane;
+            tt[j] = k < d ? a.tail[e0 + k] : -1;
+            ww[j] = k < d ? a.weight[e0 + k] : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) cg[j] = tt[j] >= 0 ? A::ld(a.curr + tt[j]) : -1;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (g0 + j * 32 >= d) break; // warp-uniform
+            const bool has = tt[j] >= 0;
+            const int32_t t = tt[j], c = cg[j];
+            stage[lane] = ww[j];
+            const unsigned peers = __match_any_sync(full, has ? c : (-1 - lane));
+            __syncwarp();
+            if (has && lane == __ffs(peers) - 1) {
+                uint32_t h = slot_hash(c, logcap);
+                bool fresh = false;
+                for (;;) {
+                    const int32_t kk = keys[h];
+                    if (kk == c) break;
+                    if (kk == EMPTY) {
+                        const int32_t old = atomicCAS(&keys[h], EMPTY, c);
+                        if (old == EMPTY) {
+                            fresh = true;
+                            break;
+                        }
+                        if (old == c) break;
+                    }
+                    h = (h + 1) & (cap - 1);
+                }
+                const unsigned above = peers & ~((2u << lane) - 1u);
+                double acc = fresh ? stage[lane] : __dadd_rn(vals[h], stage[lane]);
+                if (above) acc = vg_fold_above(acc, stage, above);
+                vals[h] = acc;
+            }
+            const unsigned selfm = __ballot_sync(full, has && t == v);
+            {
+                unsigned m = selfm;
+                while (m) {
+                    const int b = __ffs(m) - 1;
+                    selfLoop = __dadd_rn(selfLoop, stage[b]);
+                    m &= m - 1;
+                }
+            }
+            __syncwarp();
+        }
+    }
+    // counter[0]: the current community's entry, if any neighbour is in it
+    double counter0 = 0.0;
+    {
+        uint32_t h = slot_hash(cc, logcap);
+        for (int probe = 0; probe < cap; probe++) {
+            const int32_t kk = keys[h];
+            if (kk == cc) {
+                counter0 = vals[h];
+                break;
+            }
+            if (kk == EMPTY) break;
+            h = (h + 1) & (cap - 1);
+        }
+    }
+    // the other communities, compacted to the front of the table: a kept slot
+    // moves to the count of kept slots before it, never past a slot not yet read
+    int nk = 0;
+    for (int base = 0; base < cap; base += 32) {
+        const int32_t kk = keys[base + lane];
+        const double vv = vals[base + lane];
+        const bool keep = kk != EMPTY && kk != cc;
+        const unsigned bm = __ballot_sync(full, keep);
+        __syncwarp();
+        if (keep) {
+            const int dst = nk + __popc(bm & ((1u << lane) - 1u));
+            keys[dst] = kk;
+            vals[dst] = vv;
+        }
+        nk += __popc(bm);
+        __syncwarp();
+    }
+    const double vd = A::ld(a.vdeg + v);
+    const double ccDeg = A::ld(a.cdeg + cc);
+    const double eix = __dsub_rn(counter0, selfLoop);
+    const double ax = __dsub_rn(ccDeg, vd);
+    double gain;
+    int32_t cand;
+    bool ok;
+    warp_best(a, keys, vals, 0, 32, nk, eix, vd, ax, cst, ok, gain, cand);
+    if (lane == 0) {
+        int32_t ccSize, csz;
+        sizes_for_rule(a, ok, cand, cc, ccSize, csz);
+        commit_vertex(a, v, cc, ccSize, vd, d > 0, counter0, ok, cand, csz);
+    }
+    __syncwarp();
+}
+
 template <int CAP, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, CAP <= 256 ? 4 : 1) k_sweep_warp(
     SweepArgs a, const int32_t *__restrict__ list, int64_t count) {
     extern __shared__ unsigned char smem_raw[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
     double *vals = reinterpret_cast<double *>(smem_raw) + (size_t)warp * CAP;
     int32_t *keys = reinterpret_cast<int32_t *>(reinterpret_cast<double *>(smem_raw) +
                                                 (size_t)WARPS * CAP) +
@@ -723,125 +865,13 @@ __global__ void __launch_bounds__(WARPS * 32, CAP <= 256 ? 4 : 1) k_sweep_warp(
                         reinterpret_cast<double *>(smem_raw) + (size_t)WARPS * CAP) +
                                                (size_t)WARPS * CAP) +
                     (size_t)warp * 32;
-    const unsigned full = 0xffffffffu;
     const int64_t wg = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t idx = wg; idx < count; idx += nw) {
         const int32_t v = list[idx];
         double cst;
         if (!vertex_live(a, v, cst)) continue;
-        const int32_t cc = a.curr[v];
-        if (a.active && !a.active[v]) {
-            if (lane == 0) a.cw[v] = a.frozen[v];
-            continue;
-        }
-        const int64_t e0 = a.rowptr[v];
-        const int d = (int)(a.rowptr[v + 1] - e0);
-        int logcap = 5;
-        while ((1 << logcap) < 2 * d) logcap++;
-        const int cap = 1 << logcap;
-        for (int s = lane; s < cap; s += 32) keys[s] = EMPTY;
-        __syncwarp();
-        double selfLoop = 0.0;
-        // groups of four 32-edge chunks: the group's tails and weights are loaded
-        // together, then their communities, so a group costs two round trips
-        for (int g0 = 0; g0 < d; g0 += 4 * 32) {
-            int32_t tt[4], cg[4];
-            double ww[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int k = g0 + j * 32 + lane;
-                tt[j] = k < d ? a.tail[e0 + k] : -1;
-                ww[j] = k < d ? a.weight[e0 + k] : 0.0;
-            }
-#pragma unroll
-            for (int j = 0; j < 4; j++) cg[j] = tt[j] >= 0 ? a.curr[tt[j]] : -1;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                if (g0 + j * 32 >= d) break; // warp-uniform
-                const bool has = tt[j] >= 0;
-                const int32_t t = tt[j], c = cg[j];
-                stage[lane] = ww[j];
-                const unsigned peers = __match_any_sync(full, has ? c : (-1 - lane));
-                __syncwarp();
-                if (has && lane == __ffs(peers) - 1) {
-                    uint32_t h = slot_hash(c, logcap);
-                    bool fresh = false;
-                    for (;;) {
-                        const int32_t kk = keys[h];
-                        if (kk == c) break;
-                        if (kk == EMPTY) {
-                            const int32_t old = atomicCAS(&keys[h], EMPTY, c);
-                            if (old == EMPTY) {
-                                fresh = true;
-                                break;
-                            }
-                            if (old == c) break;
-                        }
-                        h = (h + 1) & (cap - 1);
-                    }
-                    const unsigned above = peers & ~((2u << lane) - 1u);
-                    double acc = fresh ? stage[lane] : __dadd_rn(vals[h], stage[lane]);
-                    if (above) acc = vg_fold_above(acc, stage, above);
-                    vals[h] = acc;
-                }
-                const unsigned selfm = __ballot_sync(full, has && t == v);
-                {
-                    unsigned m = selfm;
-                    while (m) {
-                        const int b = __ffs(m) - 1;
-                        selfLoop = __dadd_rn(selfLoop, stage[b]);
-                        m &= m - 1;
-                    }
-                }
-                __syncwarp();
-            }
-        }
-        // counter[0]: the current community's entry, if any neighbour is in it
-        double counter0 = 0.0;
-        {
-            uint32_t h = slot_hash(cc, logcap);
-            for (int probe = 0; probe < cap; probe++) {
-                const int32_t kk = keys[h];
-                if (kk == cc) {
-                    counter0 = vals[h];
-                    break;
-                }
-                if (kk == EMPTY) break;
-                h = (h + 1) & (cap - 1);
-            }
-        }
-        // the other communities, compacted to the front of the table: a kept slot
-        // moves to the count of kept slots before it, never past a slot not yet read
-        int nk = 0;
-        for (int base = 0; base < cap; base += 32) {
-            const int32_t kk = keys[base + lane];
-            const double vv = vals[base + lane];
-            const bool keep = kk != EMPTY && kk != cc;
-            const unsigned bm = __ballot_sync(full, keep);
-            __syncwarp();
-            if (keep) {
-                const int dst = nk + __popc(bm & ((1u << lane) - 1u));
-                keys[dst] = kk;
-                vals[dst] = vv;
-            }
-            nk += __popc(bm);
-            __syncwarp();
-        }
-        const double vd = a.vdeg[v];
-        const double ccDeg = __ldg(a.cdeg + cc);
-        const double eix = __dsub_rn(counter0, selfLoop);
-        const double ax = __dsub_rn(ccDeg, vd);
-        double gain;
-        int32_t cand;
-        bool ok;
-        warp_best(a, keys, vals, 0, 32, nk, eix, vd, ax, cst, ok, gain, cand);
-        if (lane == 0) {
-            int32_t ccSize, csz;
-            sizes_for_rule(a, ok, cand, cc, ccSize, csz);
-            commit_vertex(a, v, cc, ccSize, vd, d > 0, counter0, ok, cand, csz);
-        }
-        __syncwarp();
+        warp_vertex(a, v, cst, keys, vals, stage);
     }
 }
 
@@ -851,13 +881,156 @@ __global__ void __launch_bounds__(WARPS * 32, CAP <= 256 ? 4 : 1) k_sweep_warp(
 // meet in the table through atomics (table in shared memory, or in a global
 // scratch region per CTA for the largest degrees).
 
-struct CtaShared {
-    double red_g[CT_THREADS / 32];
-    int32_t red_c[CT_THREADS / 32];
-    int red_ok[CT_THREADS / 32];
-    double self_part[CT_THREADS / 32];
+template <int NT> struct CtaShared {
+    double red_g[NT / 32];
+    int32_t red_c[NT / 32];
+    int red_ok[NT / 32];
+    double self_part[NT / 32];
     double counter0;
 };
+
+// vertex v (row a.rowptr[v] = e0, degree d) by the whole block of NT threads; keys/vals:
+// a shared table of at least twice `slots`, the most communities its row can hold
+// (rounded up to a power of two), stage: NT doubles
+template <int NT, class A>
+__device__ __forceinline__ void cta_vertex(const A &a, int32_t v, int64_t e0, int64_t d,
+                                           int64_t slots, double cst, int32_t *keys, double *vals,
+                                           double *stage, CtaShared<NT> &sh) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu;
+    const int32_t cc = A::ld(a.curr + v);
+    if (a.active && !A::ld(a.active + v)) {
+        if (threadIdx.x == 0) a.cw[v] = A::ld(a.frozen + v);
+        return;
+    }
+    int logcap = 5;
+    while (((int64_t)1 << logcap) < 2 * slots) logcap++;
+    const int64_t cap = (int64_t)1 << logcap;
+    for (int64_t s = threadIdx.x; s < cap; s += NT) {
+        keys[s] = EMPTY;
+        vals[s] = 0.0;
+    }
+    double selfLoop = 0.0; // per-warp partial, in CSR order inside the warp's slices
+    __syncthreads();
+    for (int64_t off = 0; off < d; off += NT) {
+        const int64_t k = off + threadIdx.x;
+        const bool has = k < d;
+        int32_t t = -1, c = -1;
+        double w = 0.0;
+        if (has) {
+            t = a.tail[e0 + k];
+            w = a.weight[e0 + k];
+            c = A::ld(a.curr + t);
+        }
+        stage[threadIdx.x] = w;
+        const unsigned peers = __match_any_sync(full, has ? c : (-1 - lane));
+        __syncwarp();
+        if (has && lane == __ffs(peers) - 1) {
+            double acc = stage[threadIdx.x];
+            const unsigned above = peers & ~((2u << lane) - 1u);
+            if (above) acc = vg_fold_above(acc, stage + (threadIdx.x & ~31), above);
+            uint32_t h = slot_hash(c, logcap);
+            for (;;) {
+                const int32_t kk = keys[h];
+                if (kk == c) break;
+                if (kk == EMPTY) {
+                    const int32_t old = atomicCAS(&keys[h], EMPTY, c);
+                    if (old == EMPTY || old == c) break;
+                }
+                h = (h + 1) & (uint32_t)(cap - 1);
+            }
+            atomicAdd(&vals[h], acc);
+        }
+        const unsigned selfm = __ballot_sync(full, has && t == v);
+        {
+            unsigned m = selfm;
+            while (m) {
+                const int b = __ffs(m) - 1;
+                selfLoop = __dadd_rn(selfLoop, stage[(threadIdx.x & ~31) + b]);
+                m &= m - 1;
+            }
+        }
+        __syncwarp();
+    }
+    if (lane == 0) sh.self_part[warp] = selfLoop;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int w = 0; w < NT / 32; w++) s = __dadd_rn(s, sh.self_part[w]);
+        sh.self_part[0] = s;
+        double c0 = 0.0;
+        uint32_t h = slot_hash(cc, logcap);
+        for (int64_t probe = 0; probe < cap; probe++) {
+            const int32_t kk = keys[h];
+            if (kk == cc) {
+                c0 = vals[h];
+                break;
+            }
+            if (kk == EMPTY) break;
+            h = (h + 1) & (uint32_t)(cap - 1);
+        }
+        sh.counter0 = c0;
+    }
+    __syncthreads();
+    const double counter0 = sh.counter0;
+    selfLoop = sh.self_part[0];
+    const double vd = A::ld(a.vdeg + v);
+    const double ccDeg = A::ld(a.cdeg + cc);
+    const double eix = __dsub_rn(counter0, selfLoop);
+    const double ax = __dsub_rn(ccDeg, vd);
+    double gain;
+    int32_t cand;
+    bool ok;
+    // the other communities, compacted to the front of the table in slot order:
+    // a kept slot moves to the count of kept slots before it, so no write lands
+    // on a slot not yet read (each group's reads end at the barrier before its
+    // writes)
+    int64_t nk = 0;
+    for (int64_t base = 0; base < cap; base += NT) {
+        const int64_t s = base + threadIdx.x;
+        const int32_t kk = s < cap ? keys[s] : EMPTY;
+        const double vv = s < cap ? vals[s] : 0.0;
+        const bool keep = kk != EMPTY && kk != cc;
+        const unsigned bm = __ballot_sync(full, keep);
+        if (lane == 0) sh.red_c[warp] = __popc(bm);
+        __syncthreads();
+        int before = 0, tot = 0;
+#pragma unroll
+        for (int w = 0; w < NT / 32; w++) {
+            const int c = sh.red_c[w];
+            before += w < warp ? c : 0;
+            tot += c;
+        }
+        if (keep) {
+            const int64_t dst = nk + before + __popc(bm & ((1u << lane) - 1u));
+            keys[dst] = kk;
+            vals[dst] = vv;
+        }
+        nk += tot;
+        __syncthreads();
+    }
+    // each warp its own slots (warp * 32 + lane + k * NT), then the warps' bests
+    warp_best(a, keys, vals, warp * 32, NT, nk, eix, vd, ax, cst, ok, gain, cand);
+    if (lane == 0) {
+        sh.red_g[warp] = gain;
+        sh.red_c[warp] = cand;
+        sh.red_ok[warp] = ok;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < NT / 32; w++) {
+            if (better(sh.red_ok[w] != 0, sh.red_g[w], sh.red_c[w], ok, gain, cand, a.ref)) {
+                gain = sh.red_g[w];
+                cand = sh.red_c[w];
+                ok = true;
+            }
+        }
+        int32_t ccSize, csz;
+        sizes_for_rule(a, ok, cand, cc, ccSize, csz);
+        commit_vertex(a, v, cc, ccSize, vd, d > 0, counter0, ok, cand, csz);
+    }
+    __syncthreads();
+}
 
 // CAP: the table's slots. The class runs as two launches over the same list, a
 // table of CT_CAP_S slots for the rows of at most CT_CAP_S / 2 entries (more CTAs fit
@@ -866,10 +1039,8 @@ template <int CAP>
 __global__ void __launch_bounds__(CT_THREADS) k_sweep_cta(SweepArgs a, const int32_t *__restrict__ list,
                                                           int64_t count) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ CtaShared sh;
+    __shared__ CtaShared<CT_THREADS> sh;
     __shared__ __align__(16) double stage[CT_THREADS];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned full = 0xffffffffu;
     double *vals = reinterpret_cast<double *>(smem_raw);
     int32_t *keys = reinterpret_cast<int32_t *>(vals + CAP);
     for (int64_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
@@ -879,138 +1050,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_sweep_cta(SweepArgs a, const int
         if ((CAP == CT_CAP) != (d > CT_CAP_S / 2)) continue; // the other launch's row
         double cst;
         if (!vertex_live(a, v, cst)) continue;
-        const int32_t cc = a.curr[v];
-        if (a.active && !a.active[v]) {
-            if (threadIdx.x == 0) a.cw[v] = a.frozen[v];
-            continue;
-        }
-        int logcap = 5;
-        while (((int64_t)1 << logcap) < 2 * d) logcap++;
-        const int64_t cap = (int64_t)1 << logcap;
-        for (int64_t s = threadIdx.x; s < cap; s += CT_THREADS) {
-            keys[s] = EMPTY;
-            vals[s] = 0.0;
-        }
-        double selfLoop = 0.0; // per-warp partial, in CSR order inside the warp's slices
-        __syncthreads();
-        for (int64_t off = 0; off < d; off += CT_THREADS) {
-            const int64_t k = off + threadIdx.x;
-            const bool has = k < d;
-            int32_t t = -1, c = -1;
-            double w = 0.0;
-            if (has) {
-                t = a.tail[e0 + k];
-                w = a.weight[e0 + k];
-                c = a.curr[t];
-            }
-            stage[threadIdx.x] = w;
-            const unsigned peers = __match_any_sync(full, has ? c : (-1 - lane));
-            __syncwarp();
-            if (has && lane == __ffs(peers) - 1) {
-                double acc = stage[threadIdx.x];
-                const unsigned above = peers & ~((2u << lane) - 1u);
-                if (above) acc = vg_fold_above(acc, stage + (threadIdx.x & ~31), above);
-                uint32_t h = slot_hash(c, logcap);
-                for (;;) {
-                    const int32_t kk = keys[h];
-                    if (kk == c) break;
-                    if (kk == EMPTY) {
-                        const int32_t old = atomicCAS(&keys[h], EMPTY, c);
-                        if (old == EMPTY || old == c) break;
-                    }
-                    h = (h + 1) & (uint32_t)(cap - 1);
-                }
-                atomicAdd(&vals[h], acc);
-            }
-            const unsigned selfm = __ballot_sync(full, has && t == v);
-            {
-                unsigned m = selfm;
-                while (m) {
-                    const int b = __ffs(m) - 1;
-                    selfLoop = __dadd_rn(selfLoop, stage[(threadIdx.x & ~31) + b]);
-                    m &= m - 1;
-                }
-            }
-            __syncwarp();
-        }
-        if (lane == 0) sh.self_part[warp] = selfLoop;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double s = 0.0;
-            for (int w = 0; w < CT_THREADS / 32; w++) s = __dadd_rn(s, sh.self_part[w]);
-            sh.self_part[0] = s;
-            double c0 = 0.0;
-            uint32_t h = slot_hash(cc, logcap);
-            for (int64_t probe = 0; probe < cap; probe++) {
-                const int32_t kk = keys[h];
-                if (kk == cc) {
-                    c0 = vals[h];
-                    break;
-                }
-                if (kk == EMPTY) break;
-                h = (h + 1) & (uint32_t)(cap - 1);
-            }
-            sh.counter0 = c0;
-        }
-        __syncthreads();
-        const double counter0 = sh.counter0;
-        selfLoop = sh.self_part[0];
-        const double vd = a.vdeg[v];
-        const double ccDeg = __ldg(a.cdeg + cc);
-        const double eix = __dsub_rn(counter0, selfLoop);
-        const double ax = __dsub_rn(ccDeg, vd);
-        double gain;
-        int32_t cand;
-        bool ok;
-        // the other communities, compacted to the front of the table in slot order:
-        // a kept slot moves to the count of kept slots before it, so no write lands
-        // on a slot not yet read (each group's reads end at the barrier before its
-        // writes)
-        int64_t nk = 0;
-        for (int64_t base = 0; base < cap; base += CT_THREADS) {
-            const int64_t s = base + threadIdx.x;
-            const int32_t kk = s < cap ? keys[s] : EMPTY;
-            const double vv = s < cap ? vals[s] : 0.0;
-            const bool keep = kk != EMPTY && kk != cc;
-            const unsigned bm = __ballot_sync(full, keep);
-            if (lane == 0) sh.red_c[warp] = __popc(bm);
-            __syncthreads();
-            int before = 0, tot = 0;
-#pragma unroll
-            for (int w = 0; w < CT_THREADS / 32; w++) {
-                const int c = sh.red_c[w];
-                before += w < warp ? c : 0;
-                tot += c;
-            }
-            if (keep) {
-                const int64_t dst = nk + before + __popc(bm & ((1u << lane) - 1u));
-                keys[dst] = kk;
-                vals[dst] = vv;
-            }
-            nk += tot;
-            __syncthreads();
-        }
-        // each warp its own slots (warp * 32 + lane + k * CT_THREADS), then the warps' bests
-        warp_best(a, keys, vals, warp * 32, CT_THREADS, nk, eix, vd, ax, cst, ok, gain, cand);
-        if (lane == 0) {
-            sh.red_g[warp] = gain;
-            sh.red_c[warp] = cand;
-            sh.red_ok[warp] = ok;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < CT_THREADS / 32; w++) {
-                if (better(sh.red_ok[w] != 0, sh.red_g[w], sh.red_c[w], ok, gain, cand, a.ref)) {
-                    gain = sh.red_g[w];
-                    cand = sh.red_c[w];
-                    ok = true;
-                }
-            }
-            int32_t ccSize, csz;
-            sizes_for_rule(a, ok, cand, cc, ccSize, csz);
-            commit_vertex(a, v, cc, ccSize, vd, d > 0, counter0, ok, cand, csz);
-        }
-        __syncthreads();
+        cta_vertex<CT_THREADS>(a, v, e0, d, d, cst, keys, vals, stage, sh);
     }
 }
 
@@ -1738,47 +1778,56 @@ double twice_m_one(vg_ctx *ctx, const double *vdeg, int64_t nv) {
 
 // early termination -t 1/3 (louvain.cpp:172-184): C++'s chained
 // `target == curr == past` compares the bool (target == curr) with past
-__global__ void k_swap_et13(int64_t nv, int numIters, int32_t *__restrict__ past,
-                            int32_t *__restrict__ curr, int32_t *__restrict__ target,
-                            uint8_t *__restrict__ active, const int32_t *__restrict__ ref) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nv;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t p = past[i], c = curr[i], t = target[i];
-        if (numIters > 2 && ((int32_t)(t == c) == vg_rid(ref, p))) {
-            active[i] = 0;
-        } else {
-            past[i] = c;
-            curr[i] = t;
-            target[i] = p;
-        }
+__device__ __forceinline__ void swap_et13(int64_t i, int numIters, int32_t *past, int32_t *curr,
+                                          int32_t *target, uint8_t *active,
+                                          const int32_t *__restrict__ ref) {
+    const int32_t p = past[i], c = curr[i], t = target[i];
+    if (numIters > 2 && ((int32_t)(t == c) == vg_rid(ref, p))) {
+        active[i] = 0;
+    } else {
+        past[i] = c;
+        curr[i] = t;
+        target[i] = p;
     }
 }
 
 // early termination -t 2/4 (louvain.cpp:381-400)
+__device__ __forceinline__ void swap_et24(int64_t i, int numIters, double one_minus_delta,
+                                          int32_t *past, int32_t *curr, int32_t *target,
+                                          uint8_t *active, double *pcurr, const double *pprev) {
+    if (!active[i]) return;
+    const int32_t p = past[i], c = curr[i];
+    if (numIters > 2 && c == p) {
+        const double pc = __dmul_rn(pprev[i], one_minus_delta);
+        pcurr[i] = pc;
+        if (pc <= 0.02) { // P_CUTOFF (louvain.hpp:74)
+            active[i] = 0;
+            return;
+        }
+    }
+    past[i] = c;
+    curr[i] = target[i];
+    target[i] = p;
+}
+
+__global__ void k_swap_et13(int64_t nv, int numIters, int32_t *__restrict__ past,
+                            int32_t *__restrict__ curr, int32_t *__restrict__ target,
+                            uint8_t *__restrict__ active, const int32_t *__restrict__ ref) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nv;
+         i += (int64_t)gridDim.x * blockDim.x)
+        swap_et13(i, numIters, past, curr, target, active, ref);
+}
+
 __global__ void k_swap_et24(int64_t nv, int numIters, double one_minus_delta,
                             int32_t *__restrict__ past, int32_t *__restrict__ curr,
                             int32_t *__restrict__ target, uint8_t *__restrict__ active,
                             double *__restrict__ pcurr, const double *__restrict__ pprev) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nv;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        if (!active[i]) continue;
-        const int32_t p = past[i], c = curr[i];
-        bool act = true;
-        if (numIters > 2 && c == p) {
-            const double pc = __dmul_rn(pprev[i], one_minus_delta);
-            pcurr[i] = pc;
-            if (pc <= 0.02) { // P_CUTOFF (louvain.hpp:74)
-                act = false;
-                active[i] = 0;
-            }
-        }
-        if (act) {
-            past[i] = c;
-            curr[i] = target[i];
-            target[i] = p;
-        }
-    }
+         i += (int64_t)gridDim.x * blockDim.x)
+        swap_et24(i, numIters, one_minus_delta, past, curr, target, active, pcurr, pprev);
 }
+
+#include "phase_small.cuh"
 
 __global__ void k_widen(const int32_t *__restrict__ in, int64_t n, int64_t *__restrict__ out) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -2207,6 +2256,133 @@ struct PhaseTiming {
     int64_t edges = 0;
 };
 
+// How k_phase_small may be launched on the context's device: the largest cluster (0: none)
+// and the blocks of a cooperative launch; asked once per context, with the kernels'
+// attributes set for that device.
+static void small_limits(vg_ctx *ctx) {
+    if (ctx->small_cluster >= 0) return;
+    for (auto *k : {k_phase_small<false>, k_phase_small<true>})
+        VG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SP_WORK_BYTES));
+    VG_CUDA(cudaFuncSetAttribute(k_phase_small<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    int best = 0;
+    for (int size = SP_MAX_CLUSTER; size >= 1 && !best; size /= 2) {
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = size;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(size);
+        cfg.blockDim = dim3(SP_THREADS);
+        cfg.dynamicSmemBytes = SP_WORK_BYTES;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_phase_small<false>, &cfg) == cudaSuccess && n > 0)
+            best = size;
+        else
+            cudaGetLastError();
+    }
+    int coop = 0, per_sm = 0;
+    VG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
+    VG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_phase_small<true>, SP_THREADS,
+                                                          SP_WORK_BYTES));
+    ctx->small_grid = coop && per_sm > 0 ? ctx->sm_count : 0;
+    ctx->small_cluster = best;
+}
+
+// One phase of a small graph by k_phase_small; false when the graph is not one it takes
+// (then nothing has changed). Results as run_phase's.
+static bool run_phase_small(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, int et,
+                            double *mod_out, int32_t *iters_out, double *sweep_ms) {
+    const int64_t nv = g->nv;
+    if (nv == 0 || nv > SP_MAX_NV || g->ne > SP_MAX_NE) return false;
+    small_limits(ctx);
+    const bool grid = g->ne > VG_SP_CLUSTER_NE;
+    const int limit = grid ? ctx->small_grid : ctx->small_cluster;
+    int blocks = grid ? limit : 1;
+    while (!grid && blocks < limit && g->ne > (int64_t)blocks * VG_SP_NE_PER_CTA) blocks *= 2;
+    if (limit == 0) return false;
+    const bool et24 = et == 2 || et == 4;
+    // one scratch block: 16-byte parts first, then 8, 4 and 1
+    const size_t n = (size_t)nv, units = (size_t)((nv + SEG_CHUNK - 1) / SEG_CHUNK) * SP_UNITS;
+    const size_t doubles = 3 * n + 3 * units + (et ? n : 0) + (et24 ? 2 * n : 0);
+    const size_t bytes = sizeof(CommInfo) * n + sizeof(double) * doubles +
+                         sizeof(int32_t) * (5 * n + SP_CTL + 1) + (et ? n : 0);
+    DevBuf<unsigned char> scratch(ctx, bytes);
+    DevBuf<int32_t> comm(ctx, nv);
+    unsigned char *at = scratch.p;
+    auto take = [&](size_t b) {
+        unsigned char *q = at;
+        at += b;
+        return q;
+    };
+    SmallPhase sp{};
+    sp.a.rowptr = g->rowptr;
+    sp.a.tail = g->tail;
+    sp.a.weight = g->weight;
+    sp.a.ref = g->ref;
+    sp.a.ne = g->ne;
+    sp.nv = nv;
+    sp.a.cupd = (CommInfo *)take(sizeof(CommInfo) * n);
+    sp.a.vdeg = sp.vdeg = (double *)take(sizeof(double) * n);
+    sp.a.cdeg = sp.cdeg = (double *)take(sizeof(double) * n);
+    sp.a.cw = (double *)take(sizeof(double) * n);
+    sp.part = (double *)take(sizeof(double) * 3 * units);
+    if (et) sp.a.frozen = (double *)take(sizeof(double) * n);
+    if (et24) {
+        sp.pa = (double *)take(sizeof(double) * n);
+        sp.pb = (double *)take(sizeof(double) * n);
+    }
+    sp.a.csize = sp.csize = (int32_t *)take(sizeof(int32_t) * n);
+    for (auto &b : sp.buf) b = (int32_t *)take(sizeof(int32_t) * n);
+    sp.list = (int32_t *)take(sizeof(int32_t) * n);
+    sp.ctl = (int32_t *)take(sizeof(int32_t) * SP_CTL);
+    sp.arrived = (unsigned *)take(sizeof(unsigned));
+    sp.a.noprune = sp.ctl + CTL_NOPRUNE;
+    if (et) sp.a.active = sp.active = take(n);
+    sp.comm = comm.p;
+    sp.lower = p->lower;
+    sp.threshold = p->threshold;
+    sp.one_minus_delta = 1.0 - p->et_delta;
+    sp.et = et;
+    sp.integral = g->integral == 1;
+    sp.tmax = nv <= (int64_t)VG_SP_WARP_ROWS * SP_WARPS * blocks ? 0 : SP_T;
+    if (grid) VG_CUDA(cudaMemsetAsync(sp.arrived, 0, sizeof(unsigned), ctx->stream));
+    SmallOut *out = (SmallOut *)vg_pinned(ctx, sizeof(SmallOut));
+    out->status = SP_DONE;
+    sp.out = out;
+    {
+        cudaLaunchAttribute la{};
+        if (grid) {
+            la.id = cudaLaunchAttributeCooperative;
+            la.val.cooperative = 1;
+        } else {
+            la.id = cudaLaunchAttributeClusterDimension;
+            la.val.clusterDim.x = blocks;
+            la.val.clusterDim.y = la.val.clusterDim.z = 1;
+        }
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(SP_THREADS);
+        cfg.dynamicSmemBytes = SP_WORK_BYTES;
+        cfg.stream = ctx->stream;
+        cfg.attrs = &la;
+        cfg.numAttrs = 1;
+        LaunchTimer lt(ctx);
+        VG_CUDA(cudaLaunchKernelEx(&cfg, grid ? k_phase_small<true> : k_phase_small<false>, sp));
+    }
+    vg_sync(ctx);
+    if (out->status == SP_TIMEOUT)
+        vg_throw(VG_ERR_TIMEOUT, "a barrier of the small phase waited too long");
+    if (out->status == SP_REFUSED) return false;
+    if (sweep_ms) *sweep_ms = out->sweep_ns * 1e-6;
+    *mod_out = out->mod;
+    *iters_out = out->iters;
+    vg_free(ctx, g->comm, sizeof(int32_t) * nv);
+    g->comm = comm.detach();
+    return true;
+}
+
 // the phase proper; returns the communities in g->comm
 // max_iters > 0 stops after that many iterations (the autotuner's timing runs)
 static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double *mod_out,
@@ -2228,6 +2404,16 @@ static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double
         }
     }
     const bool use_et = et != 0;
+    if (ordering == 0 && max_iters == 0) {
+        double ms = 0.0;
+        if (run_phase_small(ctx, g, p, et, mod_out, iters_out, &ms)) {
+            if (timing) {
+                timing->sweep_ms = ms;
+                timing->edges = g->ne * *iters_out;
+            }
+            return;
+        }
+    }
     DevBuf<double> vdeg(ctx, nv), cw(ctx, nv);
     DevBuf<double> cdeg(ctx, nv);
     DevBuf<int32_t> csize(ctx, nv);

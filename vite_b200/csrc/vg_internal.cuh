@@ -63,6 +63,9 @@ struct vg_ctx {
     // with the events that fork it from and join it back to the main stream
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
+    // blocks the one-launch small phase may use: the largest cluster the device takes and
+    // a cooperative launch's; -1: not yet asked
+    int small_cluster = -1, small_grid = 0;
 };
 
 // the context's side stream: work enqueued on the stream vg_side_fork returns, up to
