@@ -11,6 +11,7 @@
 //      keys; segments with more than 256 distinct keys go through one stable radix
 //      sort of all their entries by (segment, c2) and each run is folded in order;
 //   3. the unique entries are compacted into the next CSR.
+#include "grid_sync.cuh"
 #include "vg_internal.cuh"
 
 #include <algorithm>
@@ -200,6 +201,167 @@ template <int CAP, int MAXU> struct HashWarpSmem {
     alignas(16) double stage[32];
 };
 
+// a segment's entries: read-only in a launch of their own, LIVE when this launch wrote them
+template <bool LIVE, class T> __device__ __forceinline__ T seg_ld(const T *p) {
+    return LIVE ? __ldcg(p) : __ldg(p);
+}
+
+// One segment (entries [b, b + L) of gk/gw) by one warp: its distinct keys in order and
+// their sums to uk/uw at b. Returns their number, or -1 when there are more than MAXU.
+template <bool LIVE, int CAP, int MAXU>
+__device__ __forceinline__ int warp_segment(HashWarpSmem<CAP, MAXU> &S, int64_t b, int64_t L,
+                                            const int32_t *gk, const double *gw, int32_t *uk,
+                                            double *uw) {
+    const int lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
+    if (L <= 32) {
+        // one chunk: the leader of each key folds its lanes in lane order (the
+        // table path's sum for a key first met in this chunk), and the leaders'
+        // (key, sum) pairs are sorted across the lanes; no table needed
+        const bool has = lane < L;
+        const int32_t k = has ? seg_ld<LIVE>(gk + b + lane) : -2 - lane;
+        const double w = has ? seg_ld<LIVE>(gw + b + lane) : 0.0;
+        S.stage[lane] = w;
+        const unsigned peers = __match_any_sync(full, k);
+        __syncwarp();
+        const bool lead = has && lane == __ffs(peers) - 1;
+        double val = w;
+        const unsigned above = peers & ~((2u << lane) - 1u);
+        if (lead && above) val = vg_fold_above(val, S.stage, above);
+        const int U = __popc(__ballot_sync(full, lead));
+        int32_t key = lead ? k : INT_MAX;
+#pragma unroll
+        for (int k2 = 2; k2 <= 32; k2 <<= 1)
+#pragma unroll
+            for (int j = k2 >> 1; j > 0; j >>= 1) {
+                const int32_t pk = __shfl_xor_sync(full, key, j);
+                const double pv = __shfl_xor_sync(full, val, j);
+                const bool up = (lane & k2) == 0;
+                const bool low = (lane & j) == 0;
+                const bool take = (low == up) ? (pk < key) : (pk > key);
+                if (take) {
+                    key = pk;
+                    val = pv;
+                }
+            }
+        if (lane < U) {
+            uk[b + lane] = key;
+            uw[b + lane] = val;
+        }
+        __syncwarp();
+        return U;
+    }
+    int logcap = 5;
+    while ((1 << logcap) < 2 * L && (1 << logcap) < CAP) logcap++;
+    const int cap = 1 << logcap; // > twice the distinct keys held (at most MAXU + 31)
+    for (int s = lane; s < cap; s += 32) S.keys[s] = H_EMPTY;
+    __syncwarp();
+    int U = 0;
+    bool over = false;
+    // groups of four 32-entry chunks, the group's loads issued together
+    for (int64_t base = 0; base < L && !over; base += 4 * 32) {
+        int32_t kq[4];
+        double wq[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int64_t i = base + j * 32 + lane;
+            kq[j] = -2 - lane; // distinct non-keys for idle lanes
+            wq[j] = 0.0;
+            if (i < L) {
+                kq[j] = seg_ld<LIVE>(gk + b + i);
+                wq[j] = seg_ld<LIVE>(gw + b + i);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (base + j * 32 >= L) break; // warp-uniform
+            const bool has = base + j * 32 + lane < L;
+            const int32_t k = kq[j];
+            const double w = wq[j];
+            S.stage[lane] = w;
+            const unsigned peers = __match_any_sync(full, k);
+            __syncwarp();
+            bool fresh = false;
+            int slot = 0;
+            if (has && lane == __ffs(peers) - 1) {
+                uint32_t h = ((uint32_t)k * 2654435761u) >> (32 - logcap);
+                for (;;) {
+                    const int32_t kk = S.keys[h];
+                    if (kk == k) break;
+                    if (kk == H_EMPTY) {
+                        const int32_t old = atomicCAS(&S.keys[h], H_EMPTY, k);
+                        if (old == H_EMPTY) {
+                            fresh = true;
+                            break;
+                        }
+                        if (old == k) break;
+                    }
+                    h = (h + 1) & (uint32_t)(cap - 1);
+                }
+                slot = (int)h;
+                double acc = fresh ? w : __dadd_rn(S.vals[h], w);
+                const unsigned above = peers & ~((2u << lane) - 1u);
+                if (above) acc = vg_fold_above(acc, S.stage, above);
+                S.vals[h] = acc;
+            }
+            const unsigned fm = __ballot_sync(full, fresh);
+            if (fresh) S.list[U + __popc(fm & lt)] = ((uint64_t)(uint32_t)k << 32) | (uint32_t)slot;
+            U += __popc(fm);
+            __syncwarp();
+            if (U > MAXU) { // too many distinct keys for the table: the next tier
+                over = true;
+                break;
+            }
+        }
+    }
+    if (over) {
+        __syncwarp();
+        return -1;
+    }
+    if (U <= 32) {
+        // bitonic network across the lanes on (key, sum)
+        int32_t key = INT_MAX;
+        double val = 0.0;
+        if (lane < U) {
+            const uint64_t e = S.list[lane];
+            key = (int32_t)(e >> 32);
+            val = S.vals[(uint32_t)e];
+        }
+#pragma unroll
+        for (int k2 = 2; k2 <= 32; k2 <<= 1)
+#pragma unroll
+            for (int j = k2 >> 1; j > 0; j >>= 1) {
+                const int32_t pk = __shfl_xor_sync(full, key, j);
+                const double pv = __shfl_xor_sync(full, val, j);
+                const bool up = (lane & k2) == 0;
+                const bool low = (lane & j) == 0;
+                // the lower lane of an ascending pair keeps the minimum
+                const bool take = (low == up) ? (pk < key) : (pk > key);
+                if (take) {
+                    key = pk;
+                    val = pv;
+                }
+            }
+        if (lane < U) {
+            uk[b + lane] = key;
+            uw[b + lane] = val;
+        }
+    } else {
+        int n2 = 64;
+        while (n2 < U) n2 <<= 1;
+        for (int i = U + lane; i < n2; i += 32) S.list[i] = ~0ULL;
+        __syncwarp();
+        bitonic<true>(S.list, n2, lane, 32);
+        for (int i = lane; i < U; i += 32) {
+            const uint64_t e = S.list[i];
+            uk[b + i] = (int32_t)(e >> 32);
+            uw[b + i] = S.vals[(uint32_t)e];
+        }
+    }
+    __syncwarp();
+    return U;
+}
+
 // rows: null for every segment 0..nc-1, else the segments rows[0 .. *nrows)
 template <int CAP, int MAXU>
 __global__ void __launch_bounds__(H_WARPS * 32) k_rows_hash(
@@ -210,7 +372,6 @@ __global__ void __launch_bounds__(H_WARPS * 32) k_rows_hash(
     extern __shared__ unsigned char hsm_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     HashWarpSmem<CAP, MAXU> &S = reinterpret_cast<HashWarpSmem<CAP, MAXU> *>(hsm_raw)[warp];
-    const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
     const int64_t wg = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t n = rows ? *nrows : nc;
@@ -218,158 +379,10 @@ __global__ void __launch_bounds__(H_WARPS * 32) k_rows_hash(
         const int64_t row = rows ? rows[idx] : idx;
         const int64_t b = rstart[row];
         const int64_t L = rstart[row + 1] - b;
-        if (L <= 32) {
-            // one chunk: the leader of each key folds its lanes in lane order (the
-            // table path's sum for a key first met in this chunk), and the leaders'
-            // (key, sum) pairs are sorted across the lanes; no table needed
-            const bool has = lane < L;
-            const int32_t k = has ? gk[b + lane] : -2 - lane;
-            const double w = has ? gw[b + lane] : 0.0;
-            S.stage[lane] = w;
-            const unsigned peers = __match_any_sync(full, k);
-            __syncwarp();
-            const bool lead = has && lane == __ffs(peers) - 1;
-            double val = w;
-            const unsigned above = peers & ~((2u << lane) - 1u);
-            if (lead && above) val = vg_fold_above(val, S.stage, above);
-            const int U = __popc(__ballot_sync(full, lead));
-            int32_t key = lead ? k : INT_MAX;
-#pragma unroll
-            for (int k2 = 2; k2 <= 32; k2 <<= 1)
-#pragma unroll
-                for (int j = k2 >> 1; j > 0; j >>= 1) {
-                    const int32_t pk = __shfl_xor_sync(full, key, j);
-                    const double pv = __shfl_xor_sync(full, val, j);
-                    const bool up = (lane & k2) == 0;
-                    const bool low = (lane & j) == 0;
-                    const bool take = (low == up) ? (pk < key) : (pk > key);
-                    if (take) {
-                        key = pk;
-                        val = pv;
-                    }
-                }
-            if (lane < U) {
-                uk[b + lane] = key;
-                uw[b + lane] = val;
-            }
-            if (lane == 0) {
-                ucount[row] = U;
-                flag[row] = 0;
-            }
-            __syncwarp();
-            continue;
-        }
-        int logcap = 5;
-        while ((1 << logcap) < 2 * L && (1 << logcap) < CAP) logcap++;
-        const int cap = 1 << logcap; // > twice the distinct keys held (at most MAXU + 31)
-        for (int s = lane; s < cap; s += 32) S.keys[s] = H_EMPTY;
-        __syncwarp();
-        int U = 0;
-        bool over = false;
-        // groups of four 32-entry chunks, the group's loads issued together
-        for (int64_t base = 0; base < L && !over; base += 4 * 32) {
-            int32_t kq[4];
-            double wq[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int64_t i = base + j * 32 + lane;
-                kq[j] = -2 - lane; // distinct non-keys for idle lanes
-                wq[j] = 0.0;
-                if (i < L) {
-                    kq[j] = gk[b + i];
-                    wq[j] = gw[b + i];
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                if (base + j * 32 >= L) break; // warp-uniform
-                const bool has = base + j * 32 + lane < L;
-                const int32_t k = kq[j];
-                const double w = wq[j];
-                S.stage[lane] = w;
-                const unsigned peers = __match_any_sync(full, k);
-                __syncwarp();
-                bool fresh = false;
-                int slot = 0;
-                if (has && lane == __ffs(peers) - 1) {
-                    uint32_t h = ((uint32_t)k * 2654435761u) >> (32 - logcap);
-                    for (;;) {
-                        const int32_t kk = S.keys[h];
-                        if (kk == k) break;
-                        if (kk == H_EMPTY) {
-                            const int32_t old = atomicCAS(&S.keys[h], H_EMPTY, k);
-                            if (old == H_EMPTY) {
-                                fresh = true;
-                                break;
-                            }
-                            if (old == k) break;
-                        }
-                        h = (h + 1) & (uint32_t)(cap - 1);
-                    }
-                    slot = (int)h;
-                    double acc = fresh ? w : __dadd_rn(S.vals[h], w);
-                    const unsigned above = peers & ~((2u << lane) - 1u);
-                    if (above) acc = vg_fold_above(acc, S.stage, above);
-                    S.vals[h] = acc;
-                }
-                const unsigned fm = __ballot_sync(full, fresh);
-                if (fresh) S.list[U + __popc(fm & lt)] = ((uint64_t)(uint32_t)k << 32) | (uint32_t)slot;
-                U += __popc(fm);
-                __syncwarp();
-                if (U > MAXU) { // too many distinct keys for the table: the next tier
-                    over = true;
-                    break;
-                }
-            }
-        }
-        if (over) {
-            if (lane == 0) flag[row] = 1;
-            __syncwarp();
-            continue;
-        }
-        if (U <= 32) {
-            // bitonic network across the lanes on (key, sum)
-            int32_t key = INT_MAX;
-            double val = 0.0;
-            if (lane < U) {
-                const uint64_t e = S.list[lane];
-                key = (int32_t)(e >> 32);
-                val = S.vals[(uint32_t)e];
-            }
-#pragma unroll
-            for (int k2 = 2; k2 <= 32; k2 <<= 1)
-#pragma unroll
-                for (int j = k2 >> 1; j > 0; j >>= 1) {
-                    const int32_t pk = __shfl_xor_sync(full, key, j);
-                    const double pv = __shfl_xor_sync(full, val, j);
-                    const bool up = (lane & k2) == 0;
-                    const bool low = (lane & j) == 0;
-                    // the lower lane of an ascending pair keeps the minimum
-                    const bool take = (low == up) ? (pk < key) : (pk > key);
-                    if (take) {
-                        key = pk;
-                        val = pv;
-                    }
-                }
-            if (lane < U) {
-                uk[b + lane] = key;
-                uw[b + lane] = val;
-            }
-        } else {
-            int n2 = 64;
-            while (n2 < U) n2 <<= 1;
-            for (int i = U + lane; i < n2; i += 32) S.list[i] = ~0ULL;
-            __syncwarp();
-            bitonic<true>(S.list, n2, lane, 32);
-            for (int i = lane; i < U; i += 32) {
-                const uint64_t e = S.list[i];
-                uk[b + i] = (int32_t)(e >> 32);
-                uw[b + i] = S.vals[(uint32_t)e];
-            }
-        }
+        const int U = warp_segment<false>(S, b, L, gk, gw, uk, uw);
         if (lane == 0) {
-            ucount[row] = U;
-            flag[row] = 0;
+            if (U >= 0) ucount[row] = U;
+            flag[row] = U < 0;
         }
         __syncwarp();
     }
@@ -645,6 +658,8 @@ void long_rows(vg_ctx *ctx, const int64_t *offs, int64_t n, int64_t total, LongR
     L.grid = (int)std::min<int64_t>(total / COPY_CHUNK + cap, 16LL * ctx->sm_count);
 }
 
+#include "rebuild_small.cuh"
+
 } // namespace
 
 // Next-level CSR with nc rows. new_row[p]: row of position p's community; new_key[p]:
@@ -864,4 +879,76 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
         VG_CHECK_LAUNCH();
     }
     return vg_graph_wrap(ctx, nc, m, ucount.detach(), tail.detach(), w.detach());
+}
+
+// vg_rebuild_new of a small graph by k_rebuild_small; null when the graph is not one it
+// takes
+vg_graph *vg_rebuild_small(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) {
+    const int64_t nv = g->nv, ne = g->ne;
+    if (nv == 0 || nv > RS_MAX_NV || ne > RS_MAX_NE) return nullptr;
+    vg_grid_limits(ctx, k_rebuild_small<false>, k_rebuild_small<true>, RS_SMEM_BYTES,
+                   ctx->rebuild_limits);
+    const bool grid = ne > VG_RS_CLUSTER_NE;
+    const int limit = grid ? ctx->rebuild_limits.grid : ctx->rebuild_limits.cluster;
+    if (limit == 0 || limit > GS_THREADS) return nullptr; // a thread per block in the prefixes
+    int blocks = grid ? limit : 1;
+    while (!grid && blocks < limit && ne > (int64_t)blocks * VG_RS_NE_PER_CTA) blocks *= 2;
+    // one scratch block: 8-byte parts first
+    const size_t n = (size_t)nv, e = (size_t)ne, nb = (size_t)blocks;
+    const size_t wide = 6 * (n + 1) + 3 * nb + 2 * e;
+    const size_t narrow = 9 * n + RS_CTL + 1 + 2 * e;
+    DevBuf<unsigned char> scratch(ctx, 8 * wide + 4 * narrow);
+    int64_t *w8 = (int64_t *)scratch.p;
+    int32_t *w4 = (int32_t *)(scratch.p + 8 * wide);
+    auto take8 = [&](size_t k) { int64_t *q = w8; w8 += k; return q; };
+    auto take4 = [&](size_t k) { int32_t *q = w4; w4 += k; return q; };
+    SmallRebuild p{};
+    p.nv = nv;
+    p.ne = ne;
+    p.integral = g->integral == 1;
+    p.rowptr = g->rowptr;
+    p.tail = g->tail;
+    p.weight = g->weight;
+    p.ref = g->ref;
+    p.pos = g->pos;
+    p.comm = comm;
+    for (int64_t **q : {&p.mbase, &p.rstart, &p.ecount, &p.moff, &p.ucount, &p.rowptr_out})
+        *q = take8(n + 1);
+    p.part = take8(3 * nb);
+    p.gw = (double *)take8(e);
+    p.uw = (double *)take8(e);
+    for (int32_t **q : {&p.first_ref, &p.first_pos, &p.next_ref, &p.next_pos, &p.mcount, &p.mfill,
+                        &p.mlist, &p.biglist, &p.longlist})
+        *q = take4(n);
+    p.ctl = take4(RS_CTL);
+    p.arrived = (unsigned *)take4(1);
+    p.gk = take4(e);
+    p.uk = take4(e);
+    SmallRebuildOut *out = (SmallRebuildOut *)vg_pinned(ctx, sizeof(SmallRebuildOut));
+    out->status = GS_DONE;
+    p.out = out;
+    vg_grid_launch(ctx, grid ? k_rebuild_small<true> : k_rebuild_small<false>, p, grid, blocks,
+                   RS_SMEM_BYTES, p.arrived);
+    vg_sync(ctx);
+    if (out->status == GS_TIMEOUT)
+        vg_throw(VG_ERR_TIMEOUT, "a barrier of the small rebuild waited too long");
+    if (out->status == GS_REFUSED) return nullptr;
+    const int64_t nc = out->nc, m = out->m;
+    DevBuf<int64_t> rowptr(ctx, nc + 1);
+    DevBuf<int32_t> tail(ctx, m), ref(ctx, g->ref ? nc : 0), pos(ctx, g->ref ? nc : 0);
+    DevBuf<double> w(ctx, m);
+    {
+        LaunchTimer lt(ctx);
+        if (m >= LANES32_ROW * nc)
+            k_rebuild_small_copy<32><<<vg_grid(ctx, (nc + 1) * 32, 256), 256, 0, ctx->stream>>>(
+                p, nc, rowptr.p, tail.p, w.p, ref.p, pos.p);
+        else
+            k_rebuild_small_copy<8><<<vg_grid(ctx, (nc + 1) * 8, 256), 256, 0, ctx->stream>>>(
+                p, nc, rowptr.p, tail.p, w.p, ref.p, pos.p);
+    }
+    VG_CHECK_LAUNCH();
+    vg_graph *h = vg_graph_wrap(ctx, nc, m, rowptr.detach(), tail.detach(), w.detach());
+    h->ref = ref.detach();
+    h->pos = pos.detach();
+    return h;
 }

@@ -12,6 +12,7 @@
 //   swap       pointer rotation (plain) or the early-termination swaps.
 // Arithmetic follows the reference's expression order with explicit
 // round-to-nearest intrinsics, so no multiply-add is ever fused.
+#include "grid_sync.cuh"
 #include "vg_internal.cuh"
 
 #include <algorithm>
@@ -2256,49 +2257,15 @@ struct PhaseTiming {
     int64_t edges = 0;
 };
 
-// How k_phase_small may be launched on the context's device: the largest cluster (0: none)
-// and the blocks of a cooperative launch; asked once per context, with the kernels'
-// attributes set for that device.
-static void small_limits(vg_ctx *ctx) {
-    if (ctx->small_cluster >= 0) return;
-    for (auto *k : {k_phase_small<false>, k_phase_small<true>})
-        VG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SP_WORK_BYTES));
-    VG_CUDA(cudaFuncSetAttribute(k_phase_small<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    int best = 0;
-    for (int size = SP_MAX_CLUSTER; size >= 1 && !best; size /= 2) {
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = size;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(size);
-        cfg.blockDim = dim3(SP_THREADS);
-        cfg.dynamicSmemBytes = SP_WORK_BYTES;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, k_phase_small<false>, &cfg) == cudaSuccess && n > 0)
-            best = size;
-        else
-            cudaGetLastError();
-    }
-    int coop = 0, per_sm = 0;
-    VG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
-    VG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_phase_small<true>, SP_THREADS,
-                                                          SP_WORK_BYTES));
-    ctx->small_grid = coop && per_sm > 0 ? ctx->sm_count : 0;
-    ctx->small_cluster = best;
-}
-
 // One phase of a small graph by k_phase_small; false when the graph is not one it takes
 // (then nothing has changed). Results as run_phase's.
 static bool run_phase_small(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, int et,
                             double *mod_out, int32_t *iters_out, double *sweep_ms) {
     const int64_t nv = g->nv;
     if (nv == 0 || nv > SP_MAX_NV || g->ne > SP_MAX_NE) return false;
-    small_limits(ctx);
+    vg_grid_limits(ctx, k_phase_small<false>, k_phase_small<true>, SP_WORK_BYTES, ctx->phase_limits);
     const bool grid = g->ne > VG_SP_CLUSTER_NE;
-    const int limit = grid ? ctx->small_grid : ctx->small_cluster;
+    const int limit = grid ? ctx->phase_limits.grid : ctx->phase_limits.cluster;
     int blocks = grid ? limit : 1;
     while (!grid && blocks < limit && g->ne > (int64_t)blocks * VG_SP_NE_PER_CTA) blocks *= 2;
     if (limit == 0) return false;
@@ -2347,34 +2314,15 @@ static bool run_phase_small(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, 
     sp.et = et;
     sp.integral = g->integral == 1;
     sp.tmax = nv <= (int64_t)VG_SP_WARP_ROWS * SP_WARPS * blocks ? 0 : SP_T;
-    if (grid) VG_CUDA(cudaMemsetAsync(sp.arrived, 0, sizeof(unsigned), ctx->stream));
     SmallOut *out = (SmallOut *)vg_pinned(ctx, sizeof(SmallOut));
-    out->status = SP_DONE;
+    out->status = GS_DONE;
     sp.out = out;
-    {
-        cudaLaunchAttribute la{};
-        if (grid) {
-            la.id = cudaLaunchAttributeCooperative;
-            la.val.cooperative = 1;
-        } else {
-            la.id = cudaLaunchAttributeClusterDimension;
-            la.val.clusterDim.x = blocks;
-            la.val.clusterDim.y = la.val.clusterDim.z = 1;
-        }
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(blocks);
-        cfg.blockDim = dim3(SP_THREADS);
-        cfg.dynamicSmemBytes = SP_WORK_BYTES;
-        cfg.stream = ctx->stream;
-        cfg.attrs = &la;
-        cfg.numAttrs = 1;
-        LaunchTimer lt(ctx);
-        VG_CUDA(cudaLaunchKernelEx(&cfg, grid ? k_phase_small<true> : k_phase_small<false>, sp));
-    }
+    vg_grid_launch(ctx, grid ? k_phase_small<true> : k_phase_small<false>, sp, grid, blocks,
+                   SP_WORK_BYTES, sp.arrived);
     vg_sync(ctx);
-    if (out->status == SP_TIMEOUT)
+    if (out->status == GS_TIMEOUT)
         vg_throw(VG_ERR_TIMEOUT, "a barrier of the small phase waited too long");
-    if (out->status == SP_REFUSED) return false;
+    if (out->status == GS_REFUSED) return false;
     if (sweep_ms) *sweep_ms = out->sweep_ns * 1e-6;
     *mod_out = out->mod;
     *iters_out = out->iters;

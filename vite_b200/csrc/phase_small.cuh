@@ -23,9 +23,8 @@
 // result has the bits the general path gives (real weights: up to the order of the
 // community updates' atomics, as between two runs of it).
 
-constexpr int SP_THREADS = 512;
-constexpr int SP_WARPS = SP_THREADS / 32;
-constexpr int SP_MAX_CLUSTER = 16;
+constexpr int SP_THREADS = GS_THREADS;
+constexpr int SP_WARPS = GS_WARPS;
 constexpr int SP_T = 32;       // rows up to here: one thread each
 constexpr int SP_UNITS = SEG_CHUNK == 2048 && SEG_THREADS == 256 ? 8 : -1; // warps per chunk
 #ifndef VG_SP_MAX_NV
@@ -57,12 +56,8 @@ struct SmallOut {
     double mod;      // prevMod at the break
     double sweep_ns; // time between the barriers around the sweeps
     int32_t iters;
-    int32_t status;  // SP_DONE (set before the launch), SP_REFUSED or SP_TIMEOUT
-};
-enum : int32_t {
-    SP_DONE = 0,
-    SP_REFUSED = 1, // a row may hold more communities than the block's table
-    SP_TIMEOUT = 2  // a barrier's bounded wait ran out
+    int32_t status;  // GS_DONE; GS_REFUSED when a row may hold more communities
+                     // than a block's table
 };
 
 struct SmallPhase {
@@ -83,39 +78,6 @@ struct SmallPhase {
     unsigned *arrived; // (GRID) blocks that reached the grid's barriers so far (starts at 0)
     SmallOut *out;
 };
-
-// All blocks of the launch reach the barrier, and what they wrote before it is visible
-// after it. GRID: a counter in global memory (the launch is cooperative, so every block
-// is resident); a wait of SP_SPINS polls (seconds) gives up and returns false in every
-// thread of the block. Else the cluster's hardware barrier.
-constexpr int SP_SPINS = 1 << 23;
-template <bool GRID>
-__device__ __forceinline__ bool all_blocks(unsigned *arrived, unsigned &round, int &s_dead) {
-    if constexpr (GRID) {
-        round++;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            atomicAdd(arrived, 1u);
-            const unsigned want = round * gridDim.x;
-            int spins = 0;
-            unsigned seen;
-            do {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n"
-                             : "=r"(seen)
-                             : "l"(arrived)
-                             : "memory");
-            } while (seen < want && ++spins < SP_SPINS);
-            if (seen < want) s_dead = 1;
-            __threadfence();
-        }
-        __syncthreads();
-        return !s_dead;
-    } else {
-        asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
-        return true;
-    }
-}
 
 __device__ __forceinline__ uint64_t global_ns() {
     uint64_t t;
@@ -253,7 +215,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
     unsigned round = 0;
     auto barrier = [&]() -> bool {
         const bool ok = all_blocks<GRID>(p.arrived, round, s_dead);
-        if (!ok && tid == 0) p.out->status = SP_TIMEOUT;
+        if (!ok && tid == 0) p.out->status = GS_TIMEOUT;
         return ok;
     };
     const int64_t nv = p.nv;
@@ -285,7 +247,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
     }
     if (!barrier()) return;
     if (__ldcg(p.ctl + CTL_REFUSED)) { // the same in every block
-        if (rank == 0 && tid == 0) p.out->status = SP_REFUSED;
+        if (rank == 0 && tid == 0) p.out->status = GS_REFUSED;
         return;
     }
     const int wrows = __ldcg(p.ctl + CTL_WARP_ROWS), crows = __ldcg(p.ctl + CTL_CTA_ROWS);

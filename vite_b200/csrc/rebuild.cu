@@ -150,8 +150,14 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
                             const int32_t *new_row, const int32_t *new_key, int64_t nc,
                             const int32_t *key_to_pos);
 
+vg_graph *vg_rebuild_small(vg_ctx *ctx, const vg_graph *g, const int32_t *comm);
+
 vg_graph *vg_rebuild_new(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) {
     const int64_t nv = g->nv;
+    if (vg_graph *h = vg_rebuild_small(ctx, g, comm)) {
+        h->integral = g->integral == 1 ? 1 : -1; // sums of the same integers
+        return h;
+    }
     const int grid = vg_grid(ctx, nv, 256);
     if (!g->ref) {
         // reference layout: first appearance by position is first appearance by id

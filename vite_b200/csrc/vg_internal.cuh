@@ -41,6 +41,12 @@ struct vg_error : public std::exception {
 // ---------------------------------------------------------------------------------
 // context
 
+// of a kernel whose blocks wait on one another: the largest cluster the device takes and
+// the blocks of a cooperative launch (0: none); cluster -1: not yet asked
+struct GridLimits {
+    int cluster = -1, grid = 0;
+};
+
 struct vg_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -63,9 +69,8 @@ struct vg_ctx {
     // with the events that fork it from and join it back to the main stream
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
-    // blocks the one-launch small phase may use: the largest cluster the device takes and
-    // a cooperative launch's; -1: not yet asked
-    int small_cluster = -1, small_grid = 0;
+    // blocks the one-launch kernels of small graphs may use on the device
+    GridLimits phase_limits, rebuild_limits;
 };
 
 // the context's side stream: work enqueued on the stream vg_side_fork returns, up to
