@@ -74,3 +74,23 @@ def test_small_phase_negative_weights(ctx):
     w = g.weight.copy()
     w[(np.repeat(np.arange(g.nv), np.diff(g.rowptr)) + g.tail) % 3 == 0] = -2.0
     check(ctx, vo.Graph(g.rowptr, g.tail, w), False)
+
+
+@pytest.mark.parametrize("ordering", [1, 2])
+@pytest.mark.parametrize("et", [0, 2])
+@pytest.mark.parametrize("n,m,hub", [(500, 2000, 0), (3000, 20000, 700), (30000, 100000, 0)])
+def test_small_phase_colors(ctx, n, m, hub, et, ordering):
+    """A sweep per color, with and without the community update between colors; some
+    vertices stay uncolored."""
+    g = multigraph(n, m, 9, False, 4, hub)
+    colors, nc = vo.color(g, 2)
+    kw = dict(et_type=et, et_delta=0.25, ordering=ordering)
+    ref = vo.louvain_phase(g, colors=colors, num_color=nc + 1, **kw)
+    for reorder in (False, True):
+        dev = ctx.upload(g.rowptr, g.tail, g.weight)
+        if reorder:
+            ctx.reorder(dev, 1)
+        assert ctx.color(dev, 2)[1] == nc
+        cv, mod, it = ctx.louvain_phase(dev, **kw)
+        assert it == ref[2] and float(mod).hex() == float(ref[1]).hex()
+        np.testing.assert_array_equal(cv, ref[0])

@@ -48,6 +48,38 @@ __device__ __forceinline__ bool all_blocks(unsigned *arrived, unsigned &round, i
     }
 }
 
+// exclusive prefix over the warp's lanes and the warp's total
+__device__ __forceinline__ int64_t warp_excl(int64_t x, int64_t &total) {
+    const int lane = threadIdx.x & 31;
+    int64_t s = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += y;
+    }
+    total = __shfl_sync(0xffffffffu, s, 31);
+    return s - x;
+}
+
+// exclusive prefix over the block's threads and the block's total
+__device__ __forceinline__ int64_t block_excl(int64_t x, int64_t &total, int64_t *s_w) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t wt;
+    const int64_t e = warp_excl(x, wt);
+    if (lane == 31) s_w[warp] = wt;
+    __syncthreads();
+    int64_t before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < GS_WARPS; w++) {
+        const int64_t y = s_w[w];
+        before += w < warp ? y : 0;
+        all += y;
+    }
+    __syncthreads();
+    total = all;
+    return before + e;
+}
+
 // The blocks a kernel pair may be launched with: the largest cluster the device takes for
 // `in_cluster` and the blocks of a cooperative launch of `in_grid` (0: none). Sets the
 // kernels' attributes for the current device.

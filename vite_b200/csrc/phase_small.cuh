@@ -17,6 +17,9 @@
 // 1.54 and 2.31). With at most four vertices per warp of the launch every row gets a warp:
 // a thread's row of 32 entries is a 5-12 us chain, a warp's about 2 us.
 //
+// With colors a sweep and an update per color run the same way (30,000 / 479,846, 4
+// iterations of a -c 8 phase: 1.97 -> 0.94 ms; 150,000 / 1.8e6 with hubs: 4.4 -> 2.7).
+//
 // The rows go through the same code as the general sweeps (thread_vertex, warp_vertex,
 // cta_vertex), with loads that bypass the caches a previous iteration may have filled, and
 // the sums keep the chunks and trees of k_seg_sum_* / k_apply_seg / k_mod_seg, so every
@@ -48,8 +51,12 @@ static_assert(SP_UNITS == 8, "the chunk sums below assume 2048-entry chunks of 2
 static_assert(SP_MAX_NV <= (int64_t)SEG_FINAL * SEG_CHUNK && SEG_FINAL == 1024,
               "one chunk per thread of k_mod_seg's block in the final sums");
 
-// the words of SmallPhase::ctl
-enum { CTL_WARP_ROWS, CTL_CTA_ROWS, CTL_REFUSED, CTL_NOPRUNE, SP_CTL };
+constexpr int SP_MAX_COLORS = 256;
+// rows by length: a thread (or a warp, when they are few), a warp, a block
+enum { ROW_SHORT, ROW_WARP, ROW_BLOCK, SP_CLASSES };
+// the words of SmallPhase::ctl: rows per (color, class), then those placed so far
+enum { CTL_REFUSED, CTL_NOPRUNE, CTL_COUNT };
+__host__ __device__ constexpr int sp_ctl_words(int colors) { return CTL_COUNT + 2 * SP_CLASSES * colors; }
 
 // what the kernel tells the host (pinned memory)
 struct SmallOut {
@@ -69,12 +76,14 @@ struct SmallPhase {
     uint8_t *active;
     double *pa, *pb; // early termination 2 / 4
     double *part;    // 3 doubles per warp of each chunk
-    int32_t *list;   // long rows: warp rows from the front, block rows from the back
-    int32_t *ctl;    // SP_CTL words, zeroed by the first block
+    int32_t *list;   // rows by (color, class); without colors only the long ones
+    int32_t *ctl;    // sp_ctl_words(ncolors) words, zeroed by the first block
     int32_t *comm;   // the result
     double lower, threshold, one_minus_delta;
     int32_t et, integral;
-    int32_t tmax;      // rows up to here (0 or SP_T) get a thread, longer ones a warp or a block
+    const int32_t *colors; // null: every vertex in one sweep; else a sweep and a community
+                           // update per color (louvain.cpp:724-735)
+    int32_t ncolors;       // uncolored (-1) vertices go with the last one
     unsigned *arrived; // (GRID) blocks that reached the grid's barriers so far (starts at 0)
     SmallOut *out;
 };
@@ -207,7 +216,8 @@ template <bool GRID>
 __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ CtaShared<SP_THREADS> sh;
-    __shared__ int s_dead;
+    __shared__ int s_dead, s_base[SP_CLASSES * SP_MAX_COLORS + 1];
+    __shared__ int64_t s_w[SP_WARPS];
     __shared__ double s_sum[3], s_part[3][32];
     double *work = reinterpret_cast<double *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -225,34 +235,60 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
     const int warp_id = rank + warp * blocks, warps = blocks * SP_WARPS; // neighbours on other SMs
 
     if (tid == 0) s_dead = 0;
-    if (rank == 0 && tid < SP_CTL) p.ctl[tid] = 0;
+    const int buckets = SP_CLASSES * p.ncolors;
+    int32_t *count = p.ctl + CTL_COUNT, *placed = count + buckets;
+    if (rank == 0)
+        for (int i = tid; i < sp_ctl_words(p.ncolors); i += SP_THREADS) p.ctl[i] = 0;
     if (!barrier()) return;
-    // short rows' degrees are folded at once; the rows a warp or a block takes are listed,
-    // so that they spread over the blocks wherever they lie (a coarse level's longest rows
-    // are its first ones)
+    // Short rows' degrees are folded at once. The other rows (with colors: all) are counted
+    // by color and class, then listed, so that a class spreads over the blocks wherever its
+    // rows lie (a coarse level's longest rows are its first ones).
+    auto bucket_of = [&](int64_t v, int64_t d) {
+        const int cls = d <= SP_T ? ROW_SHORT : d <= WT_MAXDEG ? ROW_WARP : ROW_BLOCK;
+        if (!p.colors) return cls == ROW_SHORT ? -1 : cls;
+        const int32_t c = __ldg(p.colors + v);
+        return (c < 0 ? p.ncolors - 1 : c) * SP_CLASSES + cls;
+    };
     for (int64_t b = warp_id; b * 32 < nv; b += warps) {
         const int64_t v = b * 32 + lane;
-        if (v >= nv) continue;
-        const int64_t e0 = a.rowptr[v], e1 = a.rowptr[v + 1];
-        const int64_t d = e1 - e0;
-        if (d <= SP_T) p.vdeg[v] = row_fold(a.weight, e0, e1);
-        if (d > p.tmax) {
-            if (d <= WT_MAXDEG) {
-                p.list[atomicAdd(p.ctl + CTL_WARP_ROWS, 1)] = (int32_t)v;
-            } else {
-                if (min(d, nv) > CT_MAXDEG) p.ctl[CTL_REFUSED] = 1;
-                p.list[nv - 1 - atomicAdd(p.ctl + CTL_CTA_ROWS, 1)] = (int32_t)v;
-            }
+        int bucket = -1;
+        if (v < nv) {
+            const int64_t e0 = a.rowptr[v], e1 = a.rowptr[v + 1];
+            const int64_t d = e1 - e0;
+            if (d <= SP_T) p.vdeg[v] = row_fold(a.weight, e0, e1);
+            if (min(d, nv) > CT_MAXDEG) p.ctl[CTL_REFUSED] = 1;
+            bucket = bucket_of(v, d);
         }
+        const unsigned peers = __match_any_sync(0xffffffffu, bucket);
+        if (bucket >= 0 && lane == __ffs(peers) - 1) atomicAdd(count + bucket, __popc(peers));
     }
     if (!barrier()) return;
     if (__ldcg(p.ctl + CTL_REFUSED)) { // the same in every block
         if (rank == 0 && tid == 0) p.out->status = GS_REFUSED;
         return;
     }
-    const int wrows = __ldcg(p.ctl + CTL_WARP_ROWS), crows = __ldcg(p.ctl + CTL_CTA_ROWS);
-    for (int i = warp_id; i < wrows + crows; i += warps) {
-        const int32_t v = __ldcg(p.list + (i < wrows ? i : nv - 1 - (i - wrows)));
+    int rows = 0; // listed
+    for (int t = 0; t < buckets; t += SP_THREADS) {
+        int64_t total;
+        const int64_t e = block_excl(t + tid < buckets ? __ldcg(count + t + tid) : 0, total, s_w);
+        if (t + tid < buckets) s_base[t + tid] = rows + (int)e;
+        rows += (int)total;
+    }
+    if (tid == 0) s_base[buckets] = rows;
+    __syncthreads();
+    for (int64_t b = warp_id; b * 32 < nv; b += warps) {
+        const int64_t v = b * 32 + lane;
+        const int bucket = v < nv ? bucket_of(v, a.rowptr[v + 1] - a.rowptr[v]) : -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, bucket);
+        const int lead = __ffs(peers) - 1;
+        int at = 0;
+        if (bucket >= 0 && lane == lead) at = atomicAdd(placed + bucket, __popc(peers));
+        at = __shfl_sync(0xffffffffu, at, lead);
+        if (bucket >= 0) p.list[s_base[bucket] + at + __popc(peers & ((1u << lane) - 1u))] = (int32_t)v;
+    }
+    if (!barrier()) return;
+    for (int i = warp_id; i < rows; i += warps) {
+        const int32_t v = __ldcg(p.list + i);
         const int64_t E0 = a.rowptr[v], E1 = a.rowptr[v + 1];
         if (E1 - E0 <= SP_T) continue;
         double s = 0.0;
@@ -300,51 +336,8 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
     a.constant = cst;
     // no block overwrites p.part before the next barrier
 
-    int ip = 0; // buf[ip], buf[ip + 1], buf[ip + 2] (mod 3): past, curr, target
-    double *pcurr = p.pa, *pprev = p.pb;
-    double prev = p.lower, sweep_ns = 0.0;
-    int iters = 0;
-    for (;;) {
-        iters++;
-        int32_t *past = p.buf[ip], *curr = p.buf[(ip + 1) % 3], *target = p.buf[(ip + 2) % 3];
-        a.curr = curr;
-        a.target = target;
-        const uint64_t t0 = rank == 0 && tid == 0 ? global_ns() : 0;
-        for (int i = rank; i < crows; i += blocks) { // uniform over the block
-            const int32_t v = __ldcg(p.list + nv - 1 - i);
-            const int64_t e0 = a.rowptr[v], d = a.rowptr[v + 1] - e0;
-            cta_vertex<SP_THREADS>(a, v, e0, d, min(d, nv), cst,
-                                   reinterpret_cast<int32_t *>(work + CT_CAP), work,
-                                   work + CT_CAP + CT_CAP / 2, sh);
-            __syncthreads();
-        }
-        for (int64_t b = warp_id; b * 32 < nv; b += warps) {
-            const int64_t v = b * 32 + lane;
-            if (v >= nv) continue;
-            const int64_t e0 = a.rowptr[v];
-            const int64_t d = a.rowptr[v + 1] - e0;
-            if (d <= p.tmax)
-                thread_vertex<SP_T, SP_THREADS>(a, (int32_t)v, e0, (int)d, cst, work + tid);
-        }
-        if (wrows) {
-            __syncthreads();
-            double *vals = work + (size_t)warp * WT_CAP;
-            int32_t *keys = reinterpret_cast<int32_t *>(work + (size_t)SP_WARPS * WT_CAP) +
-                            (size_t)warp * WT_CAP;
-            double *stage = work + (size_t)SP_WARPS * (WT_CAP + WT_CAP / 2) + (size_t)warp * 32;
-            for (int i = warp_id; i < wrows; i += warps) {
-                const int32_t v = __ldcg(p.list + i);
-                const int64_t e0 = a.rowptr[v];
-                const int d = (int)(a.rowptr[v + 1] - e0);
-                if (d <= 32)
-                    warp_short_vertex(a, v, e0, d, cst, stage);
-                else
-                    warp_vertex(a, v, cst, keys, vals, stage);
-            }
-        }
-        if (!barrier()) return;
-        if (rank == 0 && tid == 0) sweep_ns += (double)(global_ns() - t0);
-        // community update and the sums of the modularity (k_apply_seg)
+    // community update and, with sums, those of the modularity (k_apply_seg)
+    auto apply = [&](bool sums) {
         for (int64_t u = warp_id; u < units; u += warps) {
             const int64_t lo = (u / SP_UNITS) * SEG_CHUNK, hi = min(lo + SEG_CHUNK, nv);
             double le = 0.0, la2 = 0.0, frozen = 0.0;
@@ -364,10 +357,12 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
                     z.pad = 0;
                     a.cupd[i] = z;
                 }
+                if (!sums) continue;
                 le = __dadd_rn(le, __ldcg(a.cw + i));
                 la2 = __dadd_rn(la2, __dmul_rn(cd, cd));
                 if (p.active && !__ldcg(p.active + i)) frozen += 1.0;
             }
+            if (!sums) continue;
             le = warp_tree(le);
             la2 = warp_tree(la2);
             frozen = warp_tree(frozen);
@@ -377,6 +372,73 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
                 p.part[3 * u + 2] = frozen;
             }
         }
+    };
+
+    int ip = 0; // buf[ip], buf[ip + 1], buf[ip + 2] (mod 3): past, curr, target
+    double *pcurr = p.pa, *pprev = p.pb;
+    double prev = p.lower, sweep_ns = 0.0;
+    int iters = 0;
+    for (;;) {
+        iters++;
+        int32_t *past = p.buf[ip], *curr = p.buf[(ip + 1) % 3], *target = p.buf[(ip + 2) % 3];
+        a.curr = curr;
+        a.target = target;
+        const uint64_t t0 = rank == 0 && tid == 0 ? global_ns() : 0;
+        for (int color = 0; color < p.ncolors; color++) {
+            if (color) {
+                if (!barrier()) return;
+                apply(false); // the last color's update has the sums
+                if (!barrier()) return;
+            }
+            // item i of the list goes to the block (warp) i modulo their number, so that the
+            // colors' rows fall to different ones
+            const int *base = s_base + SP_CLASSES * color;
+            auto first = [](int from, int id, int n) { // smallest i >= from, i = id modulo n
+                if (from <= id) return id;
+                const int d = (from - id) % n;
+                return d ? from + n - d : from;
+            };
+            for (int i = first(base[ROW_BLOCK], rank, blocks); i < base[SP_CLASSES]; i += blocks) {
+                const int32_t v = __ldcg(p.list + i);
+                const int64_t e0 = a.rowptr[v], d = a.rowptr[v + 1] - e0;
+                cta_vertex<SP_THREADS>(a, v, e0, d, min(d, nv), cst,
+                                       reinterpret_cast<int32_t *>(work + CT_CAP), work,
+                                       work + CT_CAP + CT_CAP / 2, sh);
+                __syncthreads();
+            }
+            // short rows: all vertices in turn, or the color's list
+            const int s0 = p.colors ? base[ROW_SHORT] : 0;
+            const int s1 = p.colors ? base[ROW_WARP] : (int)nv;
+            const bool by_thread = s1 - s0 > VG_SP_WARP_ROWS * warps;
+            if (by_thread) {
+                for (int b = first(s0 / 32, warp_id, warps); b * 32 < s1; b += warps) {
+                    const int i = b * 32 + lane;
+                    if (i < s0 || i >= s1) continue;
+                    const int32_t v = p.colors ? __ldcg(p.list + i) : i;
+                    const int64_t e0 = a.rowptr[v];
+                    const int64_t d = a.rowptr[v + 1] - e0;
+                    if (d <= SP_T) thread_vertex<SP_T, SP_THREADS>(a, v, e0, (int)d, cst, work + tid);
+                }
+                __syncthreads();
+            }
+            double *vals = work + (size_t)warp * WT_CAP;
+            int32_t *keys = reinterpret_cast<int32_t *>(work + (size_t)SP_WARPS * WT_CAP) +
+                            (size_t)warp * WT_CAP;
+            double *stage = work + (size_t)SP_WARPS * (WT_CAP + WT_CAP / 2) + (size_t)warp * 32;
+            if (!by_thread) {
+                for (int i = first(s0, warp_id, warps); i < s1; i += warps) {
+                    const int32_t v = p.colors ? __ldcg(p.list + i) : i;
+                    const int64_t e0 = a.rowptr[v];
+                    const int64_t d = a.rowptr[v + 1] - e0;
+                    if (d <= SP_T) warp_short_vertex(a, v, e0, (int)d, cst, stage);
+                }
+            }
+            for (int i = first(base[ROW_WARP], warp_id, warps); i < base[ROW_BLOCK]; i += warps)
+                warp_vertex(a, __ldcg(p.list + i), cst, keys, vals, stage);
+        }
+        if (!barrier()) return;
+        if (rank == 0 && tid == 0) sweep_ns += (double)(global_ns() - t0);
+        apply(true);
         if (!barrier()) return;
         small_final<3>(chunks, [&](int q, int w, int k) {
             return __ldcg(p.part + 3 * (q * SP_UNITS + w) + k);
