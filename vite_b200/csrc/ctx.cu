@@ -2,6 +2,7 @@
 // kernel (distSumVertexDegree / distCalcConstantForSecondTerm, louvain.cpp:2161-2218).
 #include "vg_internal.cuh"
 
+#include <algorithm>
 #include <cstring>
 
 void vg_throw(vg_status s, const char *fmt, ...) {
@@ -101,12 +102,17 @@ extern "C" vg_status vg_ctx_create(int device, size_t mem_budget_bytes, vg_ctx *
         ctx->device = device;
         ctx->budget = mem_budget_bytes;
         VG_CUDA(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device));
-        VG_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
-        // the side stream and its fork/join events exist from the start, so that a
+        // the blocks of the main and the first side stream go before the other side streams'
+        int least = 0, most = 0;
+        VG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &most));
+        VG_CUDA(cudaStreamCreateWithPriority(&ctx->stream, cudaStreamNonBlocking, most));
+        // the side streams and their fork/join events exist from the start, so that a
         // fork inside a stream capture creates nothing
-        VG_CUDA(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+        for (int k = 0; k < VG_SIDE; k++)
+            VG_CUDA(cudaStreamCreateWithPriority(&ctx->side[k], cudaStreamNonBlocking,
+                                                 k == 0 ? most : least));
+        for (auto &e : ctx->join) VG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         VG_CUDA(cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
-        VG_CUDA(cudaEventCreateWithFlags(&ctx->join, cudaEventDisableTiming));
         // keep freed blocks in the stream-ordered pool instead of returning them
         cudaMemPool_t pool;
         VG_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));
@@ -122,31 +128,36 @@ extern "C" vg_status vg_ctx_create(int device, size_t mem_budget_bytes, vg_ctx *
     return VG_OK;
 }
 
-cudaStream_t vg_side_fork(vg_ctx *ctx) {
+void vg_side_fork(vg_ctx *ctx, int n) {
+    if (n == 0) return;
     VG_CUDA(cudaEventRecord(ctx->fork, ctx->stream));
-    VG_CUDA(cudaStreamWaitEvent(ctx->side, ctx->fork, 0));
-    return ctx->side;
+    for (int k = 0; k < n; k++) VG_CUDA(cudaStreamWaitEvent(ctx->side[k], ctx->fork, 0));
 }
 
-void vg_side_join(vg_ctx *ctx) {
-    VG_CUDA(cudaEventRecord(ctx->join, ctx->side));
-    VG_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->join, 0));
+void vg_side_join(vg_ctx *ctx, int n) {
+    for (int k = 0; k < n; k++) {
+        VG_CUDA(cudaEventRecord(ctx->join[k], ctx->side[k]));
+        VG_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->join[k], 0));
+    }
 }
 
 extern "C" vg_status vg_ctx_destroy(vg_ctx *ctx) {
     if (!ctx) return VG_ERR_ARG;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    if (ctx->side) cudaStreamSynchronize(ctx->side);
+    for (auto s : ctx->side)
+        if (s) cudaStreamSynchronize(s);
     for (auto &pr : ctx->pending) ctx->event_pool.push_back(pr);
     for (auto &pr : ctx->event_pool) {
         cudaEventDestroy(pr.first);
         cudaEventDestroy(pr.second);
     }
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
-    if (ctx->side) cudaStreamDestroy(ctx->side);
+    for (auto s : ctx->side)
+        if (s) cudaStreamDestroy(s);
+    for (auto e : ctx->join)
+        if (e) cudaEventDestroy(e);
     if (ctx->fork) cudaEventDestroy(ctx->fork);
-    if (ctx->join) cudaEventDestroy(ctx->join);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return VG_OK;
@@ -348,7 +359,7 @@ extern "C" vg_status vg_graph_upload(vg_ctx *ctx, int64_t nv, int64_t ne, const 
                     VG_CUDA(cudaEventCreateWithFlags(&split[b], cudaEventDisableTiming));
                 }
                 const bool two = !ctx->profile; // with profiling every launch stays on one stream
-                cudaStream_t ss = two ? ctx->side : ctx->stream;
+                cudaStream_t ss = two ? ctx->side[0] : ctx->stream;
                 int64_t k = 0;
                 for (int64_t off = 0; off < ne; off += chunk, k++) {
                     const int b = (int)(k & 1);

@@ -266,52 +266,77 @@ __device__ __forceinline__ void best_of_row(const A &a, const int32_t (&c)[T],
     }
 }
 
-// distGetMaxIndex over the candidate slots keys/vals[i], i = base + lane + k * step < nk,
-// of one warp (all lanes call it); every lane returns the warp's best (ok, gain, cand).
-// With pruning (can_prune) the slot of largest bound is evaluated first and the others
-// only when their bound reaches the best gain; without, or when the largest bound is
-// shared by two slots, every slot, four community-degree loads per lane at a time. The
-// (gain, id) order makes the result independent of the visiting order.
-template <class A>
-__device__ __forceinline__ void warp_best(const A &a, const int32_t *keys,
-                                          const double *vals, int64_t base, int64_t step,
-                                          int64_t nk, double eix, double vd, double ax, double cst,
-                                          bool &ok, double &gain, int32_t &cand) {
+// the warp's largest x; every lane's is at least +0.0 (such doubles order as their bits do)
+__device__ __forceinline__ double warp_max(double x) {
+    const unsigned full = 0xffffffffu;
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned mh = __reduce_max_sync(full, hi);
+    const unsigned ml = __reduce_max_sync(full, hi == mh ? lo : 0u);
+    return __hiloint2double((int)mh, (int)ml);
+}
+
+// the warp's best of the lanes' (ok, gain > 0, cand) in the order of better(), in every lane
+__device__ __forceinline__ void warp_argbest(bool &ok, double &gain, int32_t &cand,
+                                             const int32_t *__restrict__ ref) {
+    const unsigned full = 0xffffffffu;
+    const double m = warp_max(ok ? gain : 0.0);
+    const bool mine = ok && gain == m;
+    const unsigned at = __ballot_sync(full, mine);
+    ok = at != 0;
+    gain = ok ? m : 0.0;
+    if (!ok) {
+        cand = INT_MAX;
+        return;
+    }
+    int lead = __ffs(at) - 1;
+    if (at & (at - 1)) { // equal gains: the smallest reference id
+        const unsigned r = mine ? (unsigned)vg_rid(ref, cand) : UINT_MAX;
+        const unsigned rm = __reduce_min_sync(full, r);
+        lead = __ffs(__ballot_sync(full, r == rm)) - 1;
+    }
+    cand = __shfl_sync(full, cand, lead);
+}
+
+// distGetMaxIndex over the items i = base + lane + k * step < n of one warp (all lanes call
+// it); get(i, key, w) gives an item's community and counter, false when it is no candidate.
+// Every lane returns the warp's best (ok, gain, cand). With pruning (can_prune) the item of
+// largest bound is evaluated first and the others only when their bound reaches the best
+// gain; without, or when the largest bound is shared by two items, every item, four
+// community-degree loads per lane at a time. The (gain, id) order makes the result
+// independent of the visiting order. The warp's maxima come from integer reductions of the
+// doubles' bits (two instructions each) instead of shuffle trees.
+template <class A, class Get>
+__device__ __forceinline__ void warp_best(const A &a, Get get, int base, int step, int n, double eix,
+                                          double vd, double ax, double cst, bool &ok,
+                                          double &gain, int32_t &cand) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     ok = false;
     gain = 0.0;
     cand = INT_MAX;
-    bool scan_all = true;
     if (can_prune(a, vd, cst)) { // vd and cst are the same in every lane
-        scan_all = false;
         double ub = 0.0, u2 = 0.0, uw = 0.0;
         int32_t uc = -1;
-        for (int64_t i = base + lane; i < nk; i += step) {
-            const double w = vals[i];
+        for (int i = base + lane; i < n; i += step) {
+            int32_t k;
+            double w;
+            if (!get(i, k, w)) continue;
             const double u = gain_of(w, eix, vd, 0.0, ax, cst);
             if (u > ub) {
                 u2 = ub;
                 ub = u;
-                uc = keys[i];
+                uc = k;
                 uw = w;
             } else if (u > u2) {
                 u2 = u;
             }
         }
-        double m = ub;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(full, m, o));
-        if (m > 0.0) {
-            const int wl = __ffs(__ballot_sync(full, uc >= 0 && ub == m)) - 1;
-            double sec = lane == wl ? u2 : ub; // the warp's second-largest bound
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sec = fmax(sec, __shfl_xor_sync(full, sec, o));
-            if (sec == m) {
-                // a tie at the top (integral weights): one round over every slot
-                scan_all = true;
-                goto full_scan;
-            }
+        __syncwarp();
+        const double m = warp_max(ub);
+        if (!(m > 0.0)) return; // no candidate has a positive bound: no move
+        const int wl = __ffs(__ballot_sync(full, uc >= 0 && ub == m)) - 1;
+        const double sec = warp_max(lane == wl ? u2 : ub); // the warp's second-largest bound
+        if (sec < m) {
             double g = 0.0;
             if (lane == wl) g = gain_of(uw, eix, vd, A::ld(a.cdeg + uc), ax, cst);
             g = __shfl_sync(full, g, wl);
@@ -321,64 +346,50 @@ __device__ __forceinline__ void warp_best(const A &a, const int32_t *keys,
                 gain = g;
                 cand = c0;
             }
-            if (sec > 0.0 && (!ok || sec >= gain)) {
-                for (int64_t i = base + lane; i < nk; i += step) {
-                    const int32_t k = keys[i];
-                    if (k == c0) continue;
-                    const double w = vals[i];
-                    const double u = gain_of(w, eix, vd, 0.0, ax, cst);
-                    if (u > 0.0 && (!ok || u >= gain)) {
-                        const double gg = gain_of(w, eix, vd, A::ld(a.cdeg + k), ax, cst);
-                        if (gg > 0.0 && better(true, gg, k, ok, gain, cand, a.ref)) {
-                            gain = gg;
-                            cand = k;
-                            ok = true;
-                        }
+            if (!(sec > 0.0 && (!ok || sec >= gain))) return; // every lane holds the result
+            for (int i = base + lane; i < n; i += step) {
+                int32_t k;
+                double w;
+                if (!get(i, k, w) || k == c0) continue;
+                const double u = gain_of(w, eix, vd, 0.0, ax, cst);
+                if (u > 0.0 && (!ok || u >= gain)) {
+                    const double gg = gain_of(w, eix, vd, A::ld(a.cdeg + k), ax, cst);
+                    if (gg > 0.0 && better(true, gg, k, ok, gain, cand, a.ref)) {
+                        gain = gg;
+                        cand = k;
+                        ok = true;
                     }
                 }
-                scan_all = false;
-            } else {
-                return; // every lane holds the warp's result
             }
-        } else {
-            return; // no candidate has a positive bound: no move
+            __syncwarp();
+            warp_argbest(ok, gain, cand, a.ref);
+            return;
         }
+        // a tie at the top (integral weights): one round over every item
     }
-full_scan:
-    if (scan_all) {
-        for (int64_t i0 = base; i0 < nk; i0 += 4 * step) {
-            int32_t kq[4];
-            double aq[4];
+    for (int i0 = base; i0 < n; i0 += 4 * step) {
+        int32_t kq[4];
+        double aq[4], wq[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int64_t i = i0 + j * step + lane;
-                kq[j] = i < nk ? keys[i] : EMPTY;
-            }
+        for (int j = 0; j < 4; j++) {
+            const int i = i0 + j * step + lane;
+            if (i >= n || !get(i, kq[j], wq[j])) kq[j] = EMPTY;
+        }
 #pragma unroll
-            for (int j = 0; j < 4; j++) aq[j] = kq[j] != EMPTY ? A::ld(a.cdeg + kq[j]) : 0.0;
+        for (int j = 0; j < 4; j++) aq[j] = kq[j] != EMPTY ? A::ld(a.cdeg + kq[j]) : 0.0;
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                if (kq[j] == EMPTY) continue;
-                const double g = gain_of(vals[i0 + j * step + lane], eix, vd, aq[j], ax, cst);
-                if (g > 0.0 && better(true, g, kq[j], ok, gain, cand, a.ref)) {
-                    gain = g;
-                    cand = kq[j];
-                    ok = true;
-                }
+        for (int j = 0; j < 4; j++) {
+            if (kq[j] == EMPTY) continue;
+            const double g = gain_of(wq[j], eix, vd, aq[j], ax, cst);
+            if (g > 0.0 && better(true, g, kq[j], ok, gain, cand, a.ref)) {
+                gain = g;
+                cand = kq[j];
+                ok = true;
             }
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double og = __shfl_xor_sync(full, gain, o);
-        const int32_t oc = __shfl_xor_sync(full, cand, o);
-        const bool ook = __shfl_xor_sync(full, (int)ok, o) != 0;
-        if (better(ook, og, oc, ok, gain, cand, a.ref)) {
-            gain = og;
-            cand = oc;
-            ok = true;
-        }
-    }
+    __syncwarp();
+    warp_argbest(ok, gain, cand, a.ref);
 }
 
 // the community sizes the singleton rule (louvain.cpp:2275-2276) reads: needed only
@@ -727,18 +738,62 @@ __device__ __forceinline__ uint32_t slot_hash(int32_t c, int logcap) {
 // weights in CSR order onto the table value, so each counter is the reference's
 // exact left fold.
 
-// shared memory of a k_sweep_warp block: vals[WARPS][CAP], keys[WARPS][CAP], stage[WARPS][32]
+// A table of CAP slots: empty (keys EMPTY, for a block's table also vals 0) between
+// vertices, because the slots a vertex used are listed and reset after it: on rows of 33-128
+// entries clearing, searching and compacting the whole table was two thirds of the work.
+struct Table {
+    double *vals;
+    int32_t *keys;
+    uint16_t *used; // CAP / 2 of them
+    double *stage;  // a double per thread that shares the table
+};
+
+// shared memory of a k_sweep_warp block: vals[WARPS][CAP], keys[WARPS][CAP],
+// stage[WARPS][32], used[WARPS][CAP / 2]
 template <int CAP, int WARPS> constexpr size_t warp_smem_bytes() {
-    return (size_t)WARPS * CAP * (sizeof(double) + sizeof(int32_t)) + (size_t)WARPS * 32 * sizeof(double);
+    return (size_t)WARPS * (CAP * (sizeof(double) + sizeof(int32_t)) + 32 * sizeof(double) +
+                            CAP / 2 * sizeof(uint16_t));
 }
 
-// vertex v by one warp; keys/vals: a table of at least twice its degree (rounded up to
-// a power of two), stage: 32 doubles, all the warp's own
+// warp `warp`'s table of such a block, made empty
+template <int CAP, int WARPS> __device__ __forceinline__ Table warp_table(unsigned char *smem, int warp) {
+    double *vals = reinterpret_cast<double *>(smem);
+    double *stage = vals + (size_t)WARPS * CAP;
+    int32_t *keys = reinterpret_cast<int32_t *>(stage + WARPS * 32);
+    uint16_t *used = reinterpret_cast<uint16_t *>(keys + (size_t)WARPS * CAP);
+    Table t{vals + (size_t)warp * CAP, keys + (size_t)warp * CAP, used + (size_t)warp * (CAP / 2),
+            stage + warp * 32};
+    for (int i = threadIdx.x & 31; i < CAP; i += 32) t.keys[i] = EMPTY;
+    __syncwarp();
+    return t;
+}
+
+// slot of c in a table of `mask` + 1 slots, claimed when c has none yet (fresh)
+__device__ __forceinline__ uint32_t table_slot(int32_t *keys, int32_t c, int logcap, bool &fresh) {
+    const uint32_t mask = (1u << logcap) - 1u;
+    uint32_t h = slot_hash(c, logcap);
+    fresh = false;
+    for (;;) {
+        const int32_t kk = *(volatile int32_t *)(keys + h);
+        if (kk == c) return h;
+        if (kk == EMPTY) {
+            const int32_t old = atomicCAS(keys + h, EMPTY, c);
+            if (old == EMPTY) {
+                fresh = true;
+                return h;
+            }
+            if (old == c) return h;
+        }
+        h = (h + 1) & mask;
+    }
+}
+
+// vertex v by one warp with a table (see warp_table) of at least twice its degree
 template <class A>
-__device__ __forceinline__ void warp_vertex(const A &a, int32_t v, double cst, int32_t *keys,
-                                            double *vals, double *stage) {
+__device__ __forceinline__ void warp_vertex(const A &a, int32_t v, double cst, const Table &t) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
     const int32_t cc = A::ld(a.curr + v);
     if (a.active && !A::ld(a.active + v)) {
         if (lane == 0) a.cw[v] = A::ld(a.frozen + v);
@@ -746,12 +801,11 @@ __device__ __forceinline__ void warp_vertex(const A &a, int32_t v, double cst, i
     }
     const int64_t e0 = a.rowptr[v];
     const int d = (int)(a.rowptr[v + 1] - e0);
-    int logcap = 5;
-    while ((1 << logcap) < 2 * d) logcap++;
-    const int cap = 1 << logcap;
-    for (int s = lane; s < cap; s += 32) keys[s] = EMPTY;
-    __syncwarp();
+    const double vd = A::ld(a.vdeg + v);
+    const double ccDeg = A::ld(a.cdeg + cc);
+    const int logcap = max(5, 32 - __clz(2 * d - 1)); // smallest power of two >= 2 d
     double selfLoop = 0.0;
+    int n = 0, own = -1; // slots used; the current community's
     // groups of four 32-edge chunks: the group's tails and weights are loaded
     // together, then their communities, so a group costs two round trips
     for (int g0 = 0; g0 < d; g0 += 4 * 32) {
@@ -764,87 +818,55 @@ __device__ __forceinline__ void warp_vertex(const A &a, int32_t v, double cst, i
             ww[j] = k < d ? a.weight[e0 + k] : 0.0;
         }
 #pragma unroll
-        for (int j = 0; j < 4; j++) cg[j] = tt[j] >= 0 ? A::ld(a.curr + tt[j]) : -1;
+        for (int j = 0; j < 4; j++) cg[j] = tt[j] >= 0 ? A::ld(a.curr + tt[j]) : -1 - lane;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             if (g0 + j * 32 >= d) break; // warp-uniform
             const bool has = tt[j] >= 0;
-            const int32_t t = tt[j], c = cg[j];
-            stage[lane] = ww[j];
-            const unsigned peers = __match_any_sync(full, has ? c : (-1 - lane));
-            __syncwarp();
-            if (has && lane == __ffs(peers) - 1) {
-                uint32_t h = slot_hash(c, logcap);
-                bool fresh = false;
-                for (;;) {
-                    const int32_t kk = keys[h];
-                    if (kk == c) break;
-                    if (kk == EMPTY) {
-                        const int32_t old = atomicCAS(&keys[h], EMPTY, c);
-                        if (old == EMPTY) {
-                            fresh = true;
-                            break;
-                        }
-                        if (old == c) break;
-                    }
-                    h = (h + 1) & (cap - 1);
-                }
-                const unsigned above = peers & ~((2u << lane) - 1u);
-                double acc = fresh ? stage[lane] : __dadd_rn(vals[h], stage[lane]);
-                if (above) acc = vg_fold_above(acc, stage, above);
-                vals[h] = acc;
+            const int32_t c = cg[j];
+            const unsigned peers = __match_any_sync(full, c);
+            const bool lead = has && (peers & lt) == 0;
+            const unsigned above = lead ? peers & ~lt & ~(1u << lane) : 0u;
+            const unsigned most = __reduce_max_sync(full, (unsigned)__popc(above));
+            const unsigned selfm = __ballot_sync(full, has && tt[j] == v);
+            if (most | selfm) {
+                t.stage[lane] = ww[j];
+                __syncwarp();
             }
-            const unsigned selfm = __ballot_sync(full, has && t == v);
-            {
-                unsigned m = selfm;
-                while (m) {
-                    const int b = __ffs(m) - 1;
-                    selfLoop = __dadd_rn(selfLoop, stage[b]);
-                    m &= m - 1;
-                }
+            bool fresh = false;
+            uint32_t h = 0;
+            if (lead) {
+                h = table_slot(t.keys, c, logcap, fresh);
+                const double acc = fresh ? ww[j] : __dadd_rn(t.vals[h], ww[j]);
+                t.vals[h] = vg_fold_peers(acc, t.stage, above, most);
             }
+            const unsigned fm = __ballot_sync(full, fresh);
+            if (fresh) t.used[n + __popc(fm & lt)] = (uint16_t)h;
+            n += __popc(fm);
+            if (own < 0) {
+                const unsigned om = __ballot_sync(full, lead && c == cc);
+                if (om) own = __shfl_sync(full, (int)h, __ffs(om) - 1);
+            }
+            for (unsigned m = selfm; m; m &= m - 1)
+                selfLoop = __dadd_rn(selfLoop, t.stage[__ffs(m) - 1]);
             __syncwarp();
         }
     }
-    // counter[0]: the current community's entry, if any neighbour is in it
-    double counter0 = 0.0;
-    {
-        uint32_t h = slot_hash(cc, logcap);
-        for (int probe = 0; probe < cap; probe++) {
-            const int32_t kk = keys[h];
-            if (kk == cc) {
-                counter0 = vals[h];
-                break;
-            }
-            if (kk == EMPTY) break;
-            h = (h + 1) & (cap - 1);
-        }
-    }
-    // the other communities, compacted to the front of the table: a kept slot
-    // moves to the count of kept slots before it, never past a slot not yet read
-    int nk = 0;
-    for (int base = 0; base < cap; base += 32) {
-        const int32_t kk = keys[base + lane];
-        const double vv = vals[base + lane];
-        const bool keep = kk != EMPTY && kk != cc;
-        const unsigned bm = __ballot_sync(full, keep);
-        __syncwarp();
-        if (keep) {
-            const int dst = nk + __popc(bm & ((1u << lane) - 1u));
-            keys[dst] = kk;
-            vals[dst] = vv;
-        }
-        nk += __popc(bm);
-        __syncwarp();
-    }
-    const double vd = A::ld(a.vdeg + v);
-    const double ccDeg = A::ld(a.cdeg + cc);
+    const double counter0 = own >= 0 ? t.vals[own] : 0.0;
     const double eix = __dsub_rn(counter0, selfLoop);
     const double ax = __dsub_rn(ccDeg, vd);
     double gain;
     int32_t cand;
     bool ok;
-    warp_best(a, keys, vals, 0, 32, nk, eix, vd, ax, cst, ok, gain, cand);
+    auto get = [&](int i, int32_t &k, double &w) {
+        const int h = t.used[i];
+        k = t.keys[h];
+        w = t.vals[h];
+        return h != own;
+    };
+    warp_best(a, get, 0, 32, n, eix, vd, ax, cst, ok, gain, cand);
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) t.keys[t.used[i]] = EMPTY;
     if (lane == 0) {
         int32_t ccSize, csz;
         sizes_for_rule(a, ok, cand, cc, ccSize, csz);
@@ -856,23 +878,15 @@ __device__ __forceinline__ void warp_vertex(const A &a, int32_t v, double cst, i
 template <int CAP, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, CAP <= 256 ? 4 : 1) k_sweep_warp(
     SweepArgs a, const int32_t *__restrict__ list, int64_t count) {
-    extern __shared__ unsigned char smem_raw[];
-    const int warp = threadIdx.x >> 5;
-    double *vals = reinterpret_cast<double *>(smem_raw) + (size_t)warp * CAP;
-    int32_t *keys = reinterpret_cast<int32_t *>(reinterpret_cast<double *>(smem_raw) +
-                                                (size_t)WARPS * CAP) +
-                    (size_t)warp * CAP;
-    double *stage = reinterpret_cast<double *>(reinterpret_cast<int32_t *>(
-                        reinterpret_cast<double *>(smem_raw) + (size_t)WARPS * CAP) +
-                                               (size_t)WARPS * CAP) +
-                    (size_t)warp * 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const Table t = warp_table<CAP, WARPS>(smem_raw, threadIdx.x >> 5);
     const int64_t wg = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t idx = wg; idx < count; idx += nw) {
         const int32_t v = list[idx];
         double cst;
         if (!vertex_live(a, v, cst)) continue;
-        warp_vertex(a, v, cst, keys, vals, stage);
+        warp_vertex(a, v, cst, t);
     }
 }
 
@@ -887,94 +901,88 @@ template <int NT> struct CtaShared {
     int32_t red_c[NT / 32];
     int red_ok[NT / 32];
     double self_part[NT / 32];
-    double counter0;
+    int used; // slots of the table in use
+    int own;  // the current community's slot, -1 without one
 };
 
-// vertex v (row a.rowptr[v] = e0, degree d) by the whole block of NT threads; keys/vals:
-// a shared table of at least twice `slots`, the most communities its row can hold
-// (rounded up to a power of two), stage: NT doubles
+// shared memory of a block's table of `cap` slots: vals, stage, keys, used (see Table)
+__host__ __device__ constexpr size_t cta_smem_bytes(int cap, int nt) {
+    return (size_t)cap * (sizeof(double) + sizeof(int32_t) + sizeof(uint16_t) / 2) +
+           (size_t)nt * sizeof(double);
+}
+
+// the block's table, made empty
+template <int NT>
+__device__ __forceinline__ Table cta_table(unsigned char *smem, int cap, CtaShared<NT> &sh) {
+    Table t;
+    t.vals = reinterpret_cast<double *>(smem);
+    t.stage = t.vals + cap;
+    t.keys = reinterpret_cast<int32_t *>(t.stage + NT);
+    t.used = reinterpret_cast<uint16_t *>(t.keys + cap);
+    for (int i = threadIdx.x; i < cap; i += NT) {
+        t.keys[i] = EMPTY;
+        t.vals[i] = 0.0;
+    }
+    if (threadIdx.x == 0) {
+        sh.used = 0;
+        sh.own = -1;
+    }
+    __syncthreads();
+    return t;
+}
+
+// vertex v (row a.rowptr[v] = e0, degree d) by the whole block of NT threads with a table
+// (see cta_table) of at least twice `slots`, the most communities its row can hold
 template <int NT, class A>
 __device__ __forceinline__ void cta_vertex(const A &a, int32_t v, int64_t e0, int64_t d,
-                                           int64_t slots, double cst, int32_t *keys, double *vals,
-                                           double *stage, CtaShared<NT> &sh) {
+                                           int64_t slots, double cst, const Table &t,
+                                           CtaShared<NT> &sh) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned full = 0xffffffffu;
+    const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
     const int32_t cc = A::ld(a.curr + v);
     if (a.active && !A::ld(a.active + v)) {
         if (threadIdx.x == 0) a.cw[v] = A::ld(a.frozen + v);
         return;
     }
-    int logcap = 5;
-    while (((int64_t)1 << logcap) < 2 * slots) logcap++;
-    const int64_t cap = (int64_t)1 << logcap;
-    for (int64_t s = threadIdx.x; s < cap; s += NT) {
-        keys[s] = EMPTY;
-        vals[s] = 0.0;
-    }
+    const int logcap = max(5, 32 - __clz(2 * (int)slots - 1));
+    double *stage = t.stage + warp * 32;
     double selfLoop = 0.0; // per-warp partial, in CSR order inside the warp's slices
-    __syncthreads();
     for (int64_t off = 0; off < d; off += NT) {
         const int64_t k = off + threadIdx.x;
         const bool has = k < d;
-        int32_t t = -1, c = -1;
+        int32_t u = -1, c = -1 - lane;
         double w = 0.0;
         if (has) {
-            t = a.tail[e0 + k];
+            u = a.tail[e0 + k];
             w = a.weight[e0 + k];
-            c = A::ld(a.curr + t);
+            c = A::ld(a.curr + u);
         }
-        stage[threadIdx.x] = w;
-        const unsigned peers = __match_any_sync(full, has ? c : (-1 - lane));
-        __syncwarp();
-        if (has && lane == __ffs(peers) - 1) {
-            double acc = stage[threadIdx.x];
-            const unsigned above = peers & ~((2u << lane) - 1u);
-            if (above) acc = vg_fold_above(acc, stage + (threadIdx.x & ~31), above);
-            uint32_t h = slot_hash(c, logcap);
-            for (;;) {
-                const int32_t kk = keys[h];
-                if (kk == c) break;
-                if (kk == EMPTY) {
-                    const int32_t old = atomicCAS(&keys[h], EMPTY, c);
-                    if (old == EMPTY || old == c) break;
-                }
-                h = (h + 1) & (uint32_t)(cap - 1);
-            }
-            atomicAdd(&vals[h], acc);
+        const unsigned peers = __match_any_sync(full, c);
+        const bool lead = has && (peers & lt) == 0;
+        const unsigned above = lead ? peers & ~lt & ~(1u << lane) : 0u;
+        const unsigned most = __reduce_max_sync(full, (unsigned)__popc(above));
+        const unsigned selfm = __ballot_sync(full, has && u == v);
+        if (most | selfm) {
+            stage[lane] = w;
+            __syncwarp();
         }
-        const unsigned selfm = __ballot_sync(full, has && t == v);
-        {
-            unsigned m = selfm;
-            while (m) {
-                const int b = __ffs(m) - 1;
-                selfLoop = __dadd_rn(selfLoop, stage[(threadIdx.x & ~31) + b]);
-                m &= m - 1;
-            }
+        if (lead) {
+            const double acc = vg_fold_peers(w, stage, above, most);
+            bool fresh;
+            const uint32_t h = table_slot(t.keys, c, logcap, fresh);
+            if (fresh) t.used[atomicAdd(&sh.used, 1)] = (uint16_t)h;
+            if (c == cc) sh.own = (int)h;
+            atomicAdd(&t.vals[h], acc);
         }
+        for (unsigned m = selfm; m; m &= m - 1) selfLoop = __dadd_rn(selfLoop, stage[__ffs(m) - 1]);
         __syncwarp();
     }
     if (lane == 0) sh.self_part[warp] = selfLoop;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int w = 0; w < NT / 32; w++) s = __dadd_rn(s, sh.self_part[w]);
-        sh.self_part[0] = s;
-        double c0 = 0.0;
-        uint32_t h = slot_hash(cc, logcap);
-        for (int64_t probe = 0; probe < cap; probe++) {
-            const int32_t kk = keys[h];
-            if (kk == cc) {
-                c0 = vals[h];
-                break;
-            }
-            if (kk == EMPTY) break;
-            h = (h + 1) & (uint32_t)(cap - 1);
-        }
-        sh.counter0 = c0;
-    }
-    __syncthreads();
-    const double counter0 = sh.counter0;
-    selfLoop = sh.self_part[0];
+    const int n = sh.used, own = sh.own;
+    const double counter0 = own >= 0 ? t.vals[own] : 0.0;
+    selfLoop = 0.0;
+    for (int w = 0; w < NT / 32; w++) selfLoop = __dadd_rn(selfLoop, sh.self_part[w]);
     const double vd = A::ld(a.vdeg + v);
     const double ccDeg = A::ld(a.cdeg + cc);
     const double eix = __dsub_rn(counter0, selfLoop);
@@ -982,42 +990,25 @@ __device__ __forceinline__ void cta_vertex(const A &a, int32_t v, int64_t e0, in
     double gain;
     int32_t cand;
     bool ok;
-    // the other communities, compacted to the front of the table in slot order:
-    // a kept slot moves to the count of kept slots before it, so no write lands
-    // on a slot not yet read (each group's reads end at the barrier before its
-    // writes)
-    int64_t nk = 0;
-    for (int64_t base = 0; base < cap; base += NT) {
-        const int64_t s = base + threadIdx.x;
-        const int32_t kk = s < cap ? keys[s] : EMPTY;
-        const double vv = s < cap ? vals[s] : 0.0;
-        const bool keep = kk != EMPTY && kk != cc;
-        const unsigned bm = __ballot_sync(full, keep);
-        if (lane == 0) sh.red_c[warp] = __popc(bm);
-        __syncthreads();
-        int before = 0, tot = 0;
-#pragma unroll
-        for (int w = 0; w < NT / 32; w++) {
-            const int c = sh.red_c[w];
-            before += w < warp ? c : 0;
-            tot += c;
-        }
-        if (keep) {
-            const int64_t dst = nk + before + __popc(bm & ((1u << lane) - 1u));
-            keys[dst] = kk;
-            vals[dst] = vv;
-        }
-        nk += tot;
-        __syncthreads();
-    }
-    // each warp its own slots (warp * 32 + lane + k * NT), then the warps' bests
-    warp_best(a, keys, vals, warp * 32, NT, nk, eix, vd, ax, cst, ok, gain, cand);
+    auto get = [&](int i, int32_t &k, double &w) {
+        const int h = t.used[i];
+        k = t.keys[h];
+        w = t.vals[h];
+        return h != own;
+    };
+    // each warp its own items (warp * 32 + lane + k * NT), then the warps' bests
+    warp_best(a, get, warp * 32, NT, n, eix, vd, ax, cst, ok, gain, cand);
     if (lane == 0) {
         sh.red_g[warp] = gain;
         sh.red_c[warp] = cand;
         sh.red_ok[warp] = ok;
     }
-    __syncthreads();
+    __syncthreads(); // all reads of the table are done
+    for (int i = threadIdx.x; i < n; i += NT) {
+        const int h = t.used[i];
+        t.keys[h] = EMPTY;
+        t.vals[h] = 0.0;
+    }
     if (threadIdx.x == 0) {
         for (int w = 1; w < NT / 32; w++) {
             if (better(sh.red_ok[w] != 0, sh.red_g[w], sh.red_c[w], ok, gain, cand, a.ref)) {
@@ -1029,6 +1020,8 @@ __device__ __forceinline__ void cta_vertex(const A &a, int32_t v, int64_t e0, in
         int32_t ccSize, csz;
         sizes_for_rule(a, ok, cand, cc, ccSize, csz);
         commit_vertex(a, v, cc, ccSize, vd, d > 0, counter0, ok, cand, csz);
+        sh.used = 0;
+        sh.own = -1;
     }
     __syncthreads();
 }
@@ -1039,11 +1032,9 @@ __device__ __forceinline__ void cta_vertex(const A &a, int32_t v, int64_t e0, in
 template <int CAP>
 __global__ void __launch_bounds__(CT_THREADS) k_sweep_cta(SweepArgs a, const int32_t *__restrict__ list,
                                                           int64_t count) {
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ CtaShared<CT_THREADS> sh;
-    __shared__ __align__(16) double stage[CT_THREADS];
-    double *vals = reinterpret_cast<double *>(smem_raw);
-    int32_t *keys = reinterpret_cast<int32_t *>(vals + CAP);
+    const Table t = cta_table<CT_THREADS>(smem_raw, CAP, sh);
     for (int64_t idx = blockIdx.x; idx < count; idx += gridDim.x) {
         const int32_t v = list[idx];
         const int64_t e0 = a.rowptr[v];
@@ -1051,7 +1042,7 @@ __global__ void __launch_bounds__(CT_THREADS) k_sweep_cta(SweepArgs a, const int
         if ((CAP == CT_CAP) != (d > CT_CAP_S / 2)) continue; // the other launch's row
         double cst;
         if (!vertex_live(a, v, cst)) continue;
-        cta_vertex<CT_THREADS>(a, v, e0, d, d, cst, keys, vals, stage, sh);
+        cta_vertex<CT_THREADS>(a, v, e0, d, d, cst, t, sh);
     }
 }
 
@@ -2026,8 +2017,6 @@ static void build_buckets(vg_ctx *ctx, const vg_graph *g, const int32_t *colors,
     vg_sync(ctx); // keep `fill` alive until the copy is done
 }
 
-static size_t cta_smem_bytes(int cap = CT_CAP) { return (size_t)cap * (sizeof(double) + sizeof(int32_t)); }
-
 static void configure_kernels_once() {
     static bool done = false;
     if (done) return;
@@ -2038,9 +2027,9 @@ static void configure_kernels_once() {
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)warp_smem_bytes<WT_CAP, WT_WARPS>()));
     VG_CUDA(cudaFuncSetAttribute(k_sweep_cta<CT_CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)cta_smem_bytes()));
+                                 (int)cta_smem_bytes(CT_CAP, CT_THREADS)));
     VG_CUDA(cudaFuncSetAttribute(k_sweep_cta<CT_CAP_S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)cta_smem_bytes(CT_CAP_S)));
+                                 (int)cta_smem_bytes(CT_CAP_S, CT_THREADS)));
     done = true;
 }
 
@@ -2181,76 +2170,87 @@ static void sweep_hubs(vg_ctx *ctx, const SweepArgs &a, HubPlan &hp, int64_t k,
 // launch the sweep kernels over one color bucket; with `natural` the low-degree
 // class runs over all vertices in id order instead of its list. The classes touch
 // disjoint vertices (reading the community arrays, which no sweep kernel writes, and
-// adding to the deltas with atomics), so when the first class and another one both
-// have work, the other classes run on the context's side stream alongside the first
-// (their blocks fill the SMs the first one's tail leaves idle); with profiling on,
-// every launch stays on the main stream so that each one is timed alone.
+// adding to the deltas with atomics), so each group of classes with work runs on a stream
+// of its own, the longest rows first: the table kernels hold few warps per SM and wait on
+// their loads (warp<1024>: 19 % of the warp slots, 24 % of the issue slots used on a BA
+// level 1), so one's blocks fill what another leaves. With profiling on, every launch
+// stays on the main stream so that each one is timed alone.
 static void sweep_color(vg_ctx *ctx, const SweepArgs &a, const Buckets &b, int64_t color,
                         HubPlan &hp, bool natural, int64_t nv) {
-    const int32_t *list = b.list.p;
-    auto count = [&](int cls) { return b.start[color * NCLS + cls + 1] - b.start[color * NCLS + cls]; };
-    const bool first_busy = natural ? nv > 0 : count(0) > 0;
-    bool others = false;
-    for (int cls = 1; cls < NCLS; cls++) others = others || count(cls) > 0;
-    const bool fork = first_busy && others && !ctx->profile;
-    cudaStream_t st = fork ? vg_side_fork(ctx) : ctx->stream;
-    for (int cls = 1; cls < NCLS; cls++) {
-        const int64_t s = b.start[color * NCLS + cls];
-        const int64_t n = count(cls);
-        if (n == 0) continue;
-        if (cls == NCLS - 1) { // the hubs
+    const int32_t *list = b.list.p + b.start[color * NCLS];
+    auto at = [&](int cls) { return b.start[color * NCLS + cls] - b.start[color * NCLS]; };
+    auto count = [&](int cls) { return at(cls + 1) - at(cls); };
+    constexpr int GROUPS = 5;
+    auto rows = [&](int group) { // the group's rows
+        return group == 0 ? count(1) + count(2) : group == 1 ? count(0) : group == 2 ? count(5)
+               : group == 3 ? count(4) : count(3);
+    };
+    int busy = 0;
+    for (int k = 0; k < GROUPS; k++) busy += rows(k) > 0;
+    if (busy == 0) return;
+    // group 1 takes the main stream, or the first busy one when it has no rows
+    const int sides = ctx->profile ? 0 : busy - 1;
+    int on_main = 1;
+    if (rows(1) == 0)
+        for (on_main = 0; rows(on_main) == 0;) on_main++;
+    static_assert(GROUPS - 1 <= VG_SIDE, "a side stream for every group but one");
+    vg_side_fork(ctx, sides);
+    int used = 0;
+    for (int k = 0; k < GROUPS; k++) {
+        if (rows(k) == 0) continue;
+        cudaStream_t st = sides == 0 || k == on_main ? ctx->stream : ctx->side[used++];
+        if (k == 2) {
             sweep_hubs(ctx, a, hp, color, st);
-            continue;
-        }
-        LaunchTimer lt(ctx);
-        switch (cls) {
-        case 1:
-            k_sweep_thread<true, 32, 128><<<vg_grid(ctx, n, 128, VG_T32_GRID), 128, 0, st>>>(a, list + s, n);
-            break;
-        case 2:
-            k_sweep_warp<WS_CAP, WS_WARPS><<<vg_grid(ctx, n * 32, WS_WARPS * 32, VG_WS_GRID), WS_WARPS * 32,
-                                             warp_smem_bytes<WS_CAP, WS_WARPS>(), st>>>(
-                a, list + s, n);
-            break;
-        case 3:
+        } else if (k == 3) {
+            const int64_t n = count(4);
+            if (effective_tuning(ctx).ct_max > CT_CAP_S / 2) {
+                LaunchTimer lt(ctx);
+                k_sweep_cta<CT_CAP><<<vg_grid(ctx, n * CT_THREADS, CT_THREADS, VG_CT_GRID), CT_THREADS,
+                                      cta_smem_bytes(CT_CAP, CT_THREADS), st>>>(a, list + at(4), n);
+                VG_CHECK_LAUNCH();
+            }
+            LaunchTimer lt(ctx);
+            k_sweep_cta<CT_CAP_S><<<vg_grid(ctx, n * CT_THREADS, CT_THREADS, VG_CT_GRID_S), CT_THREADS,
+                                    cta_smem_bytes(CT_CAP_S, CT_THREADS), st>>>(a, list + at(4), n);
+        } else if (k == 4) {
+            const int64_t n = count(3);
+            LaunchTimer lt(ctx);
             k_sweep_warp<WT_CAP, WT_WARPS><<<vg_grid(ctx, n * 32, WT_WARPS * 32, VG_WS_GRID), WT_WARPS * 32,
                                              warp_smem_bytes<WT_CAP, WT_WARPS>(), st>>>(
-                a, list + s, n);
-            break;
-        case 4:
-            k_sweep_cta<CT_CAP_S><<<vg_grid(ctx, n * CT_THREADS, CT_THREADS, VG_CT_GRID_S), CT_THREADS,
-                                    cta_smem_bytes(CT_CAP_S), st>>>(a, list + s, n);
-            VG_CHECK_LAUNCH();
-            if (effective_tuning(ctx).ct_max > CT_CAP_S / 2) {
-                LaunchTimer lt2(ctx);
-                k_sweep_cta<CT_CAP><<<vg_grid(ctx, n * CT_THREADS, CT_THREADS, VG_CT_GRID), CT_THREADS,
-                                      cta_smem_bytes(), st>>>(a, list + s, n);
+                a, list + at(3), n);
+        } else if (k == 0) {
+            if (count(1) > 0) {
+                const int64_t n = count(1);
+                LaunchTimer lt(ctx);
+                k_sweep_thread<true, 32, 128><<<vg_grid(ctx, n, 128, VG_T32_GRID), 128, 0, st>>>(
+                    a, list + at(1), n);
+                VG_CHECK_LAUNCH();
             }
-            break;
-        default:
-            break;
-        }
-        VG_CHECK_LAUNCH();
-    }
-    if (first_busy) {
-        LaunchTimer lt(ctx);
-        if (natural) {
+            if (count(2) > 0) {
+                const int64_t n = count(2);
+                LaunchTimer lt(ctx);
+                k_sweep_warp<WS_CAP, WS_WARPS><<<vg_grid(ctx, n * 32, WS_WARPS * 32, VG_WS_GRID),
+                                                 WS_WARPS * 32, warp_smem_bytes<WS_CAP, WS_WARPS>(), st>>>(
+                    a, list + at(2), n);
+            }
+        } else if (natural) {
+            LaunchTimer lt(ctx);
             const int64_t tiles_blocks = (nv + TILE_WARPS * 32 - 1) / (TILE_WARPS * 32);
             const int tgrid = (int)std::max<int64_t>(
                 1, std::min<int64_t>(tiles_blocks,
                                      (int64_t)effective_tuning(ctx).tile_grid * ctx->sm_count));
             if (a.ident)
-                k_sweep_tile<TMAX, true><<<tgrid, TILE_WARPS * 32, 0, ctx->stream>>>(a, nv);
+                k_sweep_tile<TMAX, true><<<tgrid, TILE_WARPS * 32, 0, st>>>(a, nv);
             else
-                k_sweep_tile<TMAX, false><<<tgrid, TILE_WARPS * 32, 0, ctx->stream>>>(a, nv);
+                k_sweep_tile<TMAX, false><<<tgrid, TILE_WARPS * 32, 0, st>>>(a, nv);
         } else {
             const int64_t n = count(0);
-            k_sweep_thread<true, TMAX, TB><<<vg_grid(ctx, n, TB, 8), TB, 0, ctx->stream>>>(
-                a, list + b.start[color * NCLS], n);
+            LaunchTimer lt(ctx);
+            k_sweep_thread<true, TMAX, TB><<<vg_grid(ctx, n, TB, 8), TB, 0, st>>>(a, list, n);
         }
         VG_CHECK_LAUNCH();
     }
-    if (fork) vg_side_join(ctx);
+    vg_side_join(ctx, sides);
 }
 
 struct PhaseTiming {

@@ -160,10 +160,8 @@ __device__ __forceinline__ void warp_short_vertex(const A &a, int32_t v, int64_t
     const unsigned peers = __match_any_sync(full, has ? c : (-1 - lane));
     __syncwarp();
     const bool leader = has && lane == __ffs(peers) - 1;
-    if (leader) {
-        const unsigned above = peers & ~((2u << lane) - 1u);
-        if (above) w = vg_fold_above(w, stage, above);
-    }
+    const unsigned above = leader ? peers & ~((2u << lane) - 1u) : 0u;
+    w = vg_fold_peers(w, stage, above, __reduce_max_sync(full, (unsigned)__popc(above)));
     double selfLoop = 0.0;
     for (unsigned m = __ballot_sync(full, has && t == v); m; m &= m - 1)
         selfLoop = __dadd_rn(selfLoop, stage[__ffs(m) - 1]);
@@ -183,19 +181,7 @@ __device__ __forceinline__ void warp_short_vertex(const A &a, int32_t v, int64_t
             cand = c;
         }
     }
-    if (__any_sync(full, ok)) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double og = __shfl_xor_sync(full, gain, o);
-            const int32_t oc = __shfl_xor_sync(full, cand, o);
-            const bool ook = oc != INT_MAX;
-            if (better(ook, og, oc, ok, gain, cand, a.ref)) {
-                gain = og;
-                cand = oc;
-                ok = true;
-            }
-        }
-    }
+    warp_argbest(ok, gain, cand, a.ref);
     if (lane == 0) {
         int32_t ccSize, csz;
         sizes_for_rule(a, ok, cand, cc, ccSize, csz);
@@ -207,8 +193,7 @@ __device__ __forceinline__ void warp_short_vertex(const A &a, int32_t v, int64_t
 // dynamic shared memory: the rows' slots and tables, one class at a time
 constexpr size_t SP_WORK_BYTES = warp_smem_bytes<WT_CAP, SP_WARPS>();
 static_assert(SP_WORK_BYTES >= sizeof(double) * SP_T * SP_THREADS &&
-                  SP_WORK_BYTES >= CT_CAP * (sizeof(double) + sizeof(int32_t)) +
-                                       sizeof(double) * SP_THREADS &&
+                  SP_WORK_BYTES >= cta_smem_bytes(CT_CAP, SP_THREADS) &&
                   SP_WORK_BYTES >= sizeof(double) * 2 * VG_FOLD_STEP * SP_WARPS,
               "every class's tables must fit the block's work area");
 
@@ -398,12 +383,14 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
                 const int d = (from - id) % n;
                 return d ? from + n - d : from;
             };
-            for (int i = first(base[ROW_BLOCK], rank, blocks); i < base[SP_CLASSES]; i += blocks) {
-                const int32_t v = __ldcg(p.list + i);
-                const int64_t e0 = a.rowptr[v], d = a.rowptr[v + 1] - e0;
-                cta_vertex<SP_THREADS>(a, v, e0, d, min(d, nv), cst,
-                                       reinterpret_cast<int32_t *>(work + CT_CAP), work,
-                                       work + CT_CAP + CT_CAP / 2, sh);
+            int i = first(base[ROW_BLOCK], rank, blocks);
+            if (i < base[SP_CLASSES]) { // uniform over the block
+                const Table t = cta_table<SP_THREADS>(smem_raw, CT_CAP, sh);
+                for (; i < base[SP_CLASSES]; i += blocks) {
+                    const int32_t v = __ldcg(p.list + i);
+                    const int64_t e0 = a.rowptr[v], d = a.rowptr[v + 1] - e0;
+                    cta_vertex<SP_THREADS>(a, v, e0, d, min(d, nv), cst, t, sh);
+                }
                 __syncthreads();
             }
             // short rows: all vertices in turn, or the color's list
@@ -421,20 +408,20 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
                 }
                 __syncthreads();
             }
-            double *vals = work + (size_t)warp * WT_CAP;
-            int32_t *keys = reinterpret_cast<int32_t *>(work + (size_t)SP_WARPS * WT_CAP) +
-                            (size_t)warp * WT_CAP;
-            double *stage = work + (size_t)SP_WARPS * (WT_CAP + WT_CAP / 2) + (size_t)warp * 32;
             if (!by_thread) {
                 for (int i = first(s0, warp_id, warps); i < s1; i += warps) {
                     const int32_t v = p.colors ? __ldcg(p.list + i) : i;
                     const int64_t e0 = a.rowptr[v];
                     const int64_t d = a.rowptr[v + 1] - e0;
-                    if (d <= SP_T) warp_short_vertex(a, v, e0, (int)d, cst, stage);
+                    if (d <= SP_T) warp_short_vertex(a, v, e0, (int)d, cst, work + warp * 32);
                 }
             }
-            for (int i = first(base[ROW_WARP], warp_id, warps); i < base[ROW_BLOCK]; i += warps)
-                warp_vertex(a, __ldcg(p.list + i), cst, keys, vals, stage);
+            if (base[ROW_WARP] < base[ROW_BLOCK]) {
+                if (!by_thread) __syncthreads(); // the stages of the short rows
+                const Table t = warp_table<WT_CAP, SP_WARPS>(smem_raw, warp);
+                for (i = first(base[ROW_WARP], warp_id, warps); i < base[ROW_BLOCK]; i += warps)
+                    warp_vertex(a, __ldcg(p.list + i), cst, t);
+            }
         }
         if (!barrier()) return;
         if (rank == 0 && tid == 0) sweep_ns += (double)(global_ns() - t0);

@@ -47,6 +47,8 @@ struct GridLimits {
     int cluster = -1, grid = 0;
 };
 
+constexpr int VG_SIDE = 4; // side streams of a context
+
 struct vg_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -65,19 +67,20 @@ struct vg_ctx {
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> event_pool;
     // sweep launch tuning (vg_ctx_set_tuning / vg_autotune); all zero = built-in defaults
     vg_tuning tune{};
-    // a second stream for kernels that may overlap the main stream's (vg_side_stream),
-    // with the events that fork it from and join it back to the main stream
-    cudaStream_t side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
+    // streams for kernels that may overlap the main stream's and one another
+    // (vg_side_fork), with the events that fork them from and join them to the main stream
+    cudaStream_t side[VG_SIDE] = {};
+    cudaEvent_t fork = nullptr, join[VG_SIDE] = {};
     // blocks the one-launch kernels of small graphs may use on the device
     GridLimits phase_limits, rebuild_limits;
 };
 
-// the context's side stream: work enqueued on the stream vg_side_fork returns, up to
-// vg_side_join, runs concurrently with the main stream's (both ordered after what the
-// main stream held at the fork; the main stream's later work waits for the join)
-cudaStream_t vg_side_fork(vg_ctx *ctx);
-void vg_side_join(vg_ctx *ctx);
+// the context's side streams: work enqueued on the first n of them between vg_side_fork and
+// vg_side_join runs concurrently with the main stream's and one another's (all ordered
+// after what the main stream held at the fork; the main stream's later work waits for the
+// join)
+void vg_side_fork(vg_ctx *ctx, int n);
+void vg_side_join(vg_ctx *ctx, int n);
 
 // stream-ordered device allocation accounted against the context budget
 void *vg_alloc(vg_ctx *ctx, size_t bytes);
@@ -241,6 +244,17 @@ __device__ __forceinline__ double vg_fold_above(double acc, const double *stage,
         if (above & (1u << (2 * j))) acc = __dadd_rn(acc, x[j].x);
         if (above & (2u << (2 * j))) acc = __dadd_rn(acc, x[j].y);
     }
+    return acc;
+}
+
+// The same when a leader's peers are few: most, warp-uniform, is the largest number of
+// peers any leader of the warp has. One read and addition per peer up to
+// VG_FOLD_FEW (rows of many communities have one or two), else the fixed 32 above.
+constexpr unsigned VG_FOLD_FEW = 6;
+__device__ __forceinline__ double vg_fold_peers(double acc, const double *stage, unsigned above,
+                                                unsigned most) {
+    if (most > VG_FOLD_FEW) return above ? vg_fold_above(acc, stage, above) : acc;
+    for (; above; above &= above - 1) acc = __dadd_rn(acc, stage[__ffs(above) - 1]);
     return acc;
 }
 
