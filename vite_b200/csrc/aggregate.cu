@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 
 namespace {
 
@@ -150,25 +151,90 @@ __global__ void k_group_copy_long(const int32_t *__restrict__ tail, const double
     }
 }
 
-// ascending bitonic sort of n2 (power of two) packed keys, by `nt` threads
-template <bool WARP>
-__device__ void bitonic(uint64_t *sk, int n2, int t, int nt) {
-    for (int k = 2; k <= n2; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = t; i < n2; i += nt) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const uint64_t a = sk[i], b = sk[ixj];
-                    const bool up = (i & k) == 0;
-                    if ((a > b) == up) {
-                        sk[i] = b;
-                        sk[ixj] = a;
-                    }
-                }
+// Ascending bitonic sort of E keys per thread by NT threads (a warp, or a block that all call
+// it), thread t ending with elements t * E .. t * E + E - 1. Exchanges inside a thread are
+// register moves, inside a warp one shuffle, and only strides of more than a warp's keys go
+// through s (NT * E keys of shared memory).
+template <int NT, int E>
+__device__ __forceinline__ void sort_keys(int32_t (&x)[E], int32_t *s) {
+    const int t = threadIdx.x & (NT - 1);
+    auto inside = [&](int j, bool up) { // stride j < E
+#pragma unroll
+        for (int e = 0; e < E; e++)
+            if (!(e & j)) {
+                const int32_t lo = min(x[e], x[e | j]), hi = max(x[e], x[e | j]);
+                x[e] = up ? lo : hi;
+                x[e | j] = up ? hi : lo;
             }
-            if (WARP) __syncwarp();
-            else __syncthreads();
+    };
+#pragma unroll
+    for (int k = 2; k < E; k <<= 1)
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+            for (int e = 0; e < E; e++)
+                if (!(e & j)) {
+                    const int32_t lo = min(x[e], x[e | j]), hi = max(x[e], x[e | j]);
+                    x[e] = (e & k) ? hi : lo;
+                    x[e | j] = (e & k) ? lo : hi;
+                }
+    for (int k = E; k <= NT * E; k <<= 1) {
+        const bool up = ((t * E) & k) == 0;
+        int m = (k >> 1) / E; // stride in threads
+        for (; m >= 32; m >>= 1) {
+#pragma unroll
+            for (int e = 0; e < E; e++) s[e * NT + t] = x[e];
+            __syncthreads();
+            const bool low = ((t & m) == 0) == up;
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                const int32_t y = s[e * NT + (t ^ m)];
+                x[e] = low ? min(x[e], y) : max(x[e], y);
+            }
+            __syncthreads();
         }
+        for (; m > 0; m >>= 1) {
+            const bool low = ((t & m) == 0) == up;
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                const int32_t y = __shfl_xor_sync(0xffffffffu, x[e], m);
+                x[e] = low ? min(x[e], y) : max(x[e], y);
+            }
+        }
+#pragma unroll
+        for (int j = E >> 1; j > 0; j >>= 1) inside(j, up);
+    }
+}
+
+// one (key, value) per lane, keys INT_MAX on idle lanes: sorted by key across the warp. The
+// key and its lane travel in one word (two when keys pass 2^26), the value once at the end.
+__device__ __forceinline__ void sort_lanes(int32_t &key, double &val, bool narrow) {
+    const unsigned full = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31;
+    unsigned from;
+    if (narrow) {
+        unsigned x = key == INT_MAX ? UINT_MAX - 31u + lane : (unsigned)key << 5 | lane;
+#pragma unroll
+        for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                const unsigned y = __shfl_xor_sync(full, x, j);
+                x = ((lane & k) == 0) == ((lane & j) == 0) ? min(x, y) : max(x, y);
+            }
+        from = x & 31u;
+    } else {
+        uint64_t x = (uint64_t)(unsigned)key << 5 | lane;
+#pragma unroll
+        for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                const uint64_t y = __shfl_xor_sync(full, x, j);
+                x = (((lane & k) == 0) == ((lane & j) == 0)) == (x < y) ? x : y;
+            }
+        from = (unsigned)x & 31u;
+    }
+    key = __shfl_sync(full, key, from);
+    val = __shfl_sync(full, val, from);
 }
 
 // One warp per segment. The segment is read in chunks of 32 entries; inside a
@@ -194,11 +260,14 @@ static_assert(2 * H_CAP >= 3 * (H_MAXU + 32) && 2 * H_CAP_S >= 3 * (H_MAXU_S + 3
 constexpr int H_WARPS = 8;
 constexpr int32_t H_EMPTY = -1;
 
+static_assert(H_MAXU_S <= 128 && H_MAXU <= 256, "warp_segment sorts at most eight keys per lane");
+constexpr int64_t NARROW_KEYS = (int64_t)1 << 26; // below, a key and a lane fit 32 bits
+
 template <int CAP, int MAXU> struct HashWarpSmem {
     int32_t keys[CAP];
     double vals[CAP];
-    uint64_t list[MAXU + 32]; // (key << 32 | slot) of the distinct keys
     alignas(16) double stage[32];
+    int32_t list[MAXU + 32]; // the distinct keys
 };
 
 // a segment's entries: read-only in a launch of their own, LIVE when this launch wrote them
@@ -211,7 +280,7 @@ template <bool LIVE, class T> __device__ __forceinline__ T seg_ld(const T *p) {
 template <bool LIVE, int CAP, int MAXU>
 __device__ __forceinline__ int warp_segment(HashWarpSmem<CAP, MAXU> &S, int64_t b, int64_t L,
                                             const int32_t *gk, const double *gw, int32_t *uk,
-                                            double *uw) {
+                                            double *uw, bool narrow) {
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
     if (L <= 32) {
@@ -226,24 +295,12 @@ __device__ __forceinline__ int warp_segment(HashWarpSmem<CAP, MAXU> &S, int64_t 
         __syncwarp();
         const bool lead = has && lane == __ffs(peers) - 1;
         double val = w;
-        const unsigned above = peers & ~((2u << lane) - 1u);
-        if (lead && above) val = vg_fold_above(val, S.stage, above);
+        const unsigned above = lead ? peers & ~((2u << lane) - 1u) : 0u;
+        const unsigned most = __reduce_max_sync(full, (unsigned)__popc(above));
+        if (lead) val = vg_fold_peers(val, S.stage, above, most);
         const int U = __popc(__ballot_sync(full, lead));
         int32_t key = lead ? k : INT_MAX;
-#pragma unroll
-        for (int k2 = 2; k2 <= 32; k2 <<= 1)
-#pragma unroll
-            for (int j = k2 >> 1; j > 0; j >>= 1) {
-                const int32_t pk = __shfl_xor_sync(full, key, j);
-                const double pv = __shfl_xor_sync(full, val, j);
-                const bool up = (lane & k2) == 0;
-                const bool low = (lane & j) == 0;
-                const bool take = (low == up) ? (pk < key) : (pk > key);
-                if (take) {
-                    key = pk;
-                    val = pv;
-                }
-            }
+        sort_lanes(key, val, narrow);
         if (lane < U) {
             uk[b + lane] = key;
             uw[b + lane] = val;
@@ -281,9 +338,11 @@ __device__ __forceinline__ int warp_segment(HashWarpSmem<CAP, MAXU> &S, int64_t 
             S.stage[lane] = w;
             const unsigned peers = __match_any_sync(full, k);
             __syncwarp();
+            const bool lead = has && (peers & lt) == 0;
+            const unsigned above = lead ? peers & ~lt & ~(1u << lane) : 0u;
+            const unsigned most = __reduce_max_sync(full, (unsigned)__popc(above));
             bool fresh = false;
-            int slot = 0;
-            if (has && lane == __ffs(peers) - 1) {
+            if (lead) {
                 uint32_t h = ((uint32_t)k * 2654435761u) >> (32 - logcap);
                 for (;;) {
                     const int32_t kk = S.keys[h];
@@ -298,14 +357,11 @@ __device__ __forceinline__ int warp_segment(HashWarpSmem<CAP, MAXU> &S, int64_t 
                     }
                     h = (h + 1) & (uint32_t)(cap - 1);
                 }
-                slot = (int)h;
-                double acc = fresh ? w : __dadd_rn(S.vals[h], w);
-                const unsigned above = peers & ~((2u << lane) - 1u);
-                if (above) acc = vg_fold_above(acc, S.stage, above);
-                S.vals[h] = acc;
+                const double acc = fresh ? w : __dadd_rn(S.vals[h], w);
+                S.vals[h] = vg_fold_peers(acc, S.stage, above, most);
             }
             const unsigned fm = __ballot_sync(full, fresh);
-            if (fresh) S.list[U + __popc(fm & lt)] = ((uint64_t)(uint32_t)k << 32) | (uint32_t)slot;
+            if (fresh) S.list[U + __popc(fm & lt)] = k;
             U += __popc(fm);
             __syncwarp();
             if (U > MAXU) { // too many distinct keys for the table: the next tier
@@ -318,49 +374,50 @@ __device__ __forceinline__ int warp_segment(HashWarpSmem<CAP, MAXU> &S, int64_t 
         __syncwarp();
         return -1;
     }
+    auto sum_of = [&](int32_t k) { // k is in the table
+        uint32_t h = ((uint32_t)k * 2654435761u) >> (32 - logcap);
+        while (S.keys[h] != k) h = (h + 1) & (uint32_t)(cap - 1);
+        return S.vals[h];
+    };
     if (U <= 32) {
-        // bitonic network across the lanes on (key, sum)
-        int32_t key = INT_MAX;
-        double val = 0.0;
-        if (lane < U) {
-            const uint64_t e = S.list[lane];
-            key = (int32_t)(e >> 32);
-            val = S.vals[(uint32_t)e];
-        }
-#pragma unroll
-        for (int k2 = 2; k2 <= 32; k2 <<= 1)
-#pragma unroll
-            for (int j = k2 >> 1; j > 0; j >>= 1) {
-                const int32_t pk = __shfl_xor_sync(full, key, j);
-                const double pv = __shfl_xor_sync(full, val, j);
-                const bool up = (lane & k2) == 0;
-                const bool low = (lane & j) == 0;
-                // the lower lane of an ascending pair keeps the minimum
-                const bool take = (low == up) ? (pk < key) : (pk > key);
-                if (take) {
-                    key = pk;
-                    val = pv;
-                }
-            }
+        int32_t key = lane < U ? S.list[lane] : INT_MAX;
+        double val = lane < U ? sum_of(key) : 0.0;
+        sort_lanes(key, val, narrow);
         if (lane < U) {
             uk[b + lane] = key;
             uw[b + lane] = val;
         }
     } else {
-        int n2 = 64;
-        while (n2 < U) n2 <<= 1;
-        for (int i = U + lane; i < n2; i += 32) S.list[i] = ~0ULL;
-        __syncwarp();
-        bitonic<true>(S.list, n2, lane, 32);
-        for (int i = lane; i < U; i += 32) {
-            const uint64_t e = S.list[i];
-            uk[b + i] = (int32_t)(e >> 32);
-            uw[b + i] = S.vals[(uint32_t)e];
-        }
+        // two, four or eight keys per lane, their sums looked up again
+        auto sorted = [&](auto per) {
+            constexpr int E = decltype(per)::value;
+            int32_t x[E];
+#pragma unroll
+            for (int e = 0; e < E; e++) x[e] = e * 32 + lane < U ? S.list[e * 32 + lane] : INT_MAX;
+            sort_keys<32, E>(x, nullptr);
+#pragma unroll
+            for (int e = 0; e < E; e++) {
+                if (lane * E + e >= U) break;
+                uk[b + lane * E + e] = x[e];
+                uw[b + lane * E + e] = sum_of(x[e]);
+            }
+        };
+        if (U <= 64) sorted(std::integral_constant<int, 2>{});
+        else if (MAXU <= 128 || U <= 128) sorted(std::integral_constant<int, 4>{});
+        else sorted(std::integral_constant<int, 8>{});
     }
     __syncwarp();
     return U;
 }
+
+// where a tier sends the segments it cannot hold, or that are too long for a warp (a warp
+// takes some 200 cycles per 32 entries): lists by length for the two block tables, a flag
+// (the next tier, or the sorted path) for the others and without lists
+constexpr int64_t BLOCK_SMALL_L = 8192, BLOCK_LARGE_L = 131072;
+struct BlockRows {
+    int32_t *rows[2] = {nullptr, nullptr};
+    int32_t *count = nullptr; // 2
+};
 
 // rows: null for every segment 0..nc-1, else the segments rows[0 .. *nrows)
 template <int CAP, int MAXU>
@@ -368,7 +425,7 @@ __global__ void __launch_bounds__(H_WARPS * 32) k_rows_hash(
     int64_t nc, const int32_t *__restrict__ rows, const int64_t *__restrict__ nrows,
     const int64_t *__restrict__ rstart, const int32_t *__restrict__ gk,
     const double *__restrict__ gw, int32_t *__restrict__ uk, double *__restrict__ uw,
-    int64_t *__restrict__ ucount, int32_t *__restrict__ flag) {
+    int64_t *__restrict__ ucount, int32_t *__restrict__ flag, BlockRows next, bool narrow) {
     extern __shared__ unsigned char hsm_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     HashWarpSmem<CAP, MAXU> &S = reinterpret_cast<HashWarpSmem<CAP, MAXU> *>(hsm_raw)[warp];
@@ -379,12 +436,224 @@ __global__ void __launch_bounds__(H_WARPS * 32) k_rows_hash(
         const int64_t row = rows ? rows[idx] : idx;
         const int64_t b = rstart[row];
         const int64_t L = rstart[row + 1] - b;
-        const int U = warp_segment<false>(S, b, L, gk, gw, uk, uw);
+        const int U = L > BLOCK_SMALL_L ? -1 : warp_segment<false>(S, b, L, gk, gw, uk, uw, narrow);
         if (lane == 0) {
             if (U >= 0) ucount[row] = U;
-            flag[row] = U < 0;
+            const int to = U >= 0 || !next.rows[0] ? -1 : L <= BLOCK_SMALL_L ? 0 : L <= BLOCK_LARGE_L ? 1 : -1;
+            if (to >= 0) next.rows[to][atomicAdd(next.count + to, 1)] = (int32_t)row;
+            flag[row] = U < 0 && to < 0;
         }
         __syncwarp();
+    }
+}
+
+// One segment by a whole block, for those with more distinct keys than a warp's table takes.
+// Integral weights (exact in any order): the warps take 32-entry chunks in turn and add into
+// the table. Real weights: tiles of TILE entries are dealt out to the warps by a hash of the
+// key, in segment order, and each warp folds the keys of its share, so every key's sum is one
+// left fold. The distinct keys are sorted in shared memory.
+template <int NT, int CAP_, int MAXU_> struct BlockTable {
+    static constexpr int THREADS = NT, WARPS = NT / 32, CAP = CAP_, MAXU = MAXU_;
+    static constexpr int CHUNKS = 8; // 32-entry chunks of a tile per warp
+    static constexpr int TILE = 32 * CHUNKS * WARPS;
+    // every warp can add a chunk of keys after the count has passed MAXU
+    static constexpr int LIST = MAXU + 32 * WARPS;
+    static_assert(CAP > LIST, "the table never fills");
+    static_assert(MAXU == 8 * NT && TILE >= MAXU, "eight keys per thread, sorted through tile_k");
+    double vals[CAP];
+    double tile_w[TILE]; // a tile's entries by share, in segment order
+    alignas(16) double stage[WARPS][32];
+    int32_t list[LIST]; // the distinct keys
+    int32_t keys[CAP];
+    int32_t tile_k[TILE];
+    int32_t count[WARPS * WARPS + 1]; // [share][warp]
+    int used;
+};
+// Two sizes: 42 KB and five blocks per SM up to 1,024 distinct keys, and 168 KB up to 4,096.
+using BlockTableSmall = BlockTable<128, 2048, 1024>;
+using BlockTableLarge = BlockTable<512, 8192, 4096>;
+
+// entries [s0, s0 + L) of gk/gw; returns the number of distinct keys, or -1 when there are
+// more than MAXU. The whole block calls it and gets the same answer.
+template <bool LIVE, class Table>
+__device__ __forceinline__ int block_segment(Table &T, int64_t s0, int64_t L, bool integral,
+                                             const int32_t *gk, const double *gw, int32_t *uk,
+                                             double *uw) {
+    constexpr int NT = Table::THREADS, NW = Table::WARPS, CHUNKS = Table::CHUNKS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
+    int logcap = 6;
+    while ((1 << logcap) < 2 * L && (1 << logcap) < Table::CAP) logcap++;
+    const uint32_t mask = (1u << logcap) - 1u;
+    __syncthreads(); // the table of the segment before
+    for (int i = tid; i <= (int)mask; i += NT) {
+        T.keys[i] = H_EMPTY;
+        T.vals[i] = 0.0;
+    }
+    if (tid == 0) T.used = 0;
+    __syncthreads();
+    double *stage = T.stage[warp];
+    bool over = false;
+    // one chunk's entries, an entry per lane (k < 0: none), onto the table
+    auto add_chunk = [&](int32_t k, double w) {
+        const unsigned peers = __match_any_sync(full, k >= 0 ? k : -2 - lane);
+        const bool lead = k >= 0 && (peers & lt) == 0;
+        const unsigned above = lead ? peers & ~lt & ~(1u << lane) : 0u;
+        const unsigned most = __reduce_max_sync(full, (unsigned)__popc(above));
+        if (most) {
+            stage[lane] = w;
+            __syncwarp();
+        }
+        if (lead) {
+            uint32_t h = ((uint32_t)k * 2654435761u) >> (32 - logcap);
+            bool fresh = false;
+            for (;;) {
+                const int32_t kk = *(volatile int32_t *)&T.keys[h];
+                if (kk == k) break;
+                if (kk == H_EMPTY) {
+                    const int32_t old = atomicCAS(&T.keys[h], H_EMPTY, k);
+                    if (old == H_EMPTY) {
+                        fresh = true;
+                        break;
+                    }
+                    if (old == k) break;
+                }
+                h = (h + 1) & mask;
+            }
+            if (integral) {
+                atomicAdd(&T.vals[h], vg_fold_peers(w, stage, above, most));
+            } else {
+                const double acc = fresh ? w : __dadd_rn(T.vals[h], w);
+                T.vals[h] = vg_fold_peers(acc, stage, above, most);
+            }
+            if (fresh) T.list[atomicAdd(&T.used, 1)] = k;
+        }
+        __syncwarp();
+        return __any_sync(full, *(volatile int *)&T.used > Table::MAXU) != 0;
+    };
+    if (integral) {
+        // four chunks' entries loaded together
+        for (int64_t base = warp * 32; base < L && !over; base += 4 * NT) {
+            int32_t kq[4];
+            double wq[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int64_t i = base + j * NT + lane;
+                kq[j] = i < L ? seg_ld<LIVE>(gk + s0 + i) : -1;
+                wq[j] = i < L ? seg_ld<LIVE>(gw + s0 + i) : 0.0;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (!over && base + j * NT < L) over = add_chunk(kq[j], wq[j]);
+        }
+    } else {
+        for (int64_t base = 0; base < L; base += Table::TILE) { // uniform over the block
+            int32_t kq[CHUNKS], at[CHUNKS];
+            double wq[CHUNKS];
+            if (lane < NW) T.count[lane * NW + warp] = 0;
+            __syncwarp();
+            const int64_t i0 = base + warp * (32 * CHUNKS) + lane;
+#pragma unroll
+            for (int j = 0; j < CHUNKS; j++) {
+                const int64_t i = i0 + j * 32;
+                kq[j] = i < L ? seg_ld<LIVE>(gk + s0 + i) : -1;
+                wq[j] = i < L ? seg_ld<LIVE>(gw + s0 + i) : 0.0;
+            }
+            auto share_of = [](int32_t k) { return (int)((((uint32_t)k * 2654435761u) >> 8) & (NW - 1)); };
+#pragma unroll
+            for (int j = 0; j < CHUNKS; j++) {
+                // share of the key, and the entry's rank among this warp's of the share
+                const int share = kq[j] >= 0 ? share_of(kq[j]) : NW;
+                const unsigned peers = __match_any_sync(full, share);
+                int32_t *c = T.count + share * NW + warp;
+                if (share < NW) at[j] = *c + __popc(peers & lt);
+                __syncwarp();
+                if (share < NW && (peers & lt) == 0) *c += __popc(peers);
+                __syncwarp();
+            }
+            __syncthreads();
+            if (warp == 0) { // exclusive prefix over [share][warp]
+                constexpr int PER = (NW * NW + 31) / 32;
+                int64_t mine = 0, total;
+#pragma unroll
+                for (int t = 0; t < PER; t++)
+                    if (lane * PER + t < NW * NW) mine += T.count[lane * PER + t];
+                int32_t run = (int32_t)warp_excl(mine, total);
+#pragma unroll
+                for (int t = 0; t < PER; t++)
+                    if (lane * PER + t < NW * NW) {
+                        const int32_t y = T.count[lane * PER + t];
+                        T.count[lane * PER + t] = run;
+                        run += y;
+                    }
+                if (lane == 0) T.count[NW * NW] = (int32_t)total;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < CHUNKS; j++) {
+                if (kq[j] < 0) continue;
+                const int o = T.count[share_of(kq[j]) * NW + warp] + at[j];
+                T.tile_k[o] = kq[j];
+                T.tile_w[o] = wq[j];
+            }
+            __syncthreads();
+            const int c0 = T.count[warp * NW], c1 = T.count[(warp + 1) * NW];
+            for (int c = c0; c < c1 && !over; c += 32) {
+                const bool has = c + lane < c1;
+                over = add_chunk(has ? T.tile_k[c + lane] : -1, has ? T.tile_w[c + lane] : 0.0);
+            }
+            if (__syncthreads_or(over)) break;
+        }
+    }
+    __syncthreads();
+    const int U = T.used;
+    if (U > Table::MAXU) return -1;
+    auto sorted = [&](auto per) {
+        constexpr int E = decltype(per)::value;
+        int32_t x[E];
+#pragma unroll
+        for (int e = 0; e < E; e++) x[e] = e * NT + tid < U ? T.list[e * NT + tid] : INT_MAX;
+        sort_keys<NT, E>(x, T.tile_k);
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const int i = tid * E + e;
+            if (i >= U) break;
+            uint32_t h = ((uint32_t)x[e] * 2654435761u) >> (32 - logcap);
+            while (T.keys[h] != x[e]) h = (h + 1) & mask;
+            uk[s0 + i] = x[e];
+            uw[s0 + i] = T.vals[h];
+        }
+    };
+    if (U <= 2 * NT) sorted(std::integral_constant<int, 2>{});
+    else if (U <= 4 * NT) sorted(std::integral_constant<int, 4>{});
+    else sorted(std::integral_constant<int, 8>{});
+    return U;
+}
+
+// Rows in[0 .. *n_in) by a block each; those a table of this size cannot hold go to out (or,
+// without one, are flagged for the sorted path).
+template <class Table>
+__global__ void __launch_bounds__(Table::THREADS) k_rows_block(
+    const int32_t *__restrict__ in, const int32_t *__restrict__ n_in,
+    const int64_t *__restrict__ rstart, const int32_t *__restrict__ gk,
+    const double *__restrict__ gw, int32_t *__restrict__ uk, double *__restrict__ uw,
+    int64_t *__restrict__ ucount, int integral, int32_t *__restrict__ out,
+    int32_t *__restrict__ n_out, int32_t *__restrict__ flag) {
+    extern __shared__ unsigned char hsm_raw[];
+    Table &T = *reinterpret_cast<Table *>(hsm_raw);
+    const int n = *n_in;
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+        const int32_t row = in[i];
+        const int64_t s0 = rstart[row], L = rstart[row + 1] - s0;
+        const int U = block_segment<false>(T, s0, L, integral != 0, gk, gw, uk, uw);
+        if (threadIdx.x == 0) {
+            if (U >= 0)
+                ucount[row] = U;
+            else if (out)
+                out[atomicAdd(n_out, 1)] = row;
+            else
+                flag[row] = 1;
+        }
     }
 }
 
@@ -681,8 +950,15 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
         VG_CUDA(cudaFuncSetAttribute(k_rows_hash<H_CAP, H_MAXU>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)(H_WARPS * sizeof(SmemL))));
+        VG_CUDA(cudaFuncSetAttribute(k_rows_block<BlockTableSmall>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(BlockTableSmall)));
+        VG_CUDA(cudaFuncSetAttribute(k_rows_block<BlockTableLarge>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(BlockTableLarge)));
         configured = true;
     }
+    const bool narrow = nc <= NARROW_KEYS;
     int kbits = 1;
     while (kbits < 31 && ((int64_t)1 << kbits) < nc) kbits++;
     // 1. vertices grouped by new row, reference order inside a row
@@ -750,13 +1026,19 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
           k_rows_hash<H_CAP_S, H_MAXU_S>
               <<<vg_grid(ctx, nc * 32, H_WARPS * 32, VG_RH_GRID_S), H_WARPS * 32,
                  H_WARPS * sizeof(SmemS), ctx->stream>>>(nc, nullptr, nullptr, rstart.p, gk.p, gw.p,
-                                                         uk.p, uw.p, ucount.p, flag.p); }
+                                                         uk.p, uw.p, ucount.p, flag.p,
+                                                         BlockRows{}, narrow); }
         VG_CHECK_LAUNCH();
         {
             // the segments that overflowed the small table, with the large one (their
             // count stays on the device; the grid covers every segment's warp)
             DevBuf<int64_t> fpos(ctx, nc), fcount(ctx, 1);
-            DevBuf<int32_t> frows(ctx, nc);
+            DevBuf<int32_t> frows(ctx, nc), brows(ctx, 2 * nc + 2);
+            BlockRows next;
+            next.rows[0] = brows.p;
+            next.rows[1] = brows.p + nc;
+            next.count = brows.p + 2 * nc;
+            VG_CUDA(cudaMemsetAsync(next.count, 0, 2 * sizeof(int32_t), ctx->stream));
             vg_scan_i32_async(ctx, flag.p, fpos.p, nc, fcount.p);
             { LaunchTimer lt(ctx);
               k_list_flagged<<<vg_grid(ctx, nc, 256), 256, 0, ctx->stream>>>(nc, flag.p, fpos.p,
@@ -766,7 +1048,23 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
               k_rows_hash<H_CAP, H_MAXU>
                   <<<vg_grid(ctx, nc * 32, H_WARPS * 32, VG_RH_GRID), H_WARPS * 32,
                      H_WARPS * sizeof(SmemL), ctx->stream>>>(nc, frows.p, fcount.p, rstart.p, gk.p,
-                                                             gw.p, uk.p, uw.p, ucount.p, flag.p); }
+                                                             gw.p, uk.p, uw.p, ucount.p, flag.p,
+                                                             next, narrow); }
+            VG_CHECK_LAUNCH();
+            // more distinct keys: a block per segment, in two table sizes
+            const int bgrid = (int)std::min<int64_t>(nc, 5LL * ctx->sm_count);
+            { LaunchTimer lt(ctx);
+              k_rows_block<BlockTableSmall>
+                  <<<bgrid, BlockTableSmall::THREADS, sizeof(BlockTableSmall), ctx->stream>>>(
+                      next.rows[0], next.count, rstart.p, gk.p, gw.p, uk.p, uw.p, ucount.p, integral,
+                      next.rows[1], next.count + 1, nullptr); }
+            VG_CHECK_LAUNCH();
+            { LaunchTimer lt(ctx);
+              k_rows_block<BlockTableLarge>
+                  <<<(int)std::min<int64_t>(nc, ctx->sm_count), BlockTableLarge::THREADS,
+                     sizeof(BlockTableLarge), ctx->stream>>>(
+                      next.rows[1], next.count + 1, rstart.p, gk.p, gw.p, uk.p, uw.p, ucount.p,
+                      integral, nullptr, nullptr, flag.p); }
             VG_CHECK_LAUNCH();
         }
         // segments with more than H_MAXU distinct keys: one global stable sort. Their

@@ -31,25 +31,12 @@
 #endif
 constexpr int64_t RS_MAX_NV = VG_RS_MAX_NV;
 constexpr int64_t RS_MAX_NE = VG_RS_MAX_NE;
-constexpr int RS_BIG_L = 1024;    // segments longer than this go to a whole block
-constexpr int RS_BIG_CAP = 8192;  // slots of the block's table
-constexpr int RS_BIG_MAXU = 4096; // distinct keys it may hold
-constexpr int RS_TILE = 4096;     // entries a block deals out to its warps at a time
-constexpr int RS_TILE_CHUNKS = RS_TILE / (32 * GS_WARPS); // 32-entry chunks per warp
-static_assert(GS_WARPS == 16, "the deal of a tile scans 16 x 16 counts with one warp");
+static_assert(RS_MAX_NV <= NARROW_KEYS, "warp_segment is told so");
+constexpr int RS_BIG_L = 1024; // segments longer than this go to a whole block
 
 using SmallWarpTable = HashWarpSmem<H_CAP, H_MAXU>;
-struct SmallBlockTable {
-    int32_t keys[RS_BIG_CAP];
-    double vals[RS_BIG_CAP];
-    uint64_t list[RS_BIG_CAP]; // (key << 32 | slot) of the distinct keys
-    alignas(16) double stage[GS_WARPS][32];
-    double tile_w[RS_TILE]; // a tile's entries by share, in segment order
-    int32_t tile_k[RS_TILE];
-    int32_t count[GS_WARPS * GS_WARPS + 1]; // [share][warp]
-};
-static_assert(RS_BIG_CAP > RS_BIG_MAXU + 32 * GS_WARPS,
-              "every warp can add a chunk of keys after the count has passed the limit");
+using SmallBlockTable = BlockTableLarge;
+static_assert(SmallBlockTable::THREADS == GS_THREADS, "the block table's warps are the block's");
 constexpr size_t RS_SMEM_BYTES = sizeof(SmallBlockTable) > GS_WARPS * sizeof(SmallWarpTable)
                                      ? sizeof(SmallBlockTable)
                                      : GS_WARPS * sizeof(SmallWarpTable);
@@ -93,7 +80,7 @@ __device__ __forceinline__ int64_t block_prefix_of(const int64_t *part, int n, i
 template <bool GRID>
 __global__ void __launch_bounds__(GS_THREADS, 1) k_rebuild_small(SmallRebuild p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_dead, s_u;
+    __shared__ int s_dead;
     __shared__ int64_t s_w[GS_WARPS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned full = 0xffffffffu;
@@ -325,7 +312,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_rebuild_small(SmallRebuild p)
         for (int64_t r = warp_id; r < nc; r += warps) {
             const int64_t L = __ldcg(p.ecount + r);
             if (L > RS_BIG_L) continue;
-            const int U = warp_segment<true>(S, __ldcg(p.rstart + r), L, p.gk, p.gw, p.uk, p.uw);
+            const int U = warp_segment<true>(S, __ldcg(p.rstart + r), L, p.gk, p.gw, p.uk, p.uw, true);
             if (lane == 0) {
                 if (U >= 0)
                     p.ucount[r] = U;
@@ -336,137 +323,18 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_rebuild_small(SmallRebuild p)
         }
     }
     if (!barrier()) return;
-    // The other segments, a block each. Integral weights (exact in any order): the warps
-    // take chunks in turn and add into the table. Real weights: tiles of RS_TILE entries are
-    // dealt out by a hash of the key, in order, and each warp folds the keys of its share,
-    // so every key's sum is one left fold.
+    // the other segments, a block each
     const int nlong = __ldcg(p.ctl + RS_LONG_SEGS);
     for (int b = rank; b < nlong; b += blocks) { // uniform over the block
-        SmallBlockTable &T = *reinterpret_cast<SmallBlockTable *>(smem_raw);
         const int64_t r = __ldcg(p.longlist + b);
-        const int64_t s0 = __ldcg(p.rstart + r), L = __ldcg(p.ecount + r);
-        int logcap = 6;
-        while ((1 << logcap) < 2 * L && (1 << logcap) < RS_BIG_CAP) logcap++;
-        const int cap = 1 << logcap;
-        __syncthreads();
-        for (int i = tid; i < cap; i += GS_THREADS) {
-            T.keys[i] = H_EMPTY;
-            T.vals[i] = 0.0;
-        }
-        if (tid == 0) s_u = 0;
-        __syncthreads();
-        double *stage = T.stage[warp];
-        bool over = false;
-        // one chunk's entries, an entry per lane (k < 0: none), onto the table
-        auto add_chunk = [&](int32_t k, double w) {
-            stage[lane] = w;
-            const unsigned peers = __match_any_sync(full, k >= 0 ? k : -2 - lane);
-            __syncwarp();
-            if (k >= 0 && lane == __ffs(peers) - 1) {
-                uint32_t h = ((uint32_t)k * 2654435761u) >> (32 - logcap);
-                bool fresh = false;
-                for (;;) {
-                    const int32_t kk = *(volatile int32_t *)&T.keys[h];
-                    if (kk == k) break;
-                    if (kk == H_EMPTY) {
-                        const int32_t old = atomicCAS(&T.keys[h], H_EMPTY, k);
-                        if (old == H_EMPTY) {
-                            fresh = true;
-                            break;
-                        }
-                        if (old == k) break;
-                    }
-                    h = (h + 1) & (uint32_t)(cap - 1);
-                }
-                const unsigned above = peers & ~((2u << lane) - 1u);
-                if (p.integral) {
-                    if (above) w = vg_fold_above(w, stage, above);
-                    atomicAdd(&T.vals[h], w);
-                } else {
-                    double acc = fresh ? w : __dadd_rn(T.vals[h], w);
-                    if (above) acc = vg_fold_above(acc, stage, above);
-                    T.vals[h] = acc;
-                }
-                if (fresh) T.list[atomicAdd(&s_u, 1)] = ((uint64_t)(uint32_t)k << 32) | h;
-            }
-            __syncwarp();
-            return __any_sync(full, *(volatile int *)&s_u > RS_BIG_MAXU);
-        };
-        if (p.integral) {
-            for (int64_t base = warp * 32; base < L && !over; base += 32 * GS_WARPS) {
-                const int64_t i = base + lane;
-                over = add_chunk(i < L ? __ldcg(p.gk + s0 + i) : -1, i < L ? __ldcg(p.gw + s0 + i) : 0.0);
-            }
-        } else {
-            for (int64_t base = 0; base < L; base += RS_TILE) { // uniform over the block
-                int32_t kq[RS_TILE_CHUNKS], at[RS_TILE_CHUNKS];
-                double wq[RS_TILE_CHUNKS];
-                if (lane < GS_WARPS) T.count[lane * GS_WARPS + warp] = 0;
-                __syncwarp();
-                const int64_t i0 = base + warp * (RS_TILE / GS_WARPS) + lane;
-#pragma unroll
-                for (int j = 0; j < RS_TILE_CHUNKS; j++) {
-                    const int64_t i = i0 + j * 32;
-                    kq[j] = i < L ? __ldcg(p.gk + s0 + i) : -1;
-                    wq[j] = i < L ? __ldcg(p.gw + s0 + i) : 0.0;
-                }
-#pragma unroll
-                for (int j = 0; j < RS_TILE_CHUNKS; j++) {
-                    // share of the key, and the entry's rank among this warp's of the share
-                    const int share = kq[j] >= 0 ? (int)((((uint32_t)kq[j] * 2654435761u) >> 8) & (GS_WARPS - 1))
-                                                 : GS_WARPS;
-                    const unsigned peers = __match_any_sync(full, share);
-                    int32_t *c = T.count + share * GS_WARPS + warp;
-                    if (share < GS_WARPS) at[j] = *c + __popc(peers & ((1u << lane) - 1u));
-                    __syncwarp();
-                    if (share < GS_WARPS && lane == __ffs(peers) - 1) *c += __popc(peers);
-                    __syncwarp();
-                }
-                __syncthreads();
-                if (warp == 0) { // exclusive prefix over [share][warp]
-                    int64_t mine = 0, total;
-                    for (int t = 0; t < 8; t++) mine += T.count[lane * 8 + t];
-                    int32_t run = (int32_t)warp_excl(mine, total);
-                    for (int t = 0; t < 8; t++) {
-                        const int32_t y = T.count[lane * 8 + t];
-                        T.count[lane * 8 + t] = run;
-                        run += y;
-                    }
-                    if (lane == 31) T.count[GS_WARPS * GS_WARPS] = run;
-                }
-                __syncthreads();
-#pragma unroll
-                for (int j = 0; j < RS_TILE_CHUNKS; j++) {
-                    if (kq[j] < 0) continue;
-                    const int share = (int)((((uint32_t)kq[j] * 2654435761u) >> 8) & (GS_WARPS - 1));
-                    const int o = T.count[share * GS_WARPS + warp] + at[j];
-                    T.tile_k[o] = kq[j];
-                    T.tile_w[o] = wq[j];
-                }
-                __syncthreads();
-                const int c0 = T.count[warp * GS_WARPS], c1 = T.count[(warp + 1) * GS_WARPS];
-                for (int c = c0; c < c1 && !over; c += 32) {
-                    const bool has = c + lane < c1;
-                    over = add_chunk(has ? T.tile_k[c + lane] : -1, has ? T.tile_w[c + lane] : 0.0);
-                }
-                if (__syncthreads_or(over)) break;
-            }
-        }
-        if (over && lane == 0) p.ctl[RS_REFUSED] = 1;
-        __syncthreads();
-        const int U = s_u;
-        if (U <= RS_BIG_MAXU) {
-            int n2 = 64;
-            while (n2 < U) n2 <<= 1;
-            for (int i = U + tid; i < n2; i += GS_THREADS) T.list[i] = ~0ULL;
-            __syncthreads();
-            bitonic<false>(T.list, n2, tid, GS_THREADS);
-            for (int i = tid; i < U; i += GS_THREADS) {
-                const uint64_t e = T.list[i];
-                p.uk[s0 + i] = (int32_t)(e >> 32);
-                p.uw[s0 + i] = T.vals[(uint32_t)e];
-            }
-            if (tid == 0) p.ucount[r] = U;
+        const int U = block_segment<true>(*reinterpret_cast<SmallBlockTable *>(smem_raw),
+                                          __ldcg(p.rstart + r), __ldcg(p.ecount + r), p.integral,
+                                          p.gk, p.gw, p.uk, p.uw);
+        if (tid == 0) {
+            if (U >= 0)
+                p.ucount[r] = U;
+            else
+                p.ctl[RS_REFUSED] = 1;
         }
     }
     if (!barrier()) return;
