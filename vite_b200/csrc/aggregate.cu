@@ -841,7 +841,7 @@ __global__ void k_big_fold_seq(
         const int64_t i0 = headpos[h], i1 = h + 1 < nheads ? headpos[h + 1] : m;
         const double *__restrict__ sw = gw + rstart[big_row[K[i0] >> kbits]]; // segment's weights
         const uint32_t *__restrict__ rv = V + i0;
-        const double s = vg_warp_ordered_fold(
+        const double s = vg_warp_fold(
             i1 - i0, [sw, rv](int64_t j) { return sw[rv[j]]; }, stage[threadIdx.x >> 5], 0.0, true);
         if ((threadIdx.x & 31) == 0) { // the run's key and place read again: fewer live values
             const uint64_t k = K[i0];

@@ -1479,7 +1479,7 @@ __global__ void __launch_bounds__(DEG_LONG_WARPS * 32)
         } else {
             // real weights: one left fold in CSR order (lane 0's result)
             const double *__restrict__ rw = w + E0;
-            sum = vg_warp_ordered_fold(E1 - E0, [rw](int64_t j) { return rw[j]; },
+            sum = vg_warp_fold(E1 - E0, [rw](int64_t j) { return rw[j]; },
                                        stage[threadIdx.x >> 5], 0.0, false);
         }
         if (lane == 0) vdeg[v] = sum;

@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
             s = warp_tree(s);
         } else {
             const double *__restrict__ w = a.weight + E0;
-            s = vg_warp_ordered_fold(E1 - E0, [w](int64_t j) { return w[j]; },
+            s = vg_warp_fold(E1 - E0, [w](int64_t j) { return w[j]; },
                                      work + (size_t)warp * 2 * VG_FOLD_STEP, 0.0, false);
         }
         if (lane == 0) p.vdeg[v] = s;
