@@ -85,6 +85,140 @@ __global__ void k_color_round(const int64_t *__restrict__ rowptr, const int32_t 
     if ((threadIdx.x & 31) == 0 && mine) atomicAdd(ncolored, mine);
 }
 
+// The round's hashes of every vertex, P (4 or 8) words each, so that a round reads a
+// neighbour's in one 16- or 32-byte load instead of computing them once per entry (the
+// hashes were two thirds of a round's instructions).
+template <int P>
+__global__ void k_color_hash(int64_t nv, int nHash, uint32_t seed, const int32_t *__restrict__ ref,
+                             uint32_t *__restrict__ hash) {
+    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < nv;
+         v += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t r = (uint32_t)vg_rid(ref, (int32_t)v);
+        uint4 h[P / 4];
+#pragma unroll
+        for (int q = 0; q < P / 4; q++) {
+            auto one = [&](int t) { // hashes past nHash are never looked at
+                return t < nHash ? color_hash(r, (uint32_t)((int64_t)seed + 1043 * (int64_t)t)) : 0u;
+            };
+            h[q] = make_uint4(one(4 * q), one(4 * q + 1), one(4 * q + 2), one(4 * q + 3));
+        }
+#pragma unroll
+        for (int q = 0; q < P / 4; q++) reinterpret_cast<uint4 *>(hash)[v * (P / 4) + q] = h[q];
+    }
+}
+
+// k_color_round with the hashes read from k_color_hash's array. A warp takes 32 vertices, whose
+// rows are one range of entries, and reads the tails of a range of up to CR_STAGE entries
+// together into shared memory (a lane per row touches a line per lane and load). A vertex
+// stops once every hash has a smaller and a larger neighbour. FIRST: no vertex has a color of
+// an earlier round, so the neighbours' colors are not read.
+constexpr int CR_WARPS = 8, CR_STAGE = 768;
+template <int P, bool FIRST>
+__global__ void __launch_bounds__(CR_WARPS * 32) k_color_round_hashed(
+    const int64_t *__restrict__ rowptr, const int32_t *__restrict__ tail, int64_t nv,
+    int32_t *color, int nHash, int64_t nextColor, const uint32_t *__restrict__ hash,
+    unsigned long long *__restrict__ ncolored, const int32_t *__restrict__ ref) {
+    __shared__ int32_t s_tail[CR_WARPS][CR_STAGE];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int32_t *st = s_tail[threadIdx.x >> 5];
+    const uint4 *__restrict__ h4 = reinterpret_cast<const uint4 *>(hash);
+    const uint32_t all = (1u << nHash) - 1u;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    unsigned mine = 0;
+    for (int64_t tile = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; tile * 32 < nv; tile += nw) {
+        const int64_t v = tile * 32 + lane;
+        const bool valid = v < nv;
+        const bool open = valid && (FIRST || color[v] == -1);
+        if (!__any_sync(full, open)) continue;
+        int64_t e0 = 0, e1 = 0;
+        if (valid) {
+            e0 = rowptr[v];
+            e1 = rowptr[v + 1];
+        }
+        const int64_t E0 = __shfl_sync(full, e0, 0);
+        const int64_t E1 = __shfl_sync(full, e1, 31 - __clz(__ballot_sync(full, valid)));
+        const bool staged = E1 - E0 <= CR_STAGE;
+        if (staged) {
+            for (int j = lane; j < (int)(E1 - E0); j += 32) st[j] = tail[E0 + j];
+            __syncwarp();
+        }
+        if (open) {
+            uint32_t own[P];
+#pragma unroll
+            for (int q = 0; q < P / 4; q++) {
+                const uint4 x = h4[v * (P / 4) + q];
+                own[4 * q] = x.x;
+                own[4 * q + 1] = x.y;
+                own[4 * q + 2] = x.z;
+                own[4 * q + 3] = x.w;
+            }
+            uint32_t not_min = 0, not_max = 0;
+            bool can_color = true;
+            for (int64_t k = e0; k < e1; k++) {
+                const int32_t u = staged ? st[k - E0] : tail[k];
+                if (u == v) continue;
+                if (!FIRST) {
+                    const int32_t cu = color[u];
+                    if (cu != -1 && cu < nextColor) continue;
+                }
+#pragma unroll
+                for (int q = 0; q < P / 4; q++) {
+                    const uint4 x = h4[(int64_t)u * (P / 4) + q];
+                    const uint32_t h[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                    for (int t = 0; t < 4; t++) {
+                        not_max |= (uint32_t)(own[4 * q + t] <= h[t]) << (4 * q + t);
+                        not_min |= (uint32_t)(own[4 * q + t] >= h[t]) << (4 * q + t);
+                    }
+                }
+                if ((not_max & not_min & all) == all) {
+                    can_color = false;
+                    break;
+                }
+            }
+            if (can_color) {
+                const int64_t rv = vg_rid(ref, (int32_t)v);
+                const int possible = __popc(~not_min & all) + __popc(~not_max & all);
+                const int64_t col_id = rv % possible;
+                int64_t this_col = 0;
+                for (int t = 0; t < nHash; t++) {
+                    if (!(not_min & (1u << t)) && col_id == this_col) {
+                        color[v] = (int32_t)(2 * t + nextColor);
+                        mine++;
+                        break;
+                    }
+                    this_col += !(not_min & (1u << t));
+                    if (!(not_max & (1u << t)) && col_id == this_col) {
+                        color[v] = (int32_t)(2 * t + 1 + nextColor);
+                        mine++;
+                        break;
+                    }
+                    this_col += !(not_max & (1u << t));
+                }
+            }
+        }
+        __syncwarp();
+    }
+    mine = __reduce_add_sync(full, mine);
+    if (lane == 0 && mine) atomicAdd(ncolored, (unsigned long long)mine);
+}
+
+template <int P>
+void color_round_hashed(vg_ctx *ctx, const vg_graph *g, int nHash, int64_t nextColor, uint32_t seed,
+                        uint32_t *hash, unsigned long long *ncolored) {
+    const int64_t nv = g->nv;
+    {
+        LaunchTimer lt(ctx);
+        k_color_hash<P><<<vg_grid(ctx, nv, 256), 256, 0, ctx->stream>>>(nv, nHash, seed, g->ref, hash);
+    }
+    VG_CHECK_LAUNCH();
+    LaunchTimer lt(ctx);
+    auto *round = nextColor == 0 ? k_color_round_hashed<P, true> : k_color_round_hashed<P, false>;
+    round<<<vg_grid(ctx, nv, CR_WARPS * 32), CR_WARPS * 32, 0, ctx->stream>>>(
+        g->rowptr, g->tail, nv, g->colors, nHash, nextColor, hash, ncolored, g->ref);
+}
+
 __global__ void k_fill_i32(int32_t *__restrict__ x, int64_t n, int32_t val) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
@@ -110,13 +244,22 @@ int64_t vg_color_internal(vg_ctx *ctx, vg_graph *g, int64_t nHash, int32_t targe
     VG_CHECK_LAUNCH();
     DevBuf<unsigned long long> cnt(ctx, 1);
     unsigned long long *h = (unsigned long long *)vg_pinned(ctx, sizeof(unsigned long long));
+    // up to eight hashes are kept per vertex, where the context's budget has room for them
+    DevBuf<uint32_t> hash;
+    const size_t words = (size_t)nv * (nHash <= 4 ? 4 : 8);
+    if (nHash <= 8 && (!ctx->budget || ctx->in_use + sizeof(uint32_t) * words <= ctx->budget))
+        hash.alloc(ctx, words);
     uint32_t seed = 1012; // coloring.cpp:60
     int64_t nextColor = 0, lastCount = 0, currentCount = 0;
     const int64_t targetCount = (nv * target_percent) / 100;
     bool finished = false;
     while (!finished) {
         VG_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned long long), ctx->stream));
-        if (nv) {
+        if (nv && hash.p && nHash <= 4) {
+            color_round_hashed<4>(ctx, g, (int)nHash, nextColor, seed, hash.p, cnt.p);
+        } else if (nv && hash.p) {
+            color_round_hashed<8>(ctx, g, (int)nHash, nextColor, seed, hash.p, cnt.p);
+        } else if (nv) {
             LaunchTimer lt(ctx);
             k_color_round<<<vg_grid(ctx, nv, 256), 256, 0, ctx->stream>>>(
                 g->rowptr, g->tail, nv, g->colors, (int)nHash, nextColor, seed, cnt.p, g->ref);
