@@ -46,13 +46,13 @@ def check(ctx, g, real, **kw):
 
 
 # (vertices, pairs, self loops, hub entries): one vertex; rows of 31..33 entries (thread and
-# warp rows), 511..513 (warp and block rows), above 4,096 entries on fewer and on more
-# vertices than that (block table, general path); 2,048-vertex sum chunks +- 1; entries just
+# warp rows), 511..513 (warp and block rows), thousands of entries on fewer and on
+# more than 8,192 vertices (block table, general path); 2,048-vertex sum chunks +- 1; entries just
 # below and above the cluster's 16,384 and the path's 2^21; a warp per row and a thread per row
 SIZES = [(1, 0, 3, 0), (2, 8, 0, 0), (33, 500, 4, 0), (700, 900, 5, 31), (700, 900, 5, 32),
          (700, 900, 0, 33), (700, 300, 9, 511), (700, 300, 9, 513), (1500, 4000, 0, 9000),
          (2047, 4000, 3, 0), (2049, 8180, 0, 0), (2049, 8200, 7, 0), (5000, 9000, 0, 4090),
-         (9000, 9000, 0, 8000), (9400, 30000, 0, 0), (40000, 90000, 20, 600), (65537, 100000, 0, 0),
+         (9000, 9000, 0, 8000), (8193, 9000, 0, 8190), (9500, 9000, 0, 9000), (9400, 30000, 0, 0), (40000, 90000, 20, 600), (65537, 100000, 0, 0),
          (30000, (1 << 20) - 2000, 0, 0), (30000, (1 << 20) + 2000, 0, 0)]
 
 

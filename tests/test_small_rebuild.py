@@ -1,7 +1,7 @@
 """The one-launch rebuild of small graphs (rebuild_small.cuh) against the oracle (GPU), bit
 for bit: members per row around 32 (registers, bitmap), segments of entries around a chunk and
 1,024 (warp and block tables), a giant community, more distinct keys than the tables take
-(general path), entries around the launch forms' limits, both layouts."""
+(ranges of keys, and the general path), entries around the launch forms' limits, both layouts."""
 import numpy as np
 import pytest
 
@@ -23,6 +23,10 @@ def communities(n, kind, seed):
         c = rng.integers(0, n, n)
         c[rng.random(n) < 0.5] = 3 % n
         return c
+    if kind == "wide":  # one community of a tenth of the vertices, the others single
+        c = rng.permutation(n).astype(np.int64)
+        c[rng.random(n) < 0.1] = c[0]
+        return c
     if kind.startswith("random"):
         return rng.integers(0, min(n, int(kind[6:])), n) * (n // min(n, int(kind[6:])))
     return rng.permutation(n)[np.arange(n) // int(kind)].astype(np.int64)
@@ -33,7 +37,7 @@ CASES = [(1, 0, 2, "one"), (2, 5, 0, "single"), (97, 300, 3, "31"), (97, 300, 3,
          (5000, 40000, 0, "random40"), (5000, 40000, 20, "giant"), (20000, 60000, 0, "7"),
          (30000, 300000, 0, "random300"), (40000, 200000, 0, "one"), (9000, 400000, 0, "random4"),
          (16000, 8190, 1, "single"), (16000, 8194, 1, "5"), (30000, 400000, 0, "giant"),
-         (131072, 140000, 0, "3"), (131073, 140000, 0, "3"), (20000, 1 << 20, 0, "random900"),
+         (30000, 300000, 0, "wide"), (60000, 60000, 0, "wide"), (131072, 140000, 0, "3"), (131073, 140000, 0, "3"), (20000, 1 << 20, 0, "random900"),
          (20000, (1 << 20) + 9000, 0, "random900")]
 
 

@@ -473,12 +473,14 @@ template <int NT, int CAP_, int MAXU_> struct BlockTable {
 using BlockTableSmall = BlockTable<128, 2048, 1024>;
 using BlockTableLarge = BlockTable<512, 8192, 4096>;
 
-// entries [s0, s0 + L) of gk/gw; returns the number of distinct keys, or -1 when there are
-// more than MAXU. The whole block calls it and gets the same answer.
+// entries [s0, s0 + L) of gk/gw with keys in [lo, hi); the sorted keys and their sums go to
+// uk/uw at o0. Returns the number of distinct keys, or -1 when there are more than MAXU. The
+// whole block calls it and gets the same answer.
 template <bool LIVE, class Table>
 __device__ __forceinline__ int block_segment(Table &T, int64_t s0, int64_t L, bool integral,
                                              const int32_t *gk, const double *gw, int32_t *uk,
-                                             double *uw) {
+                                             double *uw, int64_t o0, int32_t lo = 0,
+                                             int32_t hi = INT_MAX) {
     constexpr int NT = Table::THREADS, NW = Table::WARPS, CHUNKS = Table::CHUNKS;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
@@ -494,6 +496,7 @@ __device__ __forceinline__ int block_segment(Table &T, int64_t s0, int64_t L, bo
     __syncthreads();
     double *stage = T.stage[warp];
     bool over = false;
+    auto in_range = [&](int32_t k) { return k >= lo && k < hi ? k : -1; };
     // one chunk's entries, an entry per lane (k < 0: none), onto the table
     auto add_chunk = [&](int32_t k, double w) {
         const unsigned peers = __match_any_sync(full, k >= 0 ? k : -2 - lane);
@@ -539,7 +542,7 @@ __device__ __forceinline__ int block_segment(Table &T, int64_t s0, int64_t L, bo
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const int64_t i = base + j * NT + lane;
-                kq[j] = i < L ? seg_ld<LIVE>(gk + s0 + i) : -1;
+                kq[j] = i < L ? in_range(seg_ld<LIVE>(gk + s0 + i)) : -1;
                 wq[j] = i < L ? seg_ld<LIVE>(gw + s0 + i) : 0.0;
             }
 #pragma unroll
@@ -556,7 +559,7 @@ __device__ __forceinline__ int block_segment(Table &T, int64_t s0, int64_t L, bo
 #pragma unroll
             for (int j = 0; j < CHUNKS; j++) {
                 const int64_t i = i0 + j * 32;
-                kq[j] = i < L ? seg_ld<LIVE>(gk + s0 + i) : -1;
+                kq[j] = i < L ? in_range(seg_ld<LIVE>(gk + s0 + i)) : -1;
                 wq[j] = i < L ? seg_ld<LIVE>(gw + s0 + i) : 0.0;
             }
             auto share_of = [](int32_t k) { return (int)((((uint32_t)k * 2654435761u) >> 8) & (NW - 1)); };
@@ -620,8 +623,8 @@ __device__ __forceinline__ int block_segment(Table &T, int64_t s0, int64_t L, bo
             if (i >= U) break;
             uint32_t h = ((uint32_t)x[e] * 2654435761u) >> (32 - logcap);
             while (T.keys[h] != x[e]) h = (h + 1) & mask;
-            uk[s0 + i] = x[e];
-            uw[s0 + i] = T.vals[h];
+            uk[o0 + i] = x[e];
+            uw[o0 + i] = T.vals[h];
         }
     };
     if (U <= 2 * NT) sorted(std::integral_constant<int, 2>{});
@@ -645,7 +648,7 @@ __global__ void __launch_bounds__(Table::THREADS) k_rows_block(
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
         const int32_t row = in[i];
         const int64_t s0 = rstart[row], L = rstart[row + 1] - s0;
-        const int U = block_segment<false>(T, s0, L, integral != 0, gk, gw, uk, uw);
+        const int U = block_segment<false>(T, s0, L, integral != 0, gk, gw, uk, uw, s0);
         if (threadIdx.x == 0) {
             if (U >= 0)
                 ucount[row] = U;
@@ -823,7 +826,7 @@ __global__ void k_big_fold_long(const uint64_t *__restrict__ K, const uint32_t *
 }
 
 // real weights: the listed runs (longer than SEQ_RUN entries), one warp each; the
-// sum stays one left fold in run order (vg_warp_ordered_fold)
+// sum stays one left fold in run order (vg_warp_fold)
 __global__ void k_big_fold_seq(
     const uint64_t *__restrict__ K, const uint32_t *__restrict__ V, int64_t m, int kbits,
     const int64_t *__restrict__ nheads_dev, const int64_t *__restrict__ headpos,

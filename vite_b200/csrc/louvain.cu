@@ -1444,8 +1444,7 @@ __global__ void k_degree_huge(const int64_t *__restrict__ rowptr, const double *
 
 // one warp per listed row. Integral weights: every partial sum is exact, so lanes
 // add strided entries and a shuffle tree combines them. Otherwise the row's left
-// fold in CSR order (vg_warp_ordered_fold: the warp fetches the weights ahead of
-// lane 0's chain of additions).
+// fold in CSR order (vg_warp_fold).
 constexpr int DEG_LONG_WARPS = 4; // warps per k_degree_long block (one chain per scheduler)
 __global__ void __launch_bounds__(DEG_LONG_WARPS * 32)
     k_degree_long(const int64_t *__restrict__ rowptr, const double *__restrict__ w,

@@ -29,6 +29,7 @@
 constexpr int SP_THREADS = GS_THREADS;
 constexpr int SP_WARPS = GS_WARPS;
 constexpr int SP_T = 32;       // rows up to here: one thread each
+constexpr int SP_CAP = 16384;  // slots of a block's table: rows of up to half as many communities
 constexpr int SP_UNITS = SEG_CHUNK == 2048 && SEG_THREADS == 256 ? 8 : -1; // warps per chunk
 #ifndef VG_SP_MAX_NV
 #define VG_SP_MAX_NV 524288
@@ -193,7 +194,7 @@ __device__ __forceinline__ void warp_short_vertex(const A &a, int32_t v, int64_t
 // dynamic shared memory: the rows' slots and tables, one class at a time
 constexpr size_t SP_WORK_BYTES = warp_smem_bytes<WT_CAP, SP_WARPS>();
 static_assert(SP_WORK_BYTES >= sizeof(double) * SP_T * SP_THREADS &&
-                  SP_WORK_BYTES >= cta_smem_bytes(CT_CAP, SP_THREADS) &&
+                  SP_WORK_BYTES >= cta_smem_bytes(SP_CAP, SP_THREADS) &&
                   SP_WORK_BYTES >= sizeof(double) * 2 * VG_FOLD_STEP * SP_WARPS,
               "every class's tables must fit the block's work area");
 
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
             const int64_t e0 = a.rowptr[v], e1 = a.rowptr[v + 1];
             const int64_t d = e1 - e0;
             if (d <= SP_T) p.vdeg[v] = row_fold(a.weight, e0, e1);
-            if (min(d, nv) > CT_MAXDEG) p.ctl[CTL_REFUSED] = 1;
+            if (min(d, nv) > SP_CAP / 2) p.ctl[CTL_REFUSED] = 1;
             bucket = bucket_of(v, d);
         }
         const unsigned peers = __match_any_sync(0xffffffffu, bucket);
@@ -385,7 +386,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
             };
             int i = first(base[ROW_BLOCK], rank, blocks);
             if (i < base[SP_CLASSES]) { // uniform over the block
-                const Table t = cta_table<SP_THREADS>(smem_raw, CT_CAP, sh);
+                const Table t = cta_table<SP_THREADS>(smem_raw, SP_CAP, sh);
                 for (; i < base[SP_CLASSES]; i += blocks) {
                     const int32_t v = __ldcg(p.list + i);
                     const int64_t e0 = a.rowptr[v], d = a.rowptr[v + 1] - e0;

@@ -155,7 +155,7 @@ vg_graph *vg_rebuild_small(vg_ctx *ctx, const vg_graph *g, const int32_t *comm);
 vg_graph *vg_rebuild_new(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) {
     const int64_t nv = g->nv;
     if (vg_graph *h = vg_rebuild_small(ctx, g, comm)) {
-        h->integral = g->integral == 1 ? 1 : -1; // sums of the same integers
+        h->integral = g->integral; // sums of the same integers; else the in-order folds serve any weights
         return h;
     }
     const int grid = vg_grid(ctx, nv, 256);
@@ -182,7 +182,7 @@ vg_graph *vg_rebuild_new(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) {
         flag.release();
         rank.release();
         vg_graph *h = vg_aggregate_rows(ctx, g, nullptr, newof.p, newof.p, nc, nullptr);
-        h->integral = g->integral == 1 ? 1 : -1; // sums of the same integers
+        h->integral = g->integral; // sums of the same integers; else the in-order folds serve any weights
         return h;
     }
     DevBuf<int32_t> first_ref(ctx, nv), first_pos(ctx, nv), flag_ref(ctx, nv), flag_pos(ctx, nv);
@@ -229,7 +229,7 @@ vg_graph *vg_rebuild_new(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) {
     }
     h->ref = r2.detach();
     h->pos = p2.detach();
-    h->integral = g->integral == 1 ? 1 : -1; // sums of the same integers
+    h->integral = g->integral; // sums of the same integers; else the in-order folds serve any weights
     return h;
 }
 

@@ -33,6 +33,11 @@ constexpr int64_t RS_MAX_NV = VG_RS_MAX_NV;
 constexpr int64_t RS_MAX_NE = VG_RS_MAX_NE;
 static_assert(RS_MAX_NV <= NARROW_KEYS, "warp_segment is told so");
 constexpr int RS_BIG_L = 1024; // segments longer than this go to a whole block
+// A block reads a segment of many keys once per 4,096 key values; a graph with a segment that
+// might be read for more entries than this is left to the general path before any is read
+// (a rebuild of 104,000 vertices with a 60,000-entry segment and 13 reads took 2.75 ms
+// here, 1.1 there; 9,700 vertices, three reads, 0.34 here, 0.97 there).
+constexpr int64_t RS_MAX_READS = 262144;
 
 using SmallWarpTable = HashWarpSmem<H_CAP, H_MAXU>;
 using SmallBlockTable = BlockTableLarge;
@@ -200,6 +205,9 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_rebuild_small(SmallRebuild p)
                 p.mbase[r] = ma + mp;
                 p.rstart[r] = ea + ep;
                 if (m > 32) p.biglist[atomicAdd(p.ctl + RS_BIG_ROWS, 1)] = (int32_t)r;
+                const int64_t reads = (nc + SmallBlockTable::MAXU - 1) / SmallBlockTable::MAXU;
+                if (reads > 1 && e > SmallBlockTable::MAXU && e * reads > RS_MAX_READS)
+                    p.ctl[RS_REFUSED] = 1;
                 if (e > RS_BIG_L) p.longlist[atomicAdd(p.ctl + RS_LONG_SEGS, 1)] = (int32_t)r;
             }
             ma += mt;
@@ -207,6 +215,10 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_rebuild_small(SmallRebuild p)
         }
     }
     if (!barrier()) return;
+    if (__ldcg(p.ctl + RS_REFUSED)) { // the same in every block
+        if (rank == 0 && tid == 0) p.out->status = GS_REFUSED;
+        return;
+    }
     for (int64_t i = gtid; i < nv; i += gthreads) {
         const int32_t row = __ldcg(row_of + p.comm[i]);
         p.mlist[__ldcg(p.mbase + row) + atomicAdd(p.mfill + row, 1)] = vg_rid(p.ref, (int32_t)i);
@@ -327,21 +339,18 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_rebuild_small(SmallRebuild p)
     const int nlong = __ldcg(p.ctl + RS_LONG_SEGS);
     for (int b = rank; b < nlong; b += blocks) { // uniform over the block
         const int64_t r = __ldcg(p.longlist + b);
-        const int U = block_segment<true>(*reinterpret_cast<SmallBlockTable *>(smem_raw),
-                                          __ldcg(p.rstart + r), __ldcg(p.ecount + r), p.integral,
-                                          p.gk, p.gw, p.uk, p.uw);
-        if (tid == 0) {
-            if (U >= 0)
-                p.ucount[r] = U;
-            else
-                p.ctl[RS_REFUSED] = 1;
+        SmallBlockTable &T = *reinterpret_cast<SmallBlockTable *>(smem_raw);
+        const int64_t s0 = __ldcg(p.rstart + r), L = __ldcg(p.ecount + r);
+        int64_t U = block_segment<true>(T, s0, L, p.integral, p.gk, p.gw, p.uk, p.uw, s0);
+        if (U < 0) { // more keys than the table takes: a range of as many key values at a time
+            U = 0;
+            for (int64_t lo = 0; lo < nc; lo += SmallBlockTable::MAXU)
+                U += block_segment<true>(T, s0, L, p.integral, p.gk, p.gw, p.uk, p.uw, s0 + U,
+                                         (int32_t)lo, (int32_t)(lo + SmallBlockTable::MAXU));
         }
+        if (tid == 0) p.ucount[r] = U;
     }
     if (!barrier()) return;
-    if (__ldcg(p.ctl + RS_REFUSED)) { // the same in every block
-        if (rank == 0 && tid == 0) p.out->status = GS_REFUSED;
-        return;
-    }
     // the next level's row offsets
     {
         int64_t a = 0, total;
