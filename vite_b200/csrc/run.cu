@@ -4,6 +4,8 @@
 // re-run under threshold cycling (:448-463) and the phase caps (:504-512).
 #include "vg_internal.cuh"
 
+#include <algorithm>
+
 
 void vg_phase_internal(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double *mod_out,
                        int32_t *iters_out, double *sweep_ms, int64_t *edges);
@@ -13,24 +15,49 @@ vg_graph *vg_rebuild_new(vg_ctx *ctx, const vg_graph *g, const int32_t *comm);
 
 namespace {
 
-struct EventTimer {
-    cudaEvent_t a = nullptr, b = nullptr;
-    cudaStream_t s;
-    explicit EventTimer(cudaStream_t st) : s(st) {
-        VG_CUDA(cudaEventCreate(&a));
-        VG_CUDA(cudaEventCreate(&b));
-        VG_CUDA(cudaEventRecord(a, s));
+// Device times of the run's steps: event pairs from the context's pool, recorded as the steps
+// are enqueued and read once at the end, so that a step does not wait for its time (two waits
+// a level were 6 % of a run on 1,201 vertices).
+struct StepTimes {
+    enum Field { LAYOUT, COLOR, PHASE, REBUILD };
+    struct Step {
+        std::pair<cudaEvent_t, cudaEvent_t> ev;
+        int level;
+        Field field;
+    };
+    vg_ctx *ctx;
+    std::vector<Step> steps;
+    explicit StepTimes(vg_ctx *c) : ctx(c) {}
+    ~StepTimes() {
+        for (auto &s : steps) ctx->event_pool.push_back(s.ev);
     }
-    double stop_ms() {
-        VG_CUDA(cudaEventRecord(b, s));
-        VG_CUDA(cudaEventSynchronize(b));
-        float ms = 0.f;
-        VG_CUDA(cudaEventElapsedTime(&ms, a, b));
-        return ms;
+    // the step `field` of level `level` starts here / ended here
+    size_t begin(int level, Field field) {
+        Step s{{nullptr, nullptr}, level, field};
+        if (!ctx->event_pool.empty()) {
+            s.ev = ctx->event_pool.back();
+            ctx->event_pool.pop_back();
+        } else {
+            VG_CUDA(cudaEventCreate(&s.ev.first));
+            const cudaError_t e = cudaEventCreate(&s.ev.second);
+            if (e != cudaSuccess) cudaEventDestroy(s.ev.first);
+            VG_CUDA(e);
+        }
+        steps.push_back(s);
+        VG_CUDA(cudaEventRecord(s.ev.first, ctx->stream));
+        return steps.size() - 1;
     }
-    ~EventTimer() {
-        if (a) cudaEventDestroy(a);
-        if (b) cudaEventDestroy(b);
+    void end(size_t step) { VG_CUDA(cudaEventRecord(steps[step].ev.second, ctx->stream)); }
+    // into levels[0 .. n), after the stream has been waited for
+    void read(vg_level_stat *levels, int32_t n) {
+        for (auto &s : steps) {
+            if (!levels || s.level >= n) continue;
+            float ms = 0.f;
+            VG_CUDA(cudaEventElapsedTime(&ms, s.ev.first, s.ev.second));
+            vg_level_stat &l = levels[s.level];
+            (s.field == LAYOUT ? l.seconds_layout : s.field == COLOR ? l.seconds_color
+             : s.field == PHASE ? l.seconds_phase : l.seconds_rebuild) = ms * 1e-3;
+        }
     }
 };
 
@@ -60,14 +87,14 @@ extern "C" vg_status vg_louvain_run(vg_ctx *ctx, const vg_graph *g0, const vg_ru
         view.num_colors = -1;
         vg_graph *cur = &view;
         VG_REQUIRE(rp->layout >= 0 && rp->layout <= 2, "layout must be 0, 1 or 2");
-        double layout_s = 0.0;
+        StepTimes times(ctx);
         if (vg_auto_layout(ctx, g0, rp->layout)) {
-            EventTimer tl(ctx->stream);
+            const size_t t = times.begin(0, StepTimes::LAYOUT);
             DevBuf<int32_t> order;
             vg_bfs_order(ctx, g0, order);
             owned = vg_apply_layout(ctx, g0, order.p);
             cur = owned;
-            layout_s = tl.stop_ms() * 1e-3;
+            times.end(t);
         }
         // the -o map lives on the device; it is copied out once at the end
         DevBuf<int32_t> commAll;
@@ -93,7 +120,6 @@ extern "C" vg_status vg_louvain_run(vg_ctx *ctx, const vg_graph *g0, const vg_ru
                 vg_level_stat ls = {};
                 ls.nv = cur->nv;
                 ls.ne = cur->ne;
-                if (phase == 0) ls.seconds_layout = layout_s;
                 vg_phase_params pp = {};
                 pp.lower = currMod;
                 pp.threshold = threshold;
@@ -101,18 +127,18 @@ extern "C" vg_status vg_louvain_run(vg_ctx *ctx, const vg_graph *g0, const vg_ru
                 pp.et_delta = rp->et_delta;
                 pp.ordering = 0;
                 if ((rp->coloring || rp->vertex_order) && phase == 0) {
-                    EventTimer tc(ctx->stream);
+                    const size_t t = times.begin(nrec, StepTimes::COLOR);
                     ls.num_colors = vg_color_internal(ctx, cur, rp->max_colors / 2, 70 /* MAX_COVG */,
                                                       rp->single_color_iter);
-                    ls.seconds_color = tc.stop_ms() * 1e-3;
+                    times.end(t);
                     pp.ordering = rp->coloring ? 1 : 2;
                 }
                 int32_t iters = 0;
                 {
-                    EventTimer tp(ctx->stream);
+                    const size_t t = times.begin(nrec, StepTimes::PHASE);
                     double sweep_ms = 0.0;
                     vg_phase_internal(ctx, cur, &pp, &currMod, &iters, &sweep_ms, &ls.edges_swept);
-                    ls.seconds_phase = tp.stop_ms() * 1e-3;
+                    times.end(t);
                     ls.seconds_sweep = sweep_ms * 1e-3;
                 }
                 ls.iters = iters;
@@ -122,7 +148,7 @@ extern "C" vg_status vg_louvain_run(vg_ctx *ctx, const vg_graph *g0, const vg_ru
                 if (accepted) {
                     if (comm_out) vg_compose_level(ctx, cur, commAll.p, g0->nv, phase == 0);
                     if (!rp->one_phase) {
-                        EventTimer tr(ctx->stream);
+                        const size_t t = times.begin(nrec, StepTimes::REBUILD);
                         vg_graph *next = vg_rebuild_new(ctx, cur, cur->comm);
                         if (cur == &view) {
                             cleanup_view();
@@ -132,7 +158,7 @@ extern "C" vg_status vg_louvain_run(vg_ctx *ctx, const vg_graph *g0, const vg_ru
                         }
                         owned = next;
                         cur = owned;
-                        ls.seconds_rebuild = tr.stop_ms() * 1e-3;
+                        times.end(t);
                     }
                 }
                 if (levels && nrec < max_levels) levels[nrec] = ls;
@@ -145,10 +171,10 @@ extern "C" vg_status vg_louvain_run(vg_ctx *ctx, const vg_graph *g0, const vg_ru
                         vg_phase_params px = {};
                         px.lower = currMod;
                         px.threshold = 1.0E-6;
-                        EventTimer tp(ctx->stream);
+                        const size_t t = times.begin(nrec, StepTimes::PHASE);
                         double sweep_ms = 0.0;
                         vg_phase_internal(ctx, cur, &px, &currMod, &iters, &sweep_ms, &lx.edges_swept);
-                        lx.seconds_phase = tp.stop_ms() * 1e-3;
+                        times.end(t);
                         lx.seconds_sweep = sweep_ms * 1e-3;
                         lx.iters = iters;
                         lx.modularity = currMod;
@@ -172,6 +198,7 @@ extern "C" vg_status vg_louvain_run(vg_ctx *ctx, const vg_graph *g0, const vg_ru
         if (nlevels_out) *nlevels_out = nrec;
         if (comm_out) vg_download_map(ctx, commAll.p, g0->nv, comm_out);
         vg_sync(ctx);
+        times.read(levels, std::min(nrec, max_levels));
     });
     if (owned) {
         vg_graph_release(ctx, owned);
