@@ -1,6 +1,7 @@
 """The coloring's kernels (hashes kept per vertex up to eight, computed per entry above)
 against the oracle (GPU): every number of hashes around the two layouts, entries around
-the kept ones' limit, rows longer than a warp's stage, self loops, isolated vertices, several rounds, both layouts."""
+the kept ones' limit, rows longer than a warp's stage, self loops, isolated vertices,
+several rounds, both layouts."""
 import numpy as np
 import pytest
 

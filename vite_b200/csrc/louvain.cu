@@ -121,6 +121,9 @@ struct SweepArgs {
     const int32_t *__restrict__ vjob = nullptr;
     const double *__restrict__ jconst = nullptr;
     const uint8_t *__restrict__ jdone = nullptr;
+    // one graph: set once its phase has ended, so that an iteration enqueued ahead of that
+    // returns at once (null: not looked at)
+    const uint8_t *__restrict__ stop = nullptr;
 
     // loads of the per-vertex and per-community arrays (curr, vdeg, cdeg, csize,
     // noprune, active, frozen): no sweep launch writes what it reads, so the read-only
@@ -133,6 +136,8 @@ struct SweepArgs {
 struct LiveArgs : SweepArgs {
     template <class T> static __device__ __forceinline__ T ld(const T *p) { return __ldcg(p); }
 };
+
+__device__ __forceinline__ bool stopped(const SweepArgs &a) { return a.stop && __ldg(a.stop); }
 
 // the constant of v's graph; false when v belongs to a graph whose phase has ended
 template <class A> __device__ __forceinline__ bool vertex_live(const A &a, int32_t v, double &cst) {
@@ -551,6 +556,7 @@ __device__ __forceinline__ void thread_vertex(const A &a, int32_t v, int64_t e0,
 template <bool LIST, int T, int NT>
 __global__ void __launch_bounds__(NT, (T <= 16 ? VG_T16_MINB : VG_T32_MINB)) k_sweep_thread(
     SweepArgs a, const int32_t *__restrict__ list, int64_t count) {
+    if (stopped(a)) return;
     __shared__ double ssum[T][NT];
     const int tid = threadIdx.x;
     for (int64_t idx = blockIdx.x * (int64_t)NT + tid; idx < count; idx += (int64_t)gridDim.x * NT) {
@@ -650,6 +656,7 @@ constexpr int TILE_WARPS = VG_TILE_WARPS;
 
 template <int T, bool IDENT>
 __global__ void __launch_bounds__(TILE_WARPS * 32, VG_TILE_MINB) k_sweep_tile(SweepArgs a, int64_t nv) {
+    if (stopped(a)) return;
     static_assert(32 * T <= TILE_CAP + 8, "the per-lane fallback layout must fit the buffer");
     __shared__ __align__(16) int32_t st_all[TILE_WARPS][TILE_CAP + 8];
     __shared__ __align__(16) double sw_all[TILE_WARPS][TILE_CAP + 8];
@@ -878,6 +885,7 @@ __device__ __forceinline__ void warp_vertex(const A &a, int32_t v, double cst, c
 template <int CAP, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, CAP <= 256 ? 4 : 1) k_sweep_warp(
     SweepArgs a, const int32_t *__restrict__ list, int64_t count) {
+    if (stopped(a)) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Table t = warp_table<CAP, WARPS>(smem_raw, threadIdx.x >> 5);
     const int64_t wg = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -1032,6 +1040,7 @@ __device__ __forceinline__ void cta_vertex(const A &a, int32_t v, int64_t e0, in
 template <int CAP>
 __global__ void __launch_bounds__(CT_THREADS) k_sweep_cta(SweepArgs a, const int32_t *__restrict__ list,
                                                           int64_t count) {
+    if (stopped(a)) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ CtaShared<CT_THREADS> sh;
     const Table t = cta_table<CT_THREADS>(smem_raw, CAP, sh);
@@ -1088,6 +1097,7 @@ __global__ void __launch_bounds__(HUB_THREADS) k_hub_accum(
     SweepArgs a, const int32_t *__restrict__ vtx, const int64_t *__restrict__ toff,
     const int64_t *__restrict__ cb, int64_t q0, int64_t q1, int32_t *__restrict__ keys,
     double *__restrict__ vals, double *__restrict__ self) {
+    if (stopped(a)) return;
     __shared__ __align__(16) double stage[HUB_THREADS];
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
@@ -1151,6 +1161,7 @@ __global__ void __launch_bounds__(HUB_THREADS) k_hub_accum(
 __global__ void k_hub_c0(SweepArgs a, const int32_t *__restrict__ vtx, const int64_t *__restrict__ toff,
                          int64_t q0, int64_t q1, const int32_t *__restrict__ keys,
                          const double *__restrict__ vals, double *__restrict__ c0) {
+    if (stopped(a)) return;
     for (int64_t q = q0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < q1;
          q += (int64_t)gridDim.x * blockDim.x) {
         const int32_t v = vtx[q];
@@ -1181,6 +1192,7 @@ __global__ void __launch_bounds__(HUB_THREADS) k_hub_eval(
     const int64_t *__restrict__ sb, int64_t q0, int64_t q1, int32_t *__restrict__ keys,
     double *__restrict__ vals, const double *__restrict__ self, const double *__restrict__ c0,
     HubBest *__restrict__ best) {
+    if (stopped(a)) return;
     __shared__ double red_g[HUB_THREADS / 32];
     __shared__ int32_t red_c[HUB_THREADS / 32], red_s[HUB_THREADS / 32], red_ok[HUB_THREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1274,6 +1286,7 @@ __global__ void __launch_bounds__(HUB_THREADS) k_hub_eval(
 __global__ void k_hub_commit(SweepArgs a, const int32_t *__restrict__ vtx, const int64_t *__restrict__ sb,
                              int64_t q0, int64_t q1, double *__restrict__ self,
                              const double *__restrict__ c0, const HubBest *__restrict__ best) {
+    if (stopped(a)) return;
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -2331,6 +2344,79 @@ static bool run_phase_small(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, 
     return true;
 }
 
+// The iterations of plain phases (bd: their loop tests on the device, J of them in seg) until
+// every one has ended; a: the arrays, without curr and target; bufs: past, curr and target of
+// the first iteration. Two iterations are in flight: the next one is enqueued before the live
+// count of the one before is waited for, so the device never waits for the host (after the
+// last iteration every graph is done and the extra one's launches return at once). Enqueued
+// directly: capturing a batch's iteration as a graph cost 1.2-1.5 ms a phase, more than its
+// replays saved (48 graphs of 1,000-256,000 vertices: phases 26.5 -> 17.0 ms).
+// sweep_ms (or null) gets the sweeps' time; returns the iterations.
+static int32_t iterate(vg_ctx *ctx, SweepArgs a, BatchDecide bd, int32_t *const (&bufs)[3], const Buckets &bk,
+                       HubPlan &hp, const SegTable &seg, int64_t nv, double *cdeg, int32_t *csize,
+                       double *part, int32_t *noprune, double *sweep_ms) {
+    const int agrid = seg_grid(ctx, seg.C);
+    int32_t *hlive = (int32_t *)vg_pinned(ctx, 2 * sizeof(int32_t));
+    int32_t *live = bd.live_count; // 2
+    // iteration `it` with bufs[pi] = past, bufs[pi+1] = curr, bufs[pi+2] = target; its live
+    // count lands in hlive[slot]
+    auto enqueue = [&](int pi, int32_t it, int slot, cudaEvent_t e0, cudaEvent_t e1) {
+        a.curr = bufs[(pi + 1) % 3];
+        a.target = bufs[(pi + 2) % 3];
+        // the first iteration of one graph: every vertex in its own community
+        a.ident = it == 1 && !a.vjob ? 1 : 0;
+        VG_CUDA(cudaMemsetAsync(live + slot, 0, sizeof(int32_t), ctx->stream));
+        if (e0) VG_CUDA(cudaEventRecord(e0, ctx->stream));
+        sweep_color(ctx, a, bk, 0, hp, true, nv);
+        if (e1) VG_CUDA(cudaEventRecord(e1, ctx->stream));
+        {
+            LaunchTimer lt(ctx);
+            k_apply_seg<<<agrid, SEG_THREADS, 0, ctx->stream>>>(seg.voff.p, seg.cb.p, seg.J, seg.C,
+                                                                cdeg, csize, a.cupd, a.cw, nullptr,
+                                                                bd.done, 1, part, noprune);
+        }
+        VG_CHECK_LAUNCH();
+        bd.live_count = live + slot;
+        bd.iter = it;
+        bd.past_idx = pi;
+        {
+            LaunchTimer lt(ctx);
+            k_mod_seg<<<(int)std::min<int64_t>(seg.J, 65535), SEG_FINAL, 0, ctx->stream>>>(
+                part, seg.cb.p, seg.J, a.constant, a.jconst, nullptr, bd);
+        }
+        VG_CHECK_LAUNCH();
+        VG_CUDA(cudaMemcpyAsync(hlive + slot, live + slot, sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                ctx->stream));
+    };
+    struct Events { // released on every path
+        cudaEvent_t e[6] = {};
+        ~Events() {
+            for (auto x : e)
+                if (x) cudaEventDestroy(x);
+        }
+    } ev; // per slot: live count read back, sweep begin, sweep end
+    for (int k = 0; k < 6; k++)
+        VG_CUDA(cudaEventCreateWithFlags(&ev.e[k], k < 2 || !sweep_ms ? cudaEventDisableTiming
+                                                                      : cudaEventDefault));
+    if (sweep_ms) *sweep_ms = 0.0;
+    for (int32_t it = 1;; it++) {
+        const int slot = it & 1, pi = (it - 1) % 3; // past <- curr <- target <- past (louvain.cpp:565-570)
+        enqueue(pi, it, slot, sweep_ms ? ev.e[2 + slot] : nullptr, sweep_ms ? ev.e[4 + slot] : nullptr);
+        VG_CUDA(cudaEventRecord(ev.e[slot], ctx->stream));
+        if (it == 1) continue;
+        const int before = slot ^ 1;
+        VG_CUDA(cudaEventSynchronize(ev.e[before]));
+        if (sweep_ms) {
+            float ms = 0.f;
+            VG_CUDA(cudaEventElapsedTime(&ms, ev.e[2 + before], ev.e[4 + before]));
+            *sweep_ms += ms;
+        }
+        if (hlive[before] == 0) return it - 1;
+    }
+}
+
+constexpr int64_t AHEAD_MAX_NE = 1 << 22;
+
 // the phase proper; returns the communities in g->comm
 // max_iters > 0 stops after that many iterations (the autotuner's timing runs)
 static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double *mod_out,
@@ -2413,6 +2499,61 @@ static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double
     const int agrid = seg_grid(ctx, seg.C);
     DevBuf<double> modv(ctx, 4);
     double *hmod = (double *)vg_pinned(ctx, 4 * sizeof(double));
+
+    // Plain phases of middling graphs: the loop test on the device, iterations enqueued ahead
+    // (300,007 vertices / 2.8e6 entries, 20 iterations: 1.46 -> 1.24 ms). Larger ones lose
+    // more by every block's look at the flag than the host's gaps cost (348,203 / 6.5e6:
+    // 1.41 -> 1.56 ms; 12,071 / 4.4e6: 0.86 -> 0.89).
+    if (ordering == 0 && et == 0 && max_iters == 0 && nv && g->ne <= AHEAD_MAX_NE) {
+        struct State { // of the loop test, one 8-byte word each
+            double prev_mod, lower, thresh;
+            int64_t iters, live, done, resbuf;
+        };
+        State h{p->lower, p->lower, p->threshold, 0, 0, 0, 0};
+        // past the words `iterate` reads back
+        State *staged = reinterpret_cast<State *>((char *)vg_pinned(ctx, 64 + sizeof(State)) + 64);
+        *staged = h;
+        DevBuf<State> st(ctx, 1);
+        VG_CUDA(cudaMemcpyAsync(st.p, staged, sizeof(State), cudaMemcpyHostToDevice, ctx->stream));
+        SweepArgs a{};
+        a.rowptr = g->rowptr;
+        a.tail = g->tail;
+        a.weight = g->weight;
+        a.vdeg = vdeg.p;
+        a.cdeg = cdeg.p;
+        a.csize = csize.p;
+        a.cupd = cupd.p;
+        a.cw = cw.p;
+        a.ref = g->ref;
+        a.noprune = noprune.p;
+        a.ne = g->ne;
+        a.constant = constant;
+        BatchDecide bd{};
+        bd.prev_mod = &st.p->prev_mod;
+        bd.lower = &st.p->lower;
+        bd.thresh = &st.p->thresh;
+        bd.iters = reinterpret_cast<int32_t *>(&st.p->iters);
+        bd.live_count = reinterpret_cast<int32_t *>(&st.p->live); // two of them
+        bd.done = reinterpret_cast<uint8_t *>(&st.p->done);
+        bd.resbuf = reinterpret_cast<int8_t *>(&st.p->resbuf);
+        a.stop = bd.done;
+        int32_t *bufs[3] = {A.p, B.p, C.p};
+        double ms = 0.0;
+        const int32_t its = iterate(ctx, a, bd, bufs, bk, hp, seg, nv, cdeg.p, csize.p, part.p,
+                                    noprune.p, timing ? &ms : nullptr);
+        VG_CUDA(cudaMemcpyAsync(staged, st.p, sizeof(State), cudaMemcpyDeviceToHost, ctx->stream));
+        vg_sync(ctx);
+        if (timing) {
+            timing->sweep_ms = ms;
+            timing->edges = g->ne * its;
+        }
+        *mod_out = staged->prev_mod;
+        *iters_out = its;
+        vg_free(ctx, g->comm, sizeof(int32_t) * nv);
+        DevBuf<int32_t> *held[3] = {&A, &B, &C};
+        g->comm = held[*reinterpret_cast<const int8_t *>(&staged->resbuf)]->detach();
+        return;
+    }
 
     int32_t *past = A.p, *curr = B.p, *target = C.p;
     double *pcurr = pA.p, *pprev = pB.p;
@@ -2592,7 +2733,6 @@ void vg_phase_batch_internal(vg_ctx *ctx, vg_graph *U, int64_t J, const int64_t 
     HubPlan hp;
     plan_hubs(ctx, U, bk, 1, hp);
     DevBuf<double> part(ctx, 3 * std::max<int64_t>(seg.C, 1));
-    const int agrid = seg_grid(ctx, seg.C);
     // per-graph loop state
     DevBuf<double> prev_mod(ctx, J), lower(ctx, J), thresh(ctx, J);
     DevBuf<int32_t> iters(ctx, J), live(ctx, 2);
@@ -2604,90 +2744,32 @@ void vg_phase_batch_internal(vg_ctx *ctx, vg_graph *U, int64_t J, const int64_t 
     VG_CUDA(cudaMemsetAsync(iters.p, 0, sizeof(int32_t) * J, ctx->stream));
     VG_CUDA(cudaMemsetAsync(done.p, 0, J, ctx->stream));
     VG_CUDA(cudaMemsetAsync(resbuf.p, 0, J, ctx->stream));
-    // Two iterations are in flight: the next one is enqueued before the live count of the
-    // one before is waited for, so the device never waits for the host (after the last
-    // iteration every graph is done and the extra one's launches return at once). Enqueued
-    // directly: capturing an iteration as a graph cost 1.2-1.5 ms a phase, more than its
-    // replays saved (48 graphs of 1,000-256,000 vertices: phases 26.5 -> 17.0 ms).
-    int32_t *hlive = (int32_t *)vg_pinned(ctx, 2 * sizeof(int32_t));
+    SweepArgs a{};
+    a.rowptr = U->rowptr;
+    a.tail = U->tail;
+    a.weight = U->weight;
+    a.vdeg = vdeg.p;
+    a.cdeg = cdeg.p;
+    a.csize = csize.p;
+    a.cupd = cupd.p;
+    a.cw = cw.p;
+    a.ref = U->ref;
+    a.noprune = noprune.p;
+    a.ne = U->ne;
+    a.constant = 0.0;
+    a.vjob = vjob;
+    a.jconst = jconst.p;
+    a.jdone = done.p;
+    BatchDecide bd{};
+    bd.prev_mod = prev_mod.p;
+    bd.lower = lower.p;
+    bd.thresh = thresh.p;
+    bd.iters = iters.p;
+    bd.done = done.p;
+    bd.resbuf = resbuf.p;
+    bd.live_count = live.p;
     int32_t *bufs[3] = {B0.p, B1.p, B2.p};
-    // iteration `it` with bufs[pi] = past, bufs[pi+1] = curr, bufs[pi+2] = target; its live
-    // count lands in hlive[slot]
-    auto enqueue = [&](int pi, int32_t it, int slot, cudaEvent_t e0, cudaEvent_t e1) {
-        SweepArgs a{};
-        a.rowptr = U->rowptr;
-        a.tail = U->tail;
-        a.weight = U->weight;
-        a.curr = bufs[(pi + 1) % 3];
-        a.target = bufs[(pi + 2) % 3];
-        a.vdeg = vdeg.p;
-        a.cdeg = cdeg.p;
-        a.csize = csize.p;
-        a.cupd = cupd.p;
-        a.cw = cw.p;
-        a.ref = U->ref;
-        a.noprune = noprune.p;
-        a.ne = U->ne;
-        a.constant = 0.0;
-        a.vjob = vjob;
-        a.jconst = jconst.p;
-        a.jdone = done.p;
-        VG_CUDA(cudaMemsetAsync(live.p + slot, 0, sizeof(int32_t), ctx->stream));
-        if (e0) VG_CUDA(cudaEventRecord(e0, ctx->stream));
-        sweep_color(ctx, a, bk, 0, hp, true, nv);
-        if (e1) VG_CUDA(cudaEventRecord(e1, ctx->stream));
-        {
-            LaunchTimer lt(ctx);
-            k_apply_seg<<<agrid, SEG_THREADS, 0, ctx->stream>>>(seg.voff.p, seg.cb.p, J, seg.C,
-                                                                cdeg.p, csize.p, cupd.p, cw.p,
-                                                                nullptr, done.p, 1, part.p,
-                                                                noprune.p);
-        }
-        VG_CHECK_LAUNCH();
-        BatchDecide bd;
-        bd.prev_mod = prev_mod.p;
-        bd.lower = lower.p;
-        bd.thresh = thresh.p;
-        bd.iters = iters.p;
-        bd.done = done.p;
-        bd.resbuf = resbuf.p;
-        bd.live_count = live.p + slot;
-        bd.iter = it;
-        bd.past_idx = pi;
-        {
-            LaunchTimer lt(ctx);
-            k_mod_seg<<<(int)std::min<int64_t>(J, 65535), SEG_FINAL, 0, ctx->stream>>>(
-                part.p, seg.cb.p, J, 0.0, jconst.p, nullptr, bd);
-        }
-        VG_CHECK_LAUNCH();
-        VG_CUDA(cudaMemcpyAsync(hlive + slot, live.p + slot, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                ctx->stream));
-    };
-    struct Events { // released on every path
-        cudaEvent_t e[6] = {};
-        ~Events() {
-            for (auto x : e)
-                if (x) cudaEventDestroy(x);
-        }
-    } ev; // per slot: live count read back, sweep begin, sweep end
-    for (int k = 0; k < 6; k++)
-        VG_CUDA(cudaEventCreateWithFlags(&ev.e[k], k < 2 || !sweep_ms ? cudaEventDisableTiming
-                                                                      : cudaEventDefault));
-    if (sweep_ms) *sweep_ms = 0.0;
-    for (int32_t it = 1;; it++) {
-        const int slot = it & 1, pi = (it - 1) % 3; // past <- curr <- target <- past (louvain.cpp:565-570)
-        enqueue(pi, it, slot, sweep_ms ? ev.e[2 + slot] : nullptr, sweep_ms ? ev.e[4 + slot] : nullptr);
-        VG_CUDA(cudaEventRecord(ev.e[slot], ctx->stream));
-        if (it == 1) continue;
-        const int before = slot ^ 1;
-        VG_CUDA(cudaEventSynchronize(ev.e[before]));
-        if (sweep_ms) {
-            float ms = 0.f;
-            VG_CUDA(cudaEventElapsedTime(&ms, ev.e[2 + before], ev.e[4 + before]));
-            *sweep_ms += ms;
-        }
-        if (hlive[before] == 0) break;
-    }
+    iterate(ctx, a, bd, bufs, bk, hp, seg, nv, cdeg.p, csize.p, part.p, noprune.p, sweep_ms);
     vg_sync(ctx);
     vg_free(ctx, U->comm, sizeof(int32_t) * nv);
     U->comm = nullptr;
