@@ -47,16 +47,23 @@ __global__ void k_sizes(const int32_t *__restrict__ c, int64_t n, unsigned long 
 }
 
 // sum of size (size - 1) / 2 over an array of counts
+// and the largest size
 __global__ void k_pairs(const unsigned long long *__restrict__ size, int64_t n,
-                        unsigned long long *__restrict__ out) {
-    unsigned long long s = 0;
+                        unsigned long long *__restrict__ out,
+                        unsigned long long *__restrict__ largest) {
+    unsigned long long s = 0, m = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const unsigned long long x = size[i];
         s += x * (x - (x ? 1 : 0)) / 2;
+        m = max(m, x);
     }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_down_sync(0xffffffffu, s, o);
+        m = max(m, __shfl_down_sync(0xffffffffu, m, o));
+    }
     if ((threadIdx.x & 31) == 0 && s) atomicAdd(out, s);
+    if ((threadIdx.x & 31) == 0) atomicMax(largest, m);
 }
 
 __global__ void k_pair_keys(const int32_t *__restrict__ a, const int32_t *__restrict__ b, int64_t n,
@@ -111,27 +118,23 @@ int bits_for(uint64_t x) {
     return b;
 }
 
-unsigned long long read_u64(vg_ctx *ctx, const unsigned long long *d) {
-    unsigned long long *h = (unsigned long long *)vg_pinned(ctx, sizeof(unsigned long long));
-    VG_CUDA(cudaMemcpyAsync(h, d, sizeof(unsigned long long), cudaMemcpyDeviceToHost, ctx->stream));
-    vg_sync(ctx);
-    return *h;
-}
-
-// compute_gini_coeff (compare.cpp:287-318) from exact sums; numColors is the
-// reference's int argument
-double gini_of(vg_ctx *ctx, const unsigned long long *size, int64_t nc, int64_t n) {
+// the numerator of compute_gini_coeff (compare.cpp:287-318), an exact sum, to *num; no size
+// is greater than `largest`, so the sort takes that many bits
+void gini_num(vg_ctx *ctx, const unsigned long long *size, int64_t nc, uint64_t largest,
+              unsigned long long *num) {
     DevBuf<uint64_t> keys(ctx, nc);
     DevBuf<uint32_t> vals(ctx, nc);
     const int grid = vg_grid(ctx, nc, 256);
     { LaunchTimer lt(ctx); k_size_keys<<<grid, 256, 0, ctx->stream>>>(size, nc, keys.p, vals.p); }
     VG_CHECK_LAUNCH();
-    vg_radix_sort_pairs(ctx, keys.p, vals.p, nc, bits_for((uint64_t)n));
-    DevBuf<unsigned long long> num(ctx, 1);
-    VG_CUDA(cudaMemsetAsync(num.p, 0, sizeof(unsigned long long), ctx->stream));
-    { LaunchTimer lt(ctx); k_gini_num<<<grid, 256, 0, ctx->stream>>>(keys.p, nc, num.p); }
+    vg_radix_sort_pairs(ctx, keys.p, vals.p, nc, bits_for(largest));
+    { LaunchTimer lt(ctx); k_gini_num<<<grid, 256, 0, ctx->stream>>>(keys.p, nc, num); }
     VG_CHECK_LAUNCH();
-    const double numFunc = (double)read_u64(ctx, num.p);
+}
+
+// the coefficient; numColors is the reference's int argument
+double gini_of(unsigned long long num, int64_t nc, int64_t n) {
+    const double numFunc = (double)num;
     const double denFunc = (double)n;
     const int numColors = (int)nc;
     return ((2 * numFunc) / (numColors * denFunc)) - ((double)(numColors + 1) / (double)numColors);
@@ -149,10 +152,11 @@ extern "C" vg_status vg_compare_communities(vg_ctx *ctx, int64_t n, const int64_
         DevBuf<int64_t> wide(ctx, n);
         DevBuf<int32_t> a(ctx, n), b(ctx, n);
         DevBuf<int> bad(ctx, 1);
-        DevBuf<unsigned long long> mx(ctx, 2), cnt(ctx, 3);
+        // per vector the largest label; pairs1, pairs2, same pairs, largest sizes, gini numerators
+        DevBuf<unsigned long long> mx(ctx, 2), cnt(ctx, 7);
         VG_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), ctx->stream));
         VG_CUDA(cudaMemsetAsync(mx.p, 0, 2 * sizeof(unsigned long long), ctx->stream));
-        VG_CUDA(cudaMemsetAsync(cnt.p, 0, 3 * sizeof(unsigned long long), ctx->stream));
+        VG_CUDA(cudaMemsetAsync(cnt.p, 0, 7 * sizeof(unsigned long long), ctx->stream));
         const int64_t *src[2] = {c1, c2};
         int32_t *dst[2] = {a.p, b.p};
         for (int k = 0; k < 2; k++) {
@@ -180,10 +184,10 @@ extern "C" vg_status vg_compare_communities(vg_ctx *ctx, int64_t n, const int64_
         { LaunchTimer lt(ctx); k_sizes<<<grid, 256, 0, ctx->stream>>>(b.p, n, s2.p); }
         VG_CHECK_LAUNCH();
         { LaunchTimer lt(ctx);
-          k_pairs<<<vg_grid(ctx, nc1, 256), 256, 0, ctx->stream>>>(s1.p, nc1, cnt.p + 0); }
+          k_pairs<<<vg_grid(ctx, nc1, 256), 256, 0, ctx->stream>>>(s1.p, nc1, cnt.p + 0, cnt.p + 3); }
         VG_CHECK_LAUNCH();
         { LaunchTimer lt(ctx);
-          k_pairs<<<vg_grid(ctx, nc2, 256), 256, 0, ctx->stream>>>(s2.p, nc2, cnt.p + 1); }
+          k_pairs<<<vg_grid(ctx, nc2, 256), 256, 0, ctx->stream>>>(s2.p, nc2, cnt.p + 1, cnt.p + 4); }
         VG_CHECK_LAUNCH();
         {
             DevBuf<uint64_t> keys(ctx, n);
@@ -195,11 +199,17 @@ extern "C" vg_status vg_compare_communities(vg_ctx *ctx, int64_t n, const int64_
             { LaunchTimer lt(ctx); k_run_pairs<<<grid, 256, 0, ctx->stream>>>(keys.p, n, cnt.p + 2); }
             VG_CHECK_LAUNCH();
         }
-        unsigned long long *hc = (unsigned long long *)vg_pinned(ctx, 3 * sizeof(unsigned long long));
-        VG_CUDA(cudaMemcpyAsync(hc, cnt.p, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+        unsigned long long *hc = (unsigned long long *)vg_pinned(ctx, 7 * sizeof(unsigned long long));
+        VG_CUDA(cudaMemcpyAsync(hc, cnt.p, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                                 ctx->stream));
         vg_sync(ctx);
         const int64_t pairs1 = (int64_t)hc[0], pairs2 = (int64_t)hc[1], ss = (int64_t)hc[2];
+        const uint64_t largest[2] = {hc[3], hc[4]};
+        gini_num(ctx, s1.p, nc1, largest[0], cnt.p + 5);
+        gini_num(ctx, s2.p, nc2, largest[1], cnt.p + 6);
+        VG_CUDA(cudaMemcpyAsync(hc + 5, cnt.p + 5, 2 * sizeof(unsigned long long),
+                                cudaMemcpyDeviceToHost, ctx->stream));
+        vg_sync(ctx);
         vg_compare_stats r{};
         r.n = n;
         r.nc1 = nc1;
@@ -211,8 +221,8 @@ extern "C" vg_status vg_compare_communities(vg_ctx *ctx, int64_t n, const int64_
         r.precision = (double)r.same_same / (double)(r.same_same + r.diff_same);
         r.recall = (double)r.same_same / (double)(r.same_same + r.same_diff);
         r.fscore = 2.0 * ((r.precision * r.recall) / (r.precision + r.recall));
-        r.gini1 = gini_of(ctx, s1.p, nc1, n);
-        r.gini2 = gini_of(ctx, s2.p, nc2, n);
+        r.gini1 = gini_of(hc[5], nc1, n);
+        r.gini2 = gini_of(hc[6], nc2, n);
         *out = r;
     });
 }
