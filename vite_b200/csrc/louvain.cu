@@ -121,6 +121,8 @@ struct SweepArgs {
     const int32_t *__restrict__ vjob = nullptr;
     const double *__restrict__ jconst = nullptr;
     const uint8_t *__restrict__ jdone = nullptr;
+    // (coloured sweeps, else null) set to 1 for each community the sweep's moves touch
+    uint8_t *__restrict__ touched = nullptr;
     // one graph: set once its phase has ended, so that an iteration enqueued ahead of that
     // returns at once (null: not looked at)
     const uint8_t *__restrict__ stop = nullptr;
@@ -439,6 +441,10 @@ __device__ __forceinline__ void commit_vertex(const A &a, int32_t v, int32_t cc,
         atomicAdd(&a.cupd[tgt].size, 1);
         atomicAdd(&a.cupd[cc].deg, -vd);
         atomicAdd(&a.cupd[cc].size, -1);
+        if (a.touched) {
+            a.touched[tgt] = 1;
+            a.touched[cc] = 1;
+        }
     }
 }
 
@@ -1666,6 +1672,38 @@ __global__ void __launch_bounds__(SEG_THREADS) k_apply_seg(
     }
 }
 
+// The update between two colors (louvain.cpp:724-735): the communities marked as touched
+// only, 16 marks per load (k_apply_seg reads every community's 16-byte update: 39 us per color
+// on 4.2 million communities, 19 us here). touched: 16-byte aligned, padded to 16.
+__global__ void k_apply_touched(int64_t nv, uint8_t *__restrict__ touched, double *__restrict__ cdeg,
+                                int32_t *__restrict__ csize, CommInfo *__restrict__ cupd,
+                                int32_t *__restrict__ noprune) {
+    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g * 16 < nv;
+         g += (int64_t)gridDim.x * blockDim.x) {
+        uint4 *at = reinterpret_cast<uint4 *>(touched) + g;
+        const uint4 m = *at;
+        if (!(m.x | m.y | m.z | m.w)) continue;
+        *at = make_uint4(0, 0, 0, 0);
+        const uint32_t w[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            for (uint32_t bits = w[q]; bits; bits &= bits - 1) { // each mark is a byte of 1
+                const int64_t i = g * 16 + q * 4 + ((__ffs(bits) - 1) >> 3);
+                const CommInfo u = cupd[i];
+                const double cd = __dadd_rn(cdeg[i], u.deg);
+                const int32_t ns = csize[i] + u.size;
+                cdeg[i] = cd;
+                csize[i] = ns;
+                if (ns > 0 && !(cd >= 0.0)) *noprune = 1; // see k_apply_seg
+                CommInfo z;
+                z.deg = 0.0;
+                z.size = 0;
+                z.pad = 0;
+                cupd[i] = z;
+            }
+    }
+}
+
 // per-graph phase state of a batch: the loop test of distLouvainMethod
 // (louvain.cpp:553-563) evaluated for every graph on the device
 struct BatchDecide {
@@ -2555,6 +2593,11 @@ static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double
         return;
     }
 
+    DevBuf<uint8_t> touched; // communities the current color's sweep moves vertices in or out of
+    if (ordering == 1 && nv) {
+        touched.alloc(ctx, (nv + 15) / 16 * 16);
+        VG_CUDA(cudaMemsetAsync(touched.p, 0, touched.n, ctx->stream));
+    }
     int32_t *past = A.p, *curr = B.p, *target = C.p;
     double *pcurr = pA.p, *pprev = pB.p;
     double prevMod = p->lower, currMod = -1.0;
@@ -2584,18 +2627,20 @@ static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double
         a.noprune = noprune.p;
         a.ne = g->ne;
         a.ident = numIters == 1 ? 1 : 0; // k_init put every vertex in its own community
+        a.touched = touched.p;
         a.constant = constant;
         if (timing) VG_CUDA(cudaEventRecord(ev0, ctx->stream));
         for (int64_t ci = 0; ci < numColor; ci++) {
             sweep_color(ctx, a, bk, ci, hp, ordering == 0, nv);
-            if (ordering == 1 && nv) { // per-color community update (louvain.cpp:724-735)
+            // per-color community update; the last color's has the sums (below)
+            if (ordering == 1 && nv && ci + 1 < numColor) {
                 LaunchTimer lt(ctx);
-                k_apply_seg<<<agrid, SEG_THREADS, 0, ctx->stream>>>(
-                    seg.voff.p, seg.cb.p, 1, seg.C, cdeg.p, csize.p, cupd.p, cw.p, a.active,
-                    nullptr, 0, part.p, noprune.p);
+                k_apply_touched<<<vg_grid(ctx, touched.n / 16, 256), 256, 0, ctx->stream>>>(
+                    nv, touched.p, cdeg.p, csize.p, cupd.p, noprune.p);
                 VG_CHECK_LAUNCH();
             }
         }
+        if (touched.p) VG_CUDA(cudaMemsetAsync(touched.p, 0, touched.n, ctx->stream));
         if (timing) VG_CUDA(cudaEventRecord(ev1, ctx->stream));
         if (nv) {
             {
