@@ -260,6 +260,13 @@ def run_reference_arm(args, rank: int, ws: int) -> None:
     print(json.dumps(line), flush=True)
 
 
+def reference_built() -> bool:
+    """Whether the compiled reference (oracle/_ref) is here to be timed and compared with."""
+    from oracle import vite_oracle as vo
+
+    return os.path.exists(vo.HARNESS)
+
+
 def reference_levels(path: str, flags: list, threads: int) -> tuple[list, dict]:
     """One reference run (oracle/_ref, all host threads) on a Vite binary file: its
     recorded levels and its totals."""
@@ -604,7 +611,7 @@ def run_ba_config(ctx, stream, args) -> dict:
                        "modularity": s["modularity"], "colors": s["num_colors"],
                        "color_s": s["seconds_color"], "phase_s": s["seconds_phase"],
                        "rebuild_s": s["seconds_rebuild"]} for s in dev.stats]}
-    if not args.no_cpu_baseline:
+    if not args.no_cpu_baseline and reference_built():
         threads = os.cpu_count() or 1
         with tempfile.TemporaryDirectory() as tmp:
             path = os.path.join(tmp, "ba.bin")
@@ -735,7 +742,7 @@ def main() -> None:
         traffic = tj.get("dram_bytes_per_sweep_level0")
 
     cpu, parity = None, None
-    if rank == 0 and ws == 1 and not args.no_cpu_baseline:
+    if rank == 0 and ws == 1 and not args.no_cpu_baseline and reference_built():
         # the reference (oracle/_ref, all host threads) once on the whole benchmark graph,
         # read from a Vite binary file: its time is the CPU baseline, its levels and -o map
         # are compared with ours

@@ -207,7 +207,8 @@ vg_status vg_vertex_degree_noalloc(int64_t nv, const int64_t *d_rowptr, const do
  * per SM of the degree <= 16 sweep in vertex order. Every class folds a vertex's
  * counters in CSR order except the two CTA-based ones, whose slices meet through
  * FP64 atomics: with unit or integral weights any setting gives the same bits, with
- * real weights results agree to the last few bits. */
+ * real weights results agree to the last few bits. The phases of small graphs (at most
+ * 524,288 vertices and 2^21 entries) run in one launch that does not use it. */
 typedef struct vg_tuning {
     int32_t t32;       /* 0 or 1 */
     int32_t ws_max;    /* 32..128 */

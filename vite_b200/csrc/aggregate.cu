@@ -8,8 +8,10 @@
 //   2. each segment is reduced by c2 with every sum a left fold in segment order,
 //      giving the reference's sums bit for bit: one warp per segment folds its
 //      entries into a shared-memory hash table in order and sorts the distinct
-//      keys; segments with more than 256 distinct keys go through one stable radix
-//      sort of all their entries by (segment, c2) and each run is folded in order;
+//      keys; segments with more than 256 distinct keys, or of more entries than a warp
+//      should take, get a block each; those past the blocks' tables (4,096 keys,
+//      131,072 entries) go through one stable radix sort of all their entries by
+//      (segment, c2) and each run is folded in order;
 //   3. the unique entries are compacted into the next CSR.
 #include "grid_sync.cuh"
 #include "vg_internal.cuh"
@@ -241,11 +243,11 @@ __device__ __forceinline__ void sort_lanes(int32_t &key, double &val, bool narro
 // chunk the lanes holding the same key elect the lowest as leader, which adds its
 // peers' weights in lane order onto the key's running sum in a shared-memory
 // table, so every sum is the left fold in segment order. Only the distinct keys
-// are then sorted: in registers across the warp when there are at most 32 of
-// them, else in shared memory. The reduction runs in two tiers: first every segment
-// with a small table (MAXU_S distinct keys at most, so more warps fit per SM), then
-// the segments that overflowed it with a large one (MAXU_L); a segment with more
-// than MAXU_L distinct keys is flagged for the sorted path.
+// are then sorted, in registers across the warp (through shared memory the sort was
+// the largest part of a segment of 100-256 keys). The reduction runs in tiers: first
+// every segment with a small table (MAXU_S distinct keys at most, so more warps fit per
+// SM), then the segments that overflowed it with a large one (MAXU_L), then a block per
+// segment (k_rows_block).
 #ifndef VG_RH_GRID
 #define VG_RH_GRID 3 // CTAs per SM in the grid of the large-table tier
 #endif
@@ -668,7 +670,7 @@ __global__ void k_list_flagged(int64_t nc, const int32_t *__restrict__ flag,
         if (flag[r]) rows[pos[r]] = (int32_t)r;
 }
 
-// Segments with more than H_MAXU distinct keys, all together: every entry becomes the key
+// Segments past the blocks' tables, all together: every entry becomes the key
 // (segment rank << kbits | neighbour key) with its index in the grouped arrays as
 // payload; one stable radix sort over all of them puts each (segment, key) run in
 // segment order, and the run is folded left to right.
@@ -1070,7 +1072,7 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
                       integral, nullptr, nullptr, flag.p); }
             VG_CHECK_LAUNCH();
         }
-        // segments with more than H_MAXU distinct keys: one global stable sort. Their
+        // segments past the blocks' tables: one global stable sort. Their
         // count, entries and chunks are scanned on the device and read back together.
         DevBuf<int64_t> bigidx(ctx, nc), boff(ctx, nc), cb(ctx, nc), tot(ctx, 4);
         { LaunchTimer lt(ctx);

@@ -10,6 +10,7 @@
 //              fused: deltas folded into the community info while the two sums
 //              of the modularity are reduced deterministically;
 //   swap       pointer rotation (plain) or the early-termination swaps.
+// Small graphs run all of a phase in one launch instead (phase_small.cuh).
 // Arithmetic follows the reference's expression order with explicit
 // round-to-nearest intrinsics, so no multiply-add is ever fused.
 #include "grid_sync.cuh"
