@@ -418,7 +418,7 @@ __device__ __forceinline__ int warp_segment(HashWarpSmem<CAP, MAXU> &S, int64_t 
 constexpr int64_t BLOCK_SMALL_L = 8192, BLOCK_LARGE_L = 131072;
 struct BlockRows {
     int32_t *rows[2] = {nullptr, nullptr};
-    int32_t *count = nullptr; // 2
+    int32_t *count = nullptr; // 2, then the rows of each list taken so far
 };
 
 // rows: null for every segment 0..nc-1, else the segments rows[0 .. *nrows)
@@ -643,11 +643,17 @@ __global__ void __launch_bounds__(Table::THREADS) k_rows_block(
     const int64_t *__restrict__ rstart, const int32_t *__restrict__ gk,
     const double *__restrict__ gw, int32_t *__restrict__ uk, double *__restrict__ uw,
     int64_t *__restrict__ ucount, int integral, int32_t *__restrict__ out,
-    int32_t *__restrict__ n_out, int32_t *__restrict__ flag) {
+    int32_t *__restrict__ n_out, int32_t *__restrict__ flag, int32_t *__restrict__ taken) {
     extern __shared__ unsigned char hsm_raw[];
+    __shared__ int s_next;
     Table &T = *reinterpret_cast<Table *>(hsm_raw);
     const int n = *n_in;
-    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    for (;;) { // the next row to whichever block is free: their lengths differ a hundredfold
+        __syncthreads();
+        if (threadIdx.x == 0) s_next = atomicAdd(taken, 1);
+        __syncthreads();
+        const int i = s_next;
+        if (i >= n) break;
         const int32_t row = in[i];
         const int64_t s0 = rstart[row], L = rstart[row + 1] - s0;
         const int U = block_segment<false>(T, s0, L, integral != 0, gk, gw, uk, uw, s0);
@@ -1038,12 +1044,12 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
             // the segments that overflowed the small table, with the large one (their
             // count stays on the device; the grid covers every segment's warp)
             DevBuf<int64_t> fpos(ctx, nc), fcount(ctx, 1);
-            DevBuf<int32_t> frows(ctx, nc), brows(ctx, 2 * nc + 2);
+            DevBuf<int32_t> frows(ctx, nc), brows(ctx, 2 * nc + 4);
             BlockRows next;
             next.rows[0] = brows.p;
             next.rows[1] = brows.p + nc;
             next.count = brows.p + 2 * nc;
-            VG_CUDA(cudaMemsetAsync(next.count, 0, 2 * sizeof(int32_t), ctx->stream));
+            VG_CUDA(cudaMemsetAsync(next.count, 0, 4 * sizeof(int32_t), ctx->stream));
             vg_scan_i32_async(ctx, flag.p, fpos.p, nc, fcount.p);
             { LaunchTimer lt(ctx);
               k_list_flagged<<<vg_grid(ctx, nc, 256), 256, 0, ctx->stream>>>(nc, flag.p, fpos.p,
@@ -1062,14 +1068,14 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
               k_rows_block<BlockTableSmall>
                   <<<bgrid, BlockTableSmall::THREADS, sizeof(BlockTableSmall), ctx->stream>>>(
                       next.rows[0], next.count, rstart.p, gk.p, gw.p, uk.p, uw.p, ucount.p, integral,
-                      next.rows[1], next.count + 1, nullptr); }
+                      next.rows[1], next.count + 1, nullptr, next.count + 2); }
             VG_CHECK_LAUNCH();
             { LaunchTimer lt(ctx);
               k_rows_block<BlockTableLarge>
                   <<<(int)std::min<int64_t>(nc, ctx->sm_count), BlockTableLarge::THREADS,
                      sizeof(BlockTableLarge), ctx->stream>>>(
                       next.rows[1], next.count + 1, rstart.p, gk.p, gw.p, uk.p, uw.p, ucount.p,
-                      integral, nullptr, nullptr, flag.p); }
+                      integral, nullptr, nullptr, flag.p, next.count + 3); }
             VG_CHECK_LAUNCH();
         }
         // segments past the blocks' tables: one global stable sort. Their
