@@ -1206,6 +1206,8 @@ vg_graph *vg_rebuild_small(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) 
     const size_t n = (size_t)nv, e = (size_t)ne, nb = (size_t)blocks;
     const size_t wide = 6 * (n + 1) + 3 * nb + 2 * e;
     const size_t narrow = 9 * n + RS_CTL + 1 + 2 * e;
+    // with what the next level may take beside it
+    if (!vg_has_room(ctx, 8 * wide + 4 * narrow + 12 * e + 16 * (n + 1))) return nullptr;
     DevBuf<unsigned char> scratch(ctx, 8 * wide + 4 * narrow);
     int64_t *w8 = (int64_t *)scratch.p;
     int32_t *w4 = (int32_t *)(scratch.p + 8 * wide);

@@ -250,7 +250,7 @@ int64_t vg_color_internal(vg_ctx *ctx, vg_graph *g, int64_t nHash, int32_t targe
     // 3,000 vertices 205 -> 219 us).
     DevBuf<uint32_t> hash;
     const size_t words = (size_t)nv * (nHash <= 4 ? 4 : 8);
-    if (nHash <= 8 && g->ne >= COLOR_HASH_NE && (!ctx->budget || ctx->in_use + sizeof(uint32_t) * words <= ctx->budget))
+    if (nHash <= 8 && g->ne >= COLOR_HASH_NE && vg_has_room(ctx, sizeof(uint32_t) * words))
         hash.alloc(ctx, words);
     uint32_t seed = 1012; // coloring.cpp:60
     int64_t nextColor = 0, lastCount = 0, currentCount = 0;

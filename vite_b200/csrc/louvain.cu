@@ -2326,6 +2326,7 @@ static bool run_phase_small(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, 
     const size_t doubles = 3 * n + 3 * units + (et ? n : 0) + (et24 ? 2 * n : 0);
     const size_t bytes = sizeof(CommInfo) * n + sizeof(double) * doubles +
                          sizeof(int32_t) * (5 * n + ctl_words + 1) + (et ? n : 0);
+    if (!vg_has_room(ctx, bytes + sizeof(int32_t) * n)) return false;
     DevBuf<unsigned char> scratch(ctx, bytes);
     DevBuf<int32_t> comm(ctx, nv);
     unsigned char *at = scratch.p;
@@ -2595,7 +2596,7 @@ static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double
     }
 
     DevBuf<uint8_t> touched; // communities the current color's sweep moves vertices in or out of
-    if (ordering == 1 && nv) {
+    if (ordering == 1 && nv && vg_has_room(ctx, nv + 16)) {
         touched.alloc(ctx, (nv + 15) / 16 * 16);
         VG_CUDA(cudaMemsetAsync(touched.p, 0, touched.n, ctx->stream));
     }
@@ -2636,8 +2637,13 @@ static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double
             // per-color community update; the last color's has the sums (below)
             if (ordering == 1 && nv && ci + 1 < numColor) {
                 LaunchTimer lt(ctx);
-                k_apply_touched<<<vg_grid(ctx, touched.n / 16, 256), 256, 0, ctx->stream>>>(
-                    nv, touched.p, cdeg.p, csize.p, cupd.p, noprune.p);
+                if (!touched.p)
+                    k_apply_seg<<<agrid, SEG_THREADS, 0, ctx->stream>>>(
+                        seg.voff.p, seg.cb.p, 1, seg.C, cdeg.p, csize.p, cupd.p, cw.p, a.active,
+                        nullptr, 0, part.p, noprune.p);
+                else
+                    k_apply_touched<<<vg_grid(ctx, touched.n / 16, 256), 256, 0, ctx->stream>>>(
+                        nv, touched.p, cdeg.p, csize.p, cupd.p, noprune.p);
                 VG_CHECK_LAUNCH();
             }
         }

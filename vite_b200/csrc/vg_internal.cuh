@@ -84,6 +84,11 @@ void vg_side_join(vg_ctx *ctx, int n);
 
 // stream-ordered device allocation accounted against the context budget
 void *vg_alloc(vg_ctx *ctx, size_t bytes);
+// whether the context's budget has room for `bytes` more (a path that trades memory for time
+// asks, and takes the leaner one otherwise)
+inline bool vg_has_room(const vg_ctx *ctx, size_t bytes) {
+    return !ctx->budget || ctx->in_use + bytes <= ctx->budget;
+}
 void vg_free(vg_ctx *ctx, void *p, size_t bytes);
 
 template <class T> struct DevBuf {
