@@ -1208,7 +1208,8 @@ vg_graph *vg_rebuild_small(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) 
     const size_t narrow = 9 * n + RS_CTL + 1 + 2 * e;
     // with what the next level may take beside it
     if (!vg_has_room(ctx, 8 * wide + 4 * narrow + 12 * e + 16 * (n + 1))) return nullptr;
-    DevBuf<unsigned char> scratch(ctx, 8 * wide + 4 * narrow);
+    DevBuf<unsigned char> scratch;
+    if (!scratch.try_alloc(ctx, 8 * wide + 4 * narrow)) return nullptr;
     int64_t *w8 = (int64_t *)scratch.p;
     int32_t *w4 = (int32_t *)(scratch.p + 8 * wide);
     auto take8 = [&](size_t k) { int64_t *q = w8; w8 += k; return q; };
@@ -1245,9 +1246,13 @@ vg_graph *vg_rebuild_small(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) 
         vg_throw(VG_ERR_TIMEOUT, "a barrier of the small rebuild waited too long");
     if (out->status == GS_REFUSED) return nullptr;
     const int64_t nc = out->nc, m = out->m;
-    DevBuf<int64_t> rowptr(ctx, nc + 1);
-    DevBuf<int32_t> tail(ctx, m), ref(ctx, g->ref ? nc : 0), pos(ctx, g->ref ? nc : 0);
-    DevBuf<double> w(ctx, m);
+    DevBuf<int64_t> rowptr;
+    DevBuf<int32_t> tail, ref, pos;
+    DevBuf<double> w;
+    const size_t maps = g->ref ? nc : 0;
+    if (!rowptr.try_alloc(ctx, nc + 1) || !tail.try_alloc(ctx, m) || !w.try_alloc(ctx, m) ||
+        !ref.try_alloc(ctx, maps) || !pos.try_alloc(ctx, maps))
+        return nullptr; // the general path holds less at a time
     {
         LaunchTimer lt(ctx);
         if (m >= LANES32_ROW * nc)

@@ -245,13 +245,11 @@ int64_t vg_color_internal(vg_ctx *ctx, vg_graph *g, int64_t nHash, int32_t targe
     VG_CHECK_LAUNCH();
     DevBuf<unsigned long long> cnt(ctx, 1);
     unsigned long long *h = (unsigned long long *)vg_pinned(ctx, sizeof(unsigned long long));
-    // Up to eight hashes are kept per vertex, where the context's budget has room for them;
-    // below COLOR_HASH_NE entries their launch costs more than it saves (a coloring of some
-    // 3,000 vertices 205 -> 219 us).
+    // Up to eight hashes are kept per vertex, where there is room for them; below COLOR_HASH_NE
+    // entries their launch costs more than it saves (a coloring of some 3,000 vertices
+    // 205 -> 219 us).
     DevBuf<uint32_t> hash;
-    const size_t words = (size_t)nv * (nHash <= 4 ? 4 : 8);
-    if (nHash <= 8 && g->ne >= COLOR_HASH_NE && vg_has_room(ctx, sizeof(uint32_t) * words))
-        hash.alloc(ctx, words);
+    if (nHash <= 8 && g->ne >= COLOR_HASH_NE) hash.try_alloc(ctx, (size_t)nv * (nHash <= 4 ? 4 : 8));
     uint32_t seed = 1012; // coloring.cpp:60
     int64_t nextColor = 0, lastCount = 0, currentCount = 0;
     const int64_t targetCount = (nv * target_percent) / 100;

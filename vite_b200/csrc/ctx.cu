@@ -22,18 +22,32 @@ int vg_grid(vg_ctx *ctx, int64_t work, int block, int per_sm) {
     return (int)g;
 }
 
+// *p and cudaSuccess, or why not; the budget's room is the callers' to look at
+static cudaError_t pool_alloc(vg_ctx *ctx, size_t bytes, void **p) {
+    const cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
+    if (e == cudaSuccess) ctx->in_use += bytes;
+    else cudaGetLastError();
+    return e;
+}
+
 void *vg_alloc(vg_ctx *ctx, size_t bytes) {
     if (bytes == 0) return nullptr;
-    if (ctx->budget && ctx->in_use + bytes > ctx->budget)
+    if (!vg_has_room(ctx, bytes))
         vg_throw(VG_ERR_OOM, "device memory budget exceeded: %zu in use + %zu requested > %zu",
                  ctx->in_use, bytes, ctx->budget);
     void *p = nullptr;
-    cudaError_t e = cudaMallocAsync(&p, bytes, ctx->stream);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
+    const cudaError_t e = pool_alloc(ctx, bytes, &p);
+    if (e != cudaSuccess)
         vg_throw(VG_ERR_OOM, "cudaMallocAsync(%zu bytes): %s", bytes, cudaGetErrorString(e));
-    }
-    ctx->in_use += bytes;
+    return p;
+}
+
+void *vg_try_alloc(vg_ctx *ctx, size_t bytes) {
+    if (bytes == 0 || !vg_has_room(ctx, bytes)) return nullptr;
+    void *p = nullptr;
+    const cudaError_t e = pool_alloc(ctx, bytes, &p);
+    if (e == cudaErrorMemoryAllocation) return nullptr;
+    VG_CUDA(e);
     return p;
 }
 

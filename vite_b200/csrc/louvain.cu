@@ -2326,9 +2326,9 @@ static bool run_phase_small(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, 
     const size_t doubles = 3 * n + 3 * units + (et ? n : 0) + (et24 ? 2 * n : 0);
     const size_t bytes = sizeof(CommInfo) * n + sizeof(double) * doubles +
                          sizeof(int32_t) * (5 * n + ctl_words + 1) + (et ? n : 0);
-    if (!vg_has_room(ctx, bytes + sizeof(int32_t) * n)) return false;
-    DevBuf<unsigned char> scratch(ctx, bytes);
-    DevBuf<int32_t> comm(ctx, nv);
+    DevBuf<unsigned char> scratch;
+    DevBuf<int32_t> comm;
+    if (!comm.try_alloc(ctx, n) || !scratch.try_alloc(ctx, bytes)) return false;
     unsigned char *at = scratch.p;
     auto take = [&](size_t b) {
         unsigned char *q = at;
@@ -2596,10 +2596,8 @@ static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double
     }
 
     DevBuf<uint8_t> touched; // communities the current color's sweep moves vertices in or out of
-    if (ordering == 1 && nv && vg_has_room(ctx, nv + 16)) {
-        touched.alloc(ctx, (nv + 15) / 16 * 16);
+    if (ordering == 1 && nv && touched.try_alloc(ctx, (nv + 15) / 16 * 16))
         VG_CUDA(cudaMemsetAsync(touched.p, 0, touched.n, ctx->stream));
-    }
     int32_t *past = A.p, *curr = B.p, *target = C.p;
     double *pcurr = pA.p, *pprev = pB.p;
     double prevMod = p->lower, currMod = -1.0;

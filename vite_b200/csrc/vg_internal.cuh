@@ -84,8 +84,10 @@ void vg_side_join(vg_ctx *ctx, int n);
 
 // stream-ordered device allocation accounted against the context budget
 void *vg_alloc(vg_ctx *ctx, size_t bytes);
-// whether the context's budget has room for `bytes` more (a path that trades memory for time
-// asks, and takes the leaner one otherwise)
+// the same for a path that trades memory for time: null when the budget or the device has no
+// room, and the leaner path is taken
+void *vg_try_alloc(vg_ctx *ctx, size_t bytes);
+// whether the context's budget has room for `bytes` more
 inline bool vg_has_room(const vg_ctx *ctx, size_t bytes) {
     return !ctx->budget || ctx->in_use + bytes <= ctx->budget;
 }
@@ -102,6 +104,13 @@ template <class T> struct DevBuf {
         ctx = c;
         n = count;
         p = count ? (T *)vg_alloc(c, count * sizeof(T)) : nullptr;
+    }
+    bool try_alloc(vg_ctx *c, size_t count) { // false: no room (vg_try_alloc), and empty
+        release();
+        ctx = c;
+        p = count ? (T *)vg_try_alloc(c, count * sizeof(T)) : nullptr;
+        n = p ? count : 0;
+        return p || count == 0;
     }
     void release() {
         if (p) vg_free(ctx, p, n * sizeof(T));
