@@ -28,7 +28,8 @@ typedef enum vg_status {
     VG_ERR_ARG = 1,      /* invalid argument (the reference asserts or MPI_Aborts, main.cpp:714-768) */
     VG_ERR_OOM = 2,      /* device memory or the context's memory budget is exhausted */
     VG_ERR_CUDA = 3,     /* a CUDA runtime call failed */
-    VG_ERR_TIMEOUT = 4,  /* a bounded device-side wait ran out */
+    VG_ERR_TIMEOUT = 4,  /* a bounded device-side wait ran out and nothing took over (no call
+                            returns it at present: see vg_ctx_set_barrier_polls) */
     VG_ERR_STATE = 5     /* call made in the wrong state (e.g. rebuild before any phase) */
 } vg_status;
 
@@ -105,6 +106,11 @@ vg_status vg_ctx_profile(vg_ctx *ctx, int32_t enable, double *kernel_ms_out,
  * up to this working set allocate without mapping new memory mid-run. Counted
  * against the budget only while held (it is released back to the pool at once). */
 vg_status vg_ctx_reserve(vg_ctx *ctx, size_t bytes);
+/* Phases and rebuilds of small graphs run as one cooperative launch whose blocks wait for
+ * one another (no reference counterpart). A wait that has read its counter `polls` times
+ * (default 2^23, some seconds) gives up; the launch then ends without a result and the step is
+ * done again by a launch per step. At least 1, else VG_ERR_ARG. */
+vg_status vg_ctx_set_barrier_polls(vg_ctx *ctx, int32_t polls);
 /* The CUDA stream (cudaStream_t) all of the context's work runs on, so callers
  * can time it with events or order their own work after it. */
 vg_status vg_ctx_stream(vg_ctx *ctx, void **stream_out);

@@ -1239,12 +1239,11 @@ vg_graph *vg_rebuild_small(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) 
     SmallRebuildOut *out = (SmallRebuildOut *)vg_pinned(ctx, sizeof(SmallRebuildOut));
     out->status = GS_DONE;
     p.out = out;
+    p.polls = ctx->barrier_polls;
     vg_grid_launch(ctx, grid ? k_rebuild_small<true> : k_rebuild_small<false>, p, grid, blocks,
                    RS_SMEM_BYTES, p.arrived);
     vg_sync(ctx);
-    if (out->status == GS_TIMEOUT)
-        vg_throw(VG_ERR_TIMEOUT, "a barrier of the small rebuild waited too long");
-    if (out->status == GS_REFUSED) return nullptr;
+    if (out->status != GS_DONE) return nullptr;
     const int64_t nc = out->nc, m = out->m;
     DevBuf<int64_t> rowptr;
     DevBuf<int32_t> tail, ref, pos;

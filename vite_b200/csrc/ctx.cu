@@ -187,6 +187,14 @@ extern "C" vg_status vg_ctx_reserve(vg_ctx *ctx, size_t bytes) {
     });
 }
 
+extern "C" vg_status vg_ctx_set_barrier_polls(vg_ctx *ctx, int32_t polls) {
+    if (!ctx) return VG_ERR_ARG;
+    return vg_guard(ctx, [&] {
+        VG_REQUIRE(polls >= 1, "a wait needs at least one poll (got %d)", polls);
+        ctx->barrier_polls = polls;
+    });
+}
+
 extern "C" vg_status vg_ctx_stream(vg_ctx *ctx, void **stream_out) {
     if (!ctx || !stream_out) return VG_ERR_ARG;
     *stream_out = (void *)ctx->stream;

@@ -11,17 +11,19 @@ constexpr int GS_MAX_CLUSTER = 16;
 // what such a kernel leaves in pinned memory (set to GS_DONE before the launch)
 enum : int32_t {
     GS_DONE = 0,
-    GS_REFUSED = 1, // not a graph the kernel takes; nothing has changed
+    GS_REFUSED = 1, // not a graph the kernel takes
     GS_TIMEOUT = 2  // a barrier's bounded wait ran out
 };
+// GS_REFUSED and GS_TIMEOUT leave the graph as it was, and the general path takes it.
 
 // All blocks of the launch reach the barrier, and what they wrote before it is visible
 // after it. GRID: a counter in global memory that starts at 0 (the launch is cooperative,
-// so every block is resident); a wait of GS_SPINS polls (seconds) gives up and returns
-// false in every thread of the block. Else the grid is one cluster: its hardware barrier.
-constexpr int GS_SPINS = 1 << 23;
+// so every block is resident); a wait of `polls` reads (vg_ctx_set_barrier_polls) gives up and
+// returns false in every thread of the block. A block that gave up arrives at no later barrier, so
+// every other one passes the barriers it had reached, gives up at its next one and returns too.
+// Else the grid is one cluster: its hardware barrier.
 template <bool GRID>
-__device__ __forceinline__ bool all_blocks(unsigned *arrived, unsigned &round, int &s_dead) {
+__device__ __forceinline__ bool all_blocks(unsigned *arrived, unsigned &round, int &s_dead, int polls) {
     if constexpr (GRID) {
         round++;
         __syncthreads();
@@ -29,14 +31,14 @@ __device__ __forceinline__ bool all_blocks(unsigned *arrived, unsigned &round, i
             __threadfence();
             atomicAdd(arrived, 1u);
             const unsigned want = round * gridDim.x;
-            int spins = 0;
+            int read = 0;
             unsigned seen;
             do {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n"
                              : "=r"(seen)
                              : "l"(arrived)
                              : "memory");
-            } while (seen < want && ++spins < GS_SPINS);
+            } while (seen < want && ++read < polls);
             if (seen < want) s_dead = 1;
             __threadfence();
         }

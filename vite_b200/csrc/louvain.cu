@@ -2370,12 +2370,11 @@ static bool run_phase_small(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, 
     SmallOut *out = (SmallOut *)vg_pinned(ctx, sizeof(SmallOut));
     out->status = GS_DONE;
     sp.out = out;
+    sp.polls = ctx->barrier_polls;
     vg_grid_launch(ctx, grid ? k_phase_small<true> : k_phase_small<false>, sp, grid, blocks,
                    SP_WORK_BYTES, sp.arrived);
     vg_sync(ctx);
-    if (out->status == GS_TIMEOUT)
-        vg_throw(VG_ERR_TIMEOUT, "a barrier of the small phase waited too long");
-    if (out->status == GS_REFUSED) return false;
+    if (out->status != GS_DONE) return false;
     if (sweep_ms) *sweep_ms = out->sweep_ns * 1e-6;
     *mod_out = out->mod;
     *iters_out = out->iters;

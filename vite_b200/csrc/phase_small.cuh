@@ -86,6 +86,7 @@ struct SmallPhase {
                            // update per color (louvain.cpp:724-735)
     int32_t ncolors;       // uncolored (-1) vertices go with the last one
     unsigned *arrived; // (GRID) blocks that reached the grid's barriers so far (starts at 0)
+    int32_t polls;     // of one wait there
     SmallOut *out;
 };
 
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
     const int rank = blockIdx.x, blocks = gridDim.x; // without GRID the grid is one cluster
     unsigned round = 0;
     auto barrier = [&]() -> bool {
-        const bool ok = all_blocks<GRID>(p.arrived, round, s_dead);
+        const bool ok = all_blocks<GRID>(p.arrived, round, s_dead, p.polls);
         if (!ok && tid == 0) p.out->status = GS_TIMEOUT;
         return ok;
     };

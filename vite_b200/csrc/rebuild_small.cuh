@@ -70,7 +70,8 @@ struct SmallRebuild {
     int64_t *part;     // 3 per block
     int32_t *gk, *uk;
     double *gw, *uw;
-    unsigned *arrived;
+    unsigned *arrived; // as in SmallPhase
+    int32_t polls;
     SmallRebuildOut *out;
 };
 enum { RS_BIG_ROWS, RS_LONG_SEGS, RS_REFUSED, RS_CTL };
@@ -95,7 +96,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_rebuild_small(SmallRebuild p)
     const int64_t gthreads = (int64_t)blocks * GS_THREADS;
     unsigned round = 0;
     auto barrier = [&]() -> bool {
-        const bool ok = all_blocks<GRID>(p.arrived, round, s_dead);
+        const bool ok = all_blocks<GRID>(p.arrived, round, s_dead, p.polls);
         if (!ok && tid == 0) p.out->status = GS_TIMEOUT;
         return ok;
     };

@@ -71,8 +71,10 @@ struct vg_ctx {
     // (vg_side_fork), with the events that fork them from and join them to the main stream
     cudaStream_t side[VG_SIDE] = {};
     cudaEvent_t fork = nullptr, join[VG_SIDE] = {};
-    // blocks the one-launch kernels of small graphs may use on the device
+    // blocks the one-launch kernels of small graphs may use on the device, and the reads after
+    // which a wait at their barriers gives up (vg_ctx_set_barrier_polls)
     GridLimits phase_limits, rebuild_limits;
+    int32_t barrier_polls = 1 << 23;
 };
 
 // the context's side streams: work enqueued on the first n of them between vg_side_fork and
