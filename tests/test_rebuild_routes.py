@@ -1,0 +1,38 @@
+"""Which rebuilds of small graphs run in one launch (GPU): those whose longest segment one block
+reads in little time. The numbers of launches, on both sides of the lines, and the oracle's bits."""
+import numpy as np
+import pytest
+
+from oracle import vite_oracle as vo
+from test_general_path import launches_of
+from test_gpu_parity import assert_graph_equal
+from test_small_phase import multigraph
+
+pytestmark = pytest.mark.gpu
+
+
+def one_long(n, members, others):
+    """One community of `members` vertices and `others` (or single) ones, at random places."""
+    rng = np.random.default_rng([n, members, others])
+    cv = 1 + (np.arange(n) % others)
+    cv[:members] = 0
+    return rng.permutation(n)[cv][rng.permutation(n)]
+
+
+# (vertices, pairs, members, others, real, one launch): entries of the long segment about
+# 2 * pairs * members / vertices, its reads one up to 4,096 communities
+@pytest.mark.parametrize("n,m,members,others,real,one", [
+    (10000, 60000, 2500, 1000, True, True), (10000, 60000, 3000, 1000, True, False),
+    (10000, 60000, 8000, 1000, True, False), (6000, 250000, 4800, 50, True, False),
+    (10000, 200000, 3000, 1000, False, True), (10000, 200000, 3500, 1000, False, False),
+    (12000, 48000, 1950, 9000, False, True), (12000, 48000, 2200, 9000, False, False),
+    (20000, 60000, 4000, 15000, True, False)])
+def test_long_segments(ctx, n, m, members, others, real, one):
+    g = multigraph(n, m, 23, real)
+    cv = one_long(n, members, others)
+    dev = ctx.upload(g.rowptr, g.tail, g.weight)
+    if not real:
+        ctx.vertex_degree(dev)  # the weights are known to be integral from here on
+    _, launches = launches_of(ctx, lambda: ctx.rebuild(dev, cv))
+    assert (launches <= 10) == one
+    assert_graph_equal(dev.download(), vo.rebuild(g, cv))

@@ -33,11 +33,16 @@ constexpr int64_t RS_MAX_NV = VG_RS_MAX_NV;
 constexpr int64_t RS_MAX_NE = VG_RS_MAX_NE;
 static_assert(RS_MAX_NV <= NARROW_KEYS, "warp_segment is told so");
 constexpr int RS_BIG_L = 1024; // segments longer than this go to a whole block
-// A block reads a segment of many keys once per 4,096 key values; a graph with a segment that
-// might be read for more entries than this is left to the general path before any is read
-// (a rebuild of 104,000 vertices with a 60,000-entry segment and 13 reads took 2.75 ms
-// here, 1.1 there; 9,700 vertices, three reads, 0.34 here, 0.97 there).
-constexpr int64_t RS_MAX_READS = 262144;
+// One block reads a long segment while the others wait at the barrier, and one of many keys
+// once per 4,096 key values. A graph with a segment that might be read for more entries than this
+// is left to the general path before any is read. Whole rebuilds here and by launches: integral
+// weights and one read, where the warps share every key, 180,000 entries 0.82 and 0.73 ms, 400,000
+// 1.08 and 0.96; several reads, 49,000 entries in all 0.50 and 0.53, 71,000 0.56 and 0.50, 124,000
+// 0.70 and 0.47; real weights and one read, where a key's entries are one warp's chain, 24,000
+// entries 0.36 and 0.54, 48,000 0.65 and 0.61, 96,000 1.8 and 1.1, 800,000 14.3 and 3.1.
+__device__ __forceinline__ int64_t rs_max_reads(bool integral, int64_t reads) {
+    return reads > 1 ? 49152 : integral ? 131072 : 32768;
+}
 
 using SmallWarpTable = HashWarpSmem<H_CAP, H_MAXU>;
 using SmallBlockTable = BlockTableLarge;
@@ -206,9 +211,10 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_rebuild_small(SmallRebuild p)
                 p.mbase[r] = ma + mp;
                 p.rstart[r] = ea + ep;
                 if (m > 32) p.biglist[atomicAdd(p.ctl + RS_BIG_ROWS, 1)] = (int32_t)r;
-                const int64_t reads = (nc + SmallBlockTable::MAXU - 1) / SmallBlockTable::MAXU;
-                if (reads > 1 && e > SmallBlockTable::MAXU && e * reads > RS_MAX_READS)
-                    p.ctl[RS_REFUSED] = 1;
+                const int64_t reads = e > SmallBlockTable::MAXU
+                                          ? (nc + SmallBlockTable::MAXU - 1) / SmallBlockTable::MAXU
+                                          : 1;
+                if (e * reads > rs_max_reads(p.integral, reads)) p.ctl[RS_REFUSED] = 1;
                 if (e > RS_BIG_L) p.longlist[atomicAdd(p.ctl + RS_LONG_SEGS, 1)] = (int32_t)r;
             }
             ma += mt;
