@@ -36,3 +36,20 @@ def test_long_segments(ctx, n, m, members, others, real, one):
     _, launches = launches_of(ctx, lambda: ctx.rebuild(dev, cv))
     assert (launches <= 10) == one
     assert_graph_equal(dev.download(), vo.rebuild(g, cv))
+
+
+@pytest.mark.parametrize("members,sorted_path", [(7000, False), (15000, True)])
+def test_long_segment_of_real_weights_is_sorted(ctx, members, sorted_path):
+    """Above the one-launch size: 28,000 and 60,000 entries, integral ones in a block's table."""
+    n = 140000
+    cv = one_long(n, members, 2000)
+    count = {}
+    for real in (False, True):
+        g = multigraph(n, 280000, 29, real)
+        dev = ctx.upload(g.rowptr, g.tail, g.weight)
+        if not real:
+            ctx.vertex_degree(dev)
+        _, count[real] = launches_of(ctx, lambda: ctx.rebuild(dev, cv))
+        assert_graph_equal(dev.download(), vo.rebuild(g, cv))
+        dev.free()
+    assert (count[True] > count[False] + 10) == sorted_path

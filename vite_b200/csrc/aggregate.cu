@@ -10,7 +10,7 @@
 //      entries into a shared-memory hash table in order and sorts the distinct
 //      keys; segments with more than 256 distinct keys, or of more entries than a warp
 //      should take, get a block each; those past the blocks' tables (4,096 keys,
-//      131,072 entries) go through one stable radix sort of all their entries by
+//      131,072 entries, real weights 32,768) go through one stable radix sort of all their entries by
 //      (segment, c2) and each run is folded in order;
 //   3. the unique entries are compacted into the next CSR.
 #include "grid_sync.cuh"
@@ -414,9 +414,15 @@ __device__ __forceinline__ int warp_segment(HashWarpSmem<CAP, MAXU> &S, int64_t 
 
 // where a tier sends the segments it cannot hold, or that are too long for a warp (a warp
 // takes some 200 cycles per 32 entries): lists by length for the two block tables, a flag
-// (the next tier, or the sorted path) for the others and without lists
-constexpr int64_t BLOCK_SMALL_L = 8192, BLOCK_LARGE_L = 131072;
+// (the next tier, or the sorted path) for the others and without lists. The large
+// table takes integral segments of up to 131,072 entries. Real weights: 32,768, because one
+// key's entries are one warp's chain: rebuilds with one long segment by its block and by the
+// sorted path, 48,000 entries 0.82 and 0.55 ms, 96,000 1.95 and 0.8. A run on 2,266,207 vertices
+// with U(0,1) weights takes 28.2 ms with either line, and 28.7 with 8,192.
+constexpr int64_t BLOCK_SMALL_L = 8192;
+constexpr int64_t block_large_l(bool integral) { return integral ? 131072 : 32768; }
 struct BlockRows {
+    int64_t large_l = 0; // entries up to which the large table takes a segment
     int32_t *rows[2] = {nullptr, nullptr};
     int32_t *count = nullptr; // 2, then the rows of each list taken so far
 };
@@ -441,7 +447,7 @@ __global__ void __launch_bounds__(H_WARPS * 32) k_rows_hash(
         const int U = L > BLOCK_SMALL_L ? -1 : warp_segment<false>(S, b, L, gk, gw, uk, uw, narrow);
         if (lane == 0) {
             if (U >= 0) ucount[row] = U;
-            const int to = U >= 0 || !next.rows[0] ? -1 : L <= BLOCK_SMALL_L ? 0 : L <= BLOCK_LARGE_L ? 1 : -1;
+            const int to = U >= 0 || !next.rows[0] ? -1 : L <= BLOCK_SMALL_L ? 0 : L <= next.large_l ? 1 : -1;
             if (to >= 0) next.rows[to][atomicAdd(next.count + to, 1)] = (int32_t)row;
             flag[row] = U < 0 && to < 0;
         }
@@ -1046,6 +1052,7 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
             DevBuf<int64_t> fpos(ctx, nc), fcount(ctx, 1);
             DevBuf<int32_t> frows(ctx, nc), brows(ctx, 2 * nc + 4);
             BlockRows next;
+            next.large_l = block_large_l(integral);
             next.rows[0] = brows.p;
             next.rows[1] = brows.p + nc;
             next.count = brows.p + 2 * nc;

@@ -39,7 +39,7 @@ constexpr int RS_BIG_L = 1024; // segments longer than this go to a whole block
 // weights and one read, where the warps share every key, 180,000 entries 0.82 and 0.73 ms, 400,000
 // 1.08 and 0.96; several reads, 49,000 entries in all 0.50 and 0.53, 71,000 0.56 and 0.50, 124,000
 // 0.70 and 0.47; real weights and one read, where a key's entries are one warp's chain, 24,000
-// entries 0.36 and 0.54, 48,000 0.65 and 0.61, 96,000 1.8 and 1.1, 800,000 14.3 and 3.1.
+// entries 0.36 and 0.54, 48,000 0.65 and 0.55, 96,000 1.8 and 0.8, 800,000 14.3 and 3.1.
 __device__ __forceinline__ int64_t rs_max_reads(bool integral, int64_t reads) {
     return reads > 1 ? 49152 : integral ? 131072 : 32768;
 }
