@@ -30,6 +30,11 @@ constexpr int SP_THREADS = GS_THREADS;
 constexpr int SP_WARPS = GS_WARPS;
 constexpr int SP_T = 32;       // rows up to here: one thread each
 constexpr int SP_CAP = 16384;  // slots of a block's table: rows of up to half as many communities
+// entries of a row (of a multigraph: the others' rows have no more than their communities) up to
+// which its one block is not waited for longer than launches would take: phases with one such
+// row by launches and here, 20,000 entries 0.51 and 0.29 ms, 50,000 0.48 and 0.43, 80,000 0.53 and
+// 0.69, 800,000 0.50 and 5.1
+constexpr int64_t SP_MAX_ROW = 49152;
 constexpr int SP_UNITS = SEG_CHUNK == 2048 && SEG_THREADS == 256 ? 8 : -1; // warps per chunk
 #ifndef VG_SP_MAX_NV
 #define VG_SP_MAX_NV 524288
@@ -64,8 +69,8 @@ struct SmallOut {
     double mod;      // prevMod at the break
     double sweep_ns; // time between the barriers around the sweeps
     int32_t iters;
-    int32_t status;  // GS_DONE; GS_REFUSED when a row may hold more communities
-                     // than a block's table
+    int32_t status;  // GS_DONE; GS_REFUSED when a row may hold more communities than a block's
+                     // table, or has more than SP_MAX_ROW entries
 };
 
 struct SmallPhase {
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
             const int64_t e0 = a.rowptr[v], e1 = a.rowptr[v + 1];
             const int64_t d = e1 - e0;
             if (d <= SP_T) p.vdeg[v] = row_fold(a.weight, e0, e1);
-            if (min(d, nv) > SP_CAP / 2) p.ctl[CTL_REFUSED] = 1;
+            if (d > SP_MAX_ROW || min(d, nv) > SP_CAP / 2) p.ctl[CTL_REFUSED] = 1;
             bucket = bucket_of(v, d);
         }
         const unsigned peers = __match_any_sync(0xffffffffu, bucket);
