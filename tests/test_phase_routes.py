@@ -30,3 +30,25 @@ def test_longest_row(ctx, n, pairs, entries, one):
     assert (launches <= 10) == one
     np.testing.assert_array_equal(cv, ref[0])
     assert (it, float(mod).hex()) == (ref[2], float(ref[1]).hex())
+
+
+@pytest.mark.parametrize("n", [20000, 140000])
+@pytest.mark.parametrize("rebuilt", [False, True])
+def test_known_row_is_not_launched_for(n, rebuilt):
+    """A row of 8,193 communities, known from the upload or from the rebuild (in one launch or by
+    several), costs one launch less than one of 8,192 whose launch gives up at its barriers."""
+    import vite_b200
+
+    count, iters = {}, {}
+    with vite_b200.Context(0) as c:
+        for entries in (8192, 8193):
+            g = hub_graph(n, n // 2, entries)
+            dev = c.upload(g.rowptr, g.tail, g.weight)
+            if rebuilt:  # every vertex alone: equal pairs become one
+                c.rebuild(dev, np.arange(n))
+            c.set_barrier_polls(1 if entries == 8192 else 1 << 23)
+            (_, _, iters[entries]), count[entries] = launches_of(
+                c, lambda: c.louvain_phase(dev, threshold=10.0))
+            dev.free()
+    assert iters[8192] == iters[8193] == 1  # no gain is enough to go on
+    assert count[8193] == count[8192] - 1 and count[8193] > 10

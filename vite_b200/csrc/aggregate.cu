@@ -944,6 +944,15 @@ void long_rows(vg_ctx *ctx, const int64_t *offs, int64_t n, int64_t total, LongR
     L.grid = (int)std::min<int64_t>(total / COPY_CHUNK + cap, 16LL * ctx->sm_count);
 }
 
+// raises *longest to the largest of count[0..n)
+__global__ void k_longest(int64_t n, const int64_t *__restrict__ count, int32_t *__restrict__ longest) {
+    int32_t most = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x)
+        most = max(most, (int32_t)min(count[i], (int64_t)INT_MAX));
+    vg_raise(longest, most);
+}
+
 #include "rebuild_small.cuh"
 
 } // namespace
@@ -1169,8 +1178,23 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
     }
     gk.release();
     gw.release();
-    // 5-6. next CSR
+    // 5-6. next CSR, and its longest row where a phase may want to know it; that lands past
+    // the word the scan's total is read back through
+    DevBuf<int32_t> longest;
+    int32_t *hl = (int32_t *)vg_pinned(ctx, 64 + sizeof(int32_t)) + 16;
+    *hl = -1;
+    if (nc && nc <= VG_ONE_LAUNCH_NV) {
+        longest.alloc(ctx, 1);
+        VG_CUDA(cudaMemsetAsync(longest.p, 0, sizeof(int32_t), ctx->stream));
+        {
+            LaunchTimer lt(ctx);
+            k_longest<<<vg_grid(ctx, nc, 256), 256, 0, ctx->stream>>>(nc, ucount.p, longest.p);
+        }
+        VG_CHECK_LAUNCH();
+        VG_CUDA(cudaMemcpyAsync(hl, longest.p, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    }
     const int64_t m = vg_exclusive_scan_i64(ctx, ucount.p, nc + 1);
+    const int32_t most = *hl;
     DevBuf<int32_t> tail(ctx, m);
     DevBuf<double> w(ctx, m);
     if (nc) {
@@ -1194,7 +1218,9 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
         }
         VG_CHECK_LAUNCH();
     }
-    return vg_graph_wrap(ctx, nc, m, ucount.detach(), tail.detach(), w.detach());
+    vg_graph *h = vg_graph_wrap(ctx, nc, m, ucount.detach(), tail.detach(), w.detach());
+    h->longest = most;
+    return h;
 }
 
 // vg_rebuild_new of a small graph by k_rebuild_small; null when the graph is not one it
@@ -1202,6 +1228,8 @@ vg_graph *vg_aggregate_rows(vg_ctx *ctx, const vg_graph *g, const int32_t *pos,
 vg_graph *vg_rebuild_small(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) {
     const int64_t nv = g->nv, ne = g->ne;
     if (nv == 0 || nv > RS_MAX_NV || ne > RS_MAX_NE) return nullptr;
+    // a segment at least as long as a row that one block may read would be refused
+    if (g->longest > rs_max_reads(g->integral == 1, 1)) return nullptr;
     vg_grid_limits(ctx, k_rebuild_small<false>, k_rebuild_small<true>, RS_SMEM_BYTES,
                    ctx->rebuild_limits);
     const bool grid = ne > VG_RS_CLUSTER_NE;
@@ -1252,6 +1280,7 @@ vg_graph *vg_rebuild_small(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) 
     vg_sync(ctx);
     if (out->status != GS_DONE) return nullptr;
     const int64_t nc = out->nc, m = out->m;
+    const int32_t longest = out->longest;
     DevBuf<int64_t> rowptr;
     DevBuf<int32_t> tail, ref, pos;
     DevBuf<double> w;
@@ -1272,5 +1301,6 @@ vg_graph *vg_rebuild_small(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) 
     vg_graph *h = vg_graph_wrap(ctx, nc, m, rowptr.detach(), tail.detach(), w.detach());
     h->ref = ref.detach();
     h->pos = pos.detach();
+    h->longest = longest;
     return h;
 }

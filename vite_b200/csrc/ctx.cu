@@ -227,7 +227,16 @@ extern "C" vg_status vg_ctx_profile(vg_ctx *ctx, int32_t enable, double *kernel_
 // graphs
 
 namespace {
-__global__ void k_integral(const double *__restrict__ w, int64_t ne, int *__restrict__ bad) {
+// rowptr: null, or raise *longest to the longest of nv rows
+__global__ void k_integral(const double *__restrict__ w, int64_t ne, int *__restrict__ bad,
+                           const int64_t *__restrict__ rowptr, int64_t nv, int32_t *__restrict__ longest) {
+    if (rowptr) {
+        int32_t most = 0;
+        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nv;
+             i += (int64_t)gridDim.x * blockDim.x)
+            most = max(most, (int32_t)(rowptr[i + 1] - rowptr[i]));
+        vg_raise(longest, most);
+    }
     int mine = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ne;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -244,17 +253,20 @@ bool vg_weights_integral(vg_ctx *ctx, vg_graph *g) {
     if (g->ne >= ((int64_t)1 << 31)) {
         r = 0;
     } else if (g->ne > 0) {
-        DevBuf<int> bad(ctx, 1);
-        VG_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), ctx->stream));
+        const bool rows = g->longest < 0 && g->nv <= VG_ONE_LAUNCH_NV;
+        DevBuf<int> bad(ctx, 2); // and the longest row
+        VG_CUDA(cudaMemsetAsync(bad.p, 0, 2 * sizeof(int), ctx->stream));
         {
             LaunchTimer lt(ctx);
-            k_integral<<<vg_grid(ctx, g->ne, 256), 256, 0, ctx->stream>>>(g->weight, g->ne, bad.p);
+            k_integral<<<vg_grid(ctx, g->ne, 256), 256, 0, ctx->stream>>>(
+                g->weight, g->ne, bad.p, rows ? g->rowptr : nullptr, g->nv, bad.p + 1);
         }
         VG_CHECK_LAUNCH();
-        int *h = (int *)vg_pinned(ctx, sizeof(int));
-        VG_CUDA(cudaMemcpyAsync(h, bad.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        int *h = (int *)vg_pinned(ctx, 2 * sizeof(int));
+        VG_CUDA(cudaMemcpyAsync(h, bad.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         vg_sync(ctx);
         r = *h ? 0 : 1;
+        if (rows) g->longest = h[1];
     }
     g->integral = (int8_t)r;
     return r == 1;
@@ -292,26 +304,30 @@ void vg_graph_release(vg_ctx *ctx, vg_graph *g) {
 
 namespace {
 // flags row offsets (n1 of them, the first taken as base) that decrease, hold a row of
-// more than INT32_MAX entries (degrees are 32-bit in the sweep), or do not end at base + ne
+// more than INT32_MAX entries (degrees are 32-bit in the sweep), or do not end at base + ne;
+// raises *longest to the longest row
 __global__ void k_check_rowptr(const int64_t *__restrict__ rp, int64_t n1, int64_t base,
-                               int64_t ne, int *__restrict__ bad) {
+                               int64_t ne, int *__restrict__ bad, int32_t *__restrict__ longest) {
+    int32_t most = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n1;
          i += (int64_t)gridDim.x * blockDim.x) {
         if (i + 1 < n1) {
             const int64_t len = rp[i + 1] - rp[i];
             if (len < 0 || len > (int64_t)INT32_MAX) *bad = 1;
+            else most = max(most, (int32_t)len);
         }
         if (i == n1 - 1 && rp[i] - base != ne) *bad = 1;
     }
+    vg_raise(longest, most);
 }
 } // namespace
 
 void vg_check_rowptr_async(vg_ctx *ctx, const int64_t *rp, int64_t n1, int64_t base, int64_t ne,
-                           int *bad) {
+                           int *bad, int32_t *longest) {
     if (n1 <= 0) return;
     {
         LaunchTimer lt(ctx);
-        k_check_rowptr<<<vg_grid(ctx, n1, 256), 256, 0, ctx->stream>>>(rp, n1, base, ne, bad);
+        k_check_rowptr<<<vg_grid(ctx, n1, 256), 256, 0, ctx->stream>>>(rp, n1, base, ne, bad, longest);
     }
     VG_CHECK_LAUNCH();
 }
@@ -357,10 +373,10 @@ extern "C" vg_status vg_graph_upload(vg_ctx *ctx, int64_t nv, int64_t ne, const 
         DevBuf<double> w(ctx, ne);
         VG_CUDA(cudaMemcpyAsync(rp.p, rowptr, sizeof(int64_t) * (nv + 1), cudaMemcpyHostToDevice,
                                 ctx->stream));
-        // bad[0]: row offsets, bad[1]: tails; read back together
-        DevBuf<int> bad(ctx, 2);
-        VG_CUDA(cudaMemsetAsync(bad.p, 0, 2 * sizeof(int), ctx->stream));
-        vg_check_rowptr_async(ctx, rp.p, nv + 1, 0, ne, bad.p);
+        // bad[0]: row offsets, bad[1]: tails, and the longest row; read back together
+        DevBuf<int> bad(ctx, 3);
+        VG_CUDA(cudaMemsetAsync(bad.p, 0, 3 * sizeof(int), ctx->stream));
+        vg_check_rowptr_async(ctx, rp.p, nv + 1, 0, ne, bad.p, bad.p + 2);
         if (ne) {
             // stage the 16-byte records through two bounded device buffers in chunks:
             // the copies run back to back on the context's stream while the side
@@ -411,13 +427,15 @@ extern "C" vg_status vg_graph_upload(vg_ctx *ctx, int64_t nv, int64_t ne, const 
             }
             destroy();
         }
-        int *hb = (int *)vg_pinned(ctx, 2 * sizeof(int));
-        VG_CUDA(cudaMemcpyAsync(hb, bad.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        int *hb = (int *)vg_pinned(ctx, 3 * sizeof(int));
+        VG_CUDA(cudaMemcpyAsync(hb, bad.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         vg_sync(ctx);
         VG_REQUIRE(hb[0] == 0, "rowptr must not decrease, and no row may hold more than 2^31 - 1 "
                                "entries");
         VG_REQUIRE(hb[1] == 0, "edge tail out of range [0, nv)");
+        const int32_t longest = hb[2];
         *out = vg_graph_wrap(ctx, nv, ne, rp.detach(), tail.detach(), w.detach());
+        (*out)->longest = longest;
     });
 }
 

@@ -107,8 +107,8 @@ extern "C" vg_status vg_graph_read_vite(vg_ctx *ctx, const char *path, vg_graph 
         DevBuf<int64_t> rp(ctx, nv + 1);
         DevBuf<int32_t> tail(ctx, ne);
         DevBuf<double> w(ctx, ne);
-        DevBuf<int> bad(ctx, 2);
-        VG_CUDA(cudaMemsetAsync(bad.p, 0, 2 * sizeof(int), ctx->stream));
+        DevBuf<int> bad(ctx, 3); // row offsets, tails, and the longest row
+        VG_CUDA(cudaMemsetAsync(bad.p, 0, 3 * sizeof(int), ctx->stream));
         // pinned buffers sized to the file (a small file needs no 64 MiB buffers), a
         // multiple of 16 bytes so edge records never straddle two chunks
         const size_t chunk = (size_t)std::min<int64_t>(
@@ -123,6 +123,7 @@ extern "C" vg_status vg_graph_read_vite(vg_ctx *ctx, const char *path, vg_graph 
             for (auto &e : done)
                 if (e) cudaEventDestroy(e);
         };
+        int32_t longest = -1;
         try {
             // reuse of pinned buffer b waits for the copy that last read it
             bool used[2] = {false, false};
@@ -143,7 +144,7 @@ extern "C" vg_status vg_graph_read_vite(vg_ctx *ctx, const char *path, vg_graph 
                                         cudaMemcpyHostToDevice, ctx->stream));
                 VG_CUDA(cudaEventRecord(done[b], ctx->stream));
             }
-            vg_check_rowptr_async(ctx, rp.p, nv + 1, base, ne, bad.p);
+            vg_check_rowptr_async(ctx, rp.p, nv + 1, base, ne, bad.p, bad.p + 2);
             if (base != 0) {
                 LaunchTimer lt(ctx);
                 k_rebase<<<vg_grid(ctx, nv + 1, 256), 256, 0, ctx->stream>>>(rp.p, nv + 1, base);
@@ -171,8 +172,8 @@ extern "C" vg_status vg_graph_read_vite(vg_ctx *ctx, const char *path, vg_graph 
                     VG_CHECK_LAUNCH();
                 }
             }
-            int *hbad = (int *)vg_pinned(ctx, 2 * sizeof(int));
-            VG_CUDA(cudaMemcpyAsync(hbad, bad.p, 2 * sizeof(int), cudaMemcpyDeviceToHost,
+            int *hbad = (int *)vg_pinned(ctx, 3 * sizeof(int));
+            VG_CUDA(cudaMemcpyAsync(hbad, bad.p, 3 * sizeof(int), cudaMemcpyDeviceToHost,
                                     ctx->stream));
             vg_sync(ctx);
             VG_REQUIRE(hbad[0] == 0, "%s: row offsets decrease, hold a row of 2^31 or more entries or "
@@ -180,6 +181,7 @@ extern "C" vg_status vg_graph_read_vite(vg_ctx *ctx, const char *path, vg_graph 
                        (long long)ne);
             VG_REQUIRE(hbad[1] == 0, "%s: an edge tail is outside [0, nv=%lld)", path,
                        (long long)nv);
+            longest = hbad[2];
         } catch (...) {
             cudaStreamSynchronize(ctx->stream); // no copy may still read the pinned buffers
             destroy();
@@ -187,6 +189,7 @@ extern "C" vg_status vg_graph_read_vite(vg_ctx *ctx, const char *path, vg_graph 
         }
         destroy();
         *out = vg_graph_wrap(ctx, nv, ne, rp.detach(), tail.detach(), w.detach());
+        (*out)->longest = longest;
     });
 }
 

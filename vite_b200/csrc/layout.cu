@@ -434,6 +434,7 @@ vg_graph *vg_apply_layout(vg_ctx *ctx, const vg_graph *g, const int32_t *order) 
     h->ref = ref.detach();
     h->pos = pos.detach();
     h->integral = g->integral;
+    h->longest = g->longest;
     return h;
 }
 

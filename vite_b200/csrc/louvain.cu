@@ -2313,6 +2313,8 @@ static bool run_phase_small(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, 
     const int64_t nv = g->nv;
     if (nv == 0 || nv > SP_MAX_NV || g->ne > SP_MAX_NE) return false;
     if (num_color > SP_MAX_COLORS) return false;
+    // a row the launch would refuse, and a wait for it (40-60 us) for nothing
+    if (g->longest > SP_MAX_ROW || std::min<int64_t>(g->longest, nv) > SP_CAP / 2) return false;
     vg_grid_limits(ctx, k_phase_small<false>, k_phase_small<true>, SP_WORK_BYTES, ctx->phase_limits);
     const bool grid = g->ne > VG_SP_CLUSTER_NE;
     const int limit = grid ? ctx->phase_limits.grid : ctx->phase_limits.cluster;
@@ -2936,7 +2938,8 @@ extern "C" vg_status vg_autotune(vg_ctx *ctx, vg_graph *const *graphs, int32_t n
                     throw;
                 }
                 if (tmp.comm) vg_free(ctx, tmp.comm, sizeof(int32_t) * tmp.nv);
-                graphs[i]->integral = tmp.integral; // the cached weight test
+                graphs[i]->integral = tmp.integral; // the cached tests
+                graphs[i]->longest = tmp.longest;
                 total += pt.sweep_ms;
             }
             return total;

@@ -37,7 +37,7 @@ constexpr int SP_CAP = 16384;  // slots of a block's table: rows of up to half a
 constexpr int64_t SP_MAX_ROW = 49152;
 constexpr int SP_UNITS = SEG_CHUNK == 2048 && SEG_THREADS == 256 ? 8 : -1; // warps per chunk
 #ifndef VG_SP_MAX_NV
-#define VG_SP_MAX_NV 524288
+#define VG_SP_MAX_NV VG_ONE_LAUNCH_NV
 #endif
 #ifndef VG_SP_MAX_NE
 #define VG_SP_MAX_NE (1 << 21)

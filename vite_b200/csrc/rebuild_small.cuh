@@ -40,7 +40,7 @@ constexpr int RS_BIG_L = 1024; // segments longer than this go to a whole block
 // 1.08 and 0.96; several reads, 49,000 entries in all 0.50 and 0.53, 71,000 0.56 and 0.50, 124,000
 // 0.70 and 0.47; real weights and one read, where a key's entries are one warp's chain, 24,000
 // entries 0.36 and 0.54, 48,000 0.65 and 0.55, 96,000 1.8 and 0.8, 800,000 14.3 and 3.1.
-__device__ __forceinline__ int64_t rs_max_reads(bool integral, int64_t reads) {
+__host__ __device__ __forceinline__ int64_t rs_max_reads(bool integral, int64_t reads) {
     return reads > 1 ? 49152 : integral ? 131072 : 32768;
 }
 
@@ -55,6 +55,7 @@ static_assert(RS_SMEM_BYTES >= RS_MAX_NV / 8, "the member bitmap must fit");
 struct SmallRebuildOut {
     int64_t nc, m; // rows and entries of the next level
     int32_t status;
+    int32_t longest; // entries of its longest row
 };
 
 struct SmallRebuild {
@@ -79,7 +80,7 @@ struct SmallRebuild {
     int32_t polls;
     SmallRebuildOut *out;
 };
-enum { RS_BIG_ROWS, RS_LONG_SEGS, RS_REFUSED, RS_CTL };
+enum { RS_BIG_ROWS, RS_LONG_SEGS, RS_REFUSED, RS_LONGEST, RS_CTL };
 
 // sum of part[0..n) with stride 3, n <= the block's threads; the whole block calls it
 __device__ __forceinline__ int64_t block_prefix_of(const int64_t *part, int n, int64_t *s_w) {
@@ -361,7 +362,14 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_rebuild_small(SmallRebuild p)
     // the next level's row offsets
     {
         int64_t a = 0, total;
-        for (int64_t r = rlo + tid; r < rhi; r += GS_THREADS) a += __ldcg(p.ucount + r);
+        int32_t most = 0;
+        for (int64_t r = rlo + tid; r < rhi; r += GS_THREADS) {
+            const int64_t u = __ldcg(p.ucount + r);
+            a += u;
+            most = max(most, (int32_t)u);
+        }
+        __syncwarp();
+        vg_raise(p.ctl + RS_LONGEST, most);
         block_excl(a, total, s_w);
         if (tid == 0) p.part[3 * rank + 2] = total;
     }
@@ -378,6 +386,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) k_rebuild_small(SmallRebuild p)
             p.rowptr_out[nc] = run;
             p.out->nc = nc;
             p.out->m = run;
+            p.out->longest = __ldcg(p.ctl + RS_LONGEST);
         }
     }
 }

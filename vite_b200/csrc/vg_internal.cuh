@@ -170,10 +170,21 @@ struct vg_graph {
     // every sum of weights is an exact integer below 2^51 whatever its order;
     // 0: not so; -1: not yet known (vg_weights_integral computes it)
     int8_t integral = -1;
+    // entries of the longest row; -1: not known (looked at up to VG_ONE_LAUNCH_NV vertices)
+    int32_t longest = -1;
 };
 
-// whether g's weights are integral in the sense above (computed once per graph)
+// vertices up to which a phase or a rebuild may run in one launch
+constexpr int64_t VG_ONE_LAUNCH_NV = 524288;
+
+// whether g's weights are integral in the sense above (computed once per graph, with `longest`)
 bool vg_weights_integral(vg_ctx *ctx, vg_graph *g);
+
+// *at becomes at least every thread's x (>= 0); whole warps call it
+__device__ __forceinline__ void vg_raise(int32_t *at, int32_t x) {
+    const int32_t most = __reduce_max_sync(0xffffffffu, x);
+    if ((threadIdx.x & 31) == 0 && most > *(volatile int32_t *)at) atomicMax(at, most);
+}
 
 // reference id of the vertex (or community) at position p
 __device__ __forceinline__ int32_t vg_rid(const int32_t *__restrict__ ref, int32_t p) {
@@ -202,9 +213,9 @@ inline bool vg_auto_layout(vg_ctx *ctx, const vg_graph *g, int mode) {
 
 // stream-ordered check of n1 row offsets (the first one is `base`): sets *bad (device
 // memory) when they decrease, a row holds more than INT32_MAX entries, or the last is
-// not base + ne
+// not base + ne; raises *longest to the longest row's entries
 void vg_check_rowptr_async(vg_ctx *ctx, const int64_t *rp, int64_t n1, int64_t base, int64_t ne,
-                           int *bad);
+                           int *bad, int32_t *longest);
 
 void vg_graph_release(vg_ctx *ctx, vg_graph *g);
 // the graph takes ownership of the three arrays
