@@ -5,6 +5,7 @@ import pytest
 
 from oracle import vite_oracle as vo
 from test_general_path import launches_of
+from test_small_phase import multigraph
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +53,17 @@ def test_known_row_is_not_launched_for(n, rebuilt):
             dev.free()
     assert iters[8192] == iters[8193] == 1  # no gain is enough to go on
     assert count[8193] == count[8192] - 1 and count[8193] > 10
+
+
+def test_short_phase_has_no_iteration_in_vain(ctx):
+    """Below 2^22 entries the loop test moves to the device, with an iteration ahead, only after
+    some iterations: a phase of one takes the launches it takes above."""
+    count = []
+    for pairs in ((1 << 21) - 4000, (1 << 21) + 4000):
+        g = multigraph(400000, pairs, 31, False)
+        dev = ctx.upload(g.rowptr, g.tail, g.weight)
+        (_, _, it), launches = launches_of(ctx, lambda: ctx.louvain_phase(dev, threshold=10.0))
+        assert it == 1
+        count.append(launches)
+        dev.free()
+    assert count[0] == count[1]

@@ -2214,6 +2214,19 @@ static void sweep_hubs(vg_ctx *ctx, const SweepArgs &a, HubPlan &hp, int64_t k,
     VG_CHECK_LAUNCH();
 }
 
+// the rows of a color in the groups of classes that sweep_color launches beside one another
+constexpr int GROUPS = 5;
+static int64_t group_rows(const Buckets &b, int64_t color, int group) {
+    auto count = [&](int cls) { return b.start[color * NCLS + cls + 1] - b.start[color * NCLS + cls]; };
+    return group == 0 ? count(1) + count(2) : group == 1 ? count(0) : group == 2 ? count(5)
+           : group == 3 ? count(4) : count(3);
+}
+static int busy_groups(const Buckets &b, int64_t color) {
+    int busy = 0;
+    for (int k = 0; k < GROUPS; k++) busy += group_rows(b, color, k) > 0;
+    return busy;
+}
+
 // launch the sweep kernels over one color bucket; with `natural` the low-degree
 // class runs over all vertices in id order instead of its list. The classes touch
 // disjoint vertices (reading the community arrays, which no sweep kernel writes, and
@@ -2227,13 +2240,8 @@ static void sweep_color(vg_ctx *ctx, const SweepArgs &a, const Buckets &b, int64
     const int32_t *list = b.list.p + b.start[color * NCLS];
     auto at = [&](int cls) { return b.start[color * NCLS + cls] - b.start[color * NCLS]; };
     auto count = [&](int cls) { return at(cls + 1) - at(cls); };
-    constexpr int GROUPS = 5;
-    auto rows = [&](int group) { // the group's rows
-        return group == 0 ? count(1) + count(2) : group == 1 ? count(0) : group == 2 ? count(5)
-               : group == 3 ? count(4) : count(3);
-    };
-    int busy = 0;
-    for (int k = 0; k < GROUPS; k++) busy += rows(k) > 0;
+    auto rows = [&](int group) { return group_rows(b, color, group); };
+    const int busy = busy_groups(b, color);
     if (busy == 0) return;
     // group 1 takes the main stream, or the first busy one when it has no rows
     const int sides = ctx->profile ? 0 : busy - 1;
@@ -2385,17 +2393,17 @@ static bool run_phase_small(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, 
     return true;
 }
 
-// The iterations of plain phases (bd: their loop tests on the device, J of them in seg) until
-// every one has ended; a: the arrays, without curr and target; bufs: past, curr and target of
-// the first iteration. Two iterations are in flight: the next one is enqueued before the live
+// The iterations of plain phases (bd: their loop tests on the device, J of them in seg) from
+// iteration `first` until every one has ended; a: the arrays, without curr and target; bufs:
+// past, curr and target of iteration 1. Two iterations are in flight: the next one is enqueued before the live
 // count of the one before is waited for, so the device never waits for the host (after the
 // last iteration every graph is done and the extra one's launches return at once). Enqueued
 // directly: capturing a batch's iteration as a graph cost 1.2-1.5 ms a phase, more than its
 // replays saved (48 graphs of 1,000-256,000 vertices: phases 26.5 -> 17.0 ms).
-// sweep_ms (or null) gets the sweeps' time; returns the iterations.
-static int32_t iterate(vg_ctx *ctx, SweepArgs a, BatchDecide bd, int32_t *const (&bufs)[3], const Buckets &bk,
-                       HubPlan &hp, const SegTable &seg, int64_t nv, double *cdeg, int32_t *csize,
-                       double *part, int32_t *noprune, double *sweep_ms) {
+// sweep_ms (or null) gets the sweeps' time; returns the last iteration's number.
+static int32_t iterate(vg_ctx *ctx, SweepArgs a, BatchDecide bd, int32_t *const (&bufs)[3], int32_t first,
+                       const Buckets &bk, HubPlan &hp, const SegTable &seg, int64_t nv, double *cdeg,
+                       int32_t *csize, double *part, int32_t *noprune, double *sweep_ms) {
     const int agrid = seg_grid(ctx, seg.C);
     int32_t *hlive = (int32_t *)vg_pinned(ctx, 2 * sizeof(int32_t));
     int32_t *live = bd.live_count; // 2
@@ -2440,11 +2448,11 @@ static int32_t iterate(vg_ctx *ctx, SweepArgs a, BatchDecide bd, int32_t *const 
         VG_CUDA(cudaEventCreateWithFlags(&ev.e[k], k < 2 || !sweep_ms ? cudaEventDisableTiming
                                                                       : cudaEventDefault));
     if (sweep_ms) *sweep_ms = 0.0;
-    for (int32_t it = 1;; it++) {
+    for (int32_t it = first;; it++) {
         const int slot = it & 1, pi = (it - 1) % 3; // past <- curr <- target <- past (louvain.cpp:565-570)
         enqueue(pi, it, slot, sweep_ms ? ev.e[2 + slot] : nullptr, sweep_ms ? ev.e[4 + slot] : nullptr);
         VG_CUDA(cudaEventRecord(ev.e[slot], ctx->stream));
-        if (it == 1) continue;
+        if (it == first) continue;
         const int before = slot ^ 1;
         VG_CUDA(cudaEventSynchronize(ev.e[before]));
         if (sweep_ms) {
@@ -2457,6 +2465,7 @@ static int32_t iterate(vg_ctx *ctx, SweepArgs a, BatchDecide bd, int32_t *const 
 }
 
 constexpr int64_t AHEAD_MAX_NE = 1 << 22;
+constexpr int AHEAD_AFTER = 8;
 
 // the phase proper; returns the communities in g->comm
 // max_iters > 0 stops after that many iterations (the autotuner's timing runs)
@@ -2541,60 +2550,18 @@ static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double
     DevBuf<double> modv(ctx, 4);
     double *hmod = (double *)vg_pinned(ctx, 4 * sizeof(double));
 
-    // Plain phases of middling graphs: the loop test on the device, iterations enqueued ahead
-    // (300,007 vertices / 2.8e6 entries, 20 iterations: 1.46 -> 1.24 ms). Larger ones lose
-    // more by every block's look at the flag than the host's gaps cost (348,203 / 6.5e6:
-    // 1.41 -> 1.56 ms; 12,071 / 4.4e6: 0.86 -> 0.89).
-    if (ordering == 0 && et == 0 && max_iters == 0 && nv && g->ne <= AHEAD_MAX_NE) {
-        struct State { // of the loop test, one 8-byte word each
-            double prev_mod, lower, thresh;
-            int64_t iters, live, done, resbuf;
-        };
-        State h{p->lower, p->lower, p->threshold, 0, 0, 0, 0};
-        // past the words `iterate` reads back
-        State *staged = reinterpret_cast<State *>((char *)vg_pinned(ctx, 64 + sizeof(State)) + 64);
-        *staged = h;
-        DevBuf<State> st(ctx, 1);
-        VG_CUDA(cudaMemcpyAsync(st.p, staged, sizeof(State), cudaMemcpyHostToDevice, ctx->stream));
-        SweepArgs a{};
-        a.rowptr = g->rowptr;
-        a.tail = g->tail;
-        a.weight = g->weight;
-        a.vdeg = vdeg.p;
-        a.cdeg = cdeg.p;
-        a.csize = csize.p;
-        a.cupd = cupd.p;
-        a.cw = cw.p;
-        a.ref = g->ref;
-        a.noprune = noprune.p;
-        a.ne = g->ne;
-        a.constant = constant;
-        BatchDecide bd{};
-        bd.prev_mod = &st.p->prev_mod;
-        bd.lower = &st.p->lower;
-        bd.thresh = &st.p->thresh;
-        bd.iters = reinterpret_cast<int32_t *>(&st.p->iters);
-        bd.live_count = reinterpret_cast<int32_t *>(&st.p->live); // two of them
-        bd.done = reinterpret_cast<uint8_t *>(&st.p->done);
-        bd.resbuf = reinterpret_cast<int8_t *>(&st.p->resbuf);
-        a.stop = bd.done;
-        int32_t *bufs[3] = {A.p, B.p, C.p};
-        double ms = 0.0;
-        const int32_t its = iterate(ctx, a, bd, bufs, bk, hp, seg, nv, cdeg.p, csize.p, part.p,
-                                    noprune.p, timing ? &ms : nullptr);
-        VG_CUDA(cudaMemcpyAsync(staged, st.p, sizeof(State), cudaMemcpyDeviceToHost, ctx->stream));
-        vg_sync(ctx);
-        if (timing) {
-            timing->sweep_ms = ms;
-            timing->edges = g->ne * its;
-        }
-        *mod_out = staged->prev_mod;
-        *iters_out = its;
-        vg_free(ctx, g->comm, sizeof(int32_t) * nv);
-        DevBuf<int32_t> *held[3] = {&A, &B, &C};
-        g->comm = held[*reinterpret_cast<const int8_t *>(&staged->resbuf)]->detach();
-        return;
-    }
+    // Plain phases of middling graphs: the loop test on the device, iterations enqueued ahead. That
+    // costs an iteration in vain and some copies, 50 us in all, and saves the host's gap in each
+    // iteration, so it pays after about eight; where three or more groups of classes run beside
+    // one another an iteration is a dozen launches, whose gap is larger, and graphs stored in the
+    // locality layout take 15 to 20 iterations: from the first one there. By the host's test and so
+    // (vertices / entries, iterations): ER 150,000 / 2.4e6, 3, 0.37 and 0.42 ms, 6, 0.54 and 0.61;
+    // RGG 250,000 / 2.3e6, 20, 1.45 and 1.23; laid out 300,007 / 2.8e6, 18, 1.21 and 1.04; BA 250,000
+    // / 4.0e6, 6, 1.29 and 1.21. Larger graphs lose more by every block's look at the flag
+    // (348,203 / 6.5e6: 1.41 -> 1.56 ms; 12,071 / 4.4e6: 0.86 -> 0.89).
+    int ahead_after = INT_MAX;
+    if (ordering == 0 && et == 0 && max_iters == 0 && nv && g->ne <= AHEAD_MAX_NE)
+        ahead_after = g->ref || busy_groups(bk, 0) >= 3 ? 0 : AHEAD_AFTER;
 
     DevBuf<uint8_t> touched; // communities the current color's sweep moves vertices in or out of
     if (ordering == 1 && nv && touched.try_alloc(ctx, (nv + 15) / 16 * 16))
@@ -2610,13 +2577,10 @@ static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double
         VG_CUDA(cudaEventCreate(&ev1));
     }
     for (;;) {
-        numIters++;
         SweepArgs a{};
         a.rowptr = g->rowptr;
         a.tail = g->tail;
         a.weight = g->weight;
-        a.curr = curr;
-        a.target = target;
         a.vdeg = vdeg.p;
         a.cdeg = cdeg.p;
         a.csize = csize.p;
@@ -2627,9 +2591,46 @@ static void run_phase(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, double
         a.ref = g->ref;
         a.noprune = noprune.p;
         a.ne = g->ne;
-        a.ident = numIters == 1 ? 1 : 0; // k_init put every vertex in its own community
         a.touched = touched.p;
         a.constant = constant;
+        if (numIters == ahead_after) {
+            struct State { // of the loop test, one 8-byte word each
+                double prev_mod, lower, thresh;
+                int64_t iters, live, done, resbuf;
+            };
+            // past the words `iterate` reads back
+            State *staged = reinterpret_cast<State *>((char *)vg_pinned(ctx, 64 + sizeof(State)) + 64);
+            *staged = State{prevMod, lower, p->threshold, 0, 0, 0, 0};
+            DevBuf<State> st(ctx, 1);
+            VG_CUDA(cudaMemcpyAsync(st.p, staged, sizeof(State), cudaMemcpyHostToDevice, ctx->stream));
+            BatchDecide bd{};
+            bd.prev_mod = &st.p->prev_mod;
+            bd.lower = &st.p->lower;
+            bd.thresh = &st.p->thresh;
+            bd.iters = reinterpret_cast<int32_t *>(&st.p->iters);
+            bd.live_count = reinterpret_cast<int32_t *>(&st.p->live); // two of them
+            bd.done = reinterpret_cast<uint8_t *>(&st.p->done);
+            bd.resbuf = reinterpret_cast<int8_t *>(&st.p->resbuf);
+            a.stop = bd.done;
+            int32_t *bufs[3] = {A.p, B.p, C.p};
+            double ms = 0.0;
+            const int32_t its = iterate(ctx, a, bd, bufs, numIters + 1, bk, hp, seg, nv, cdeg.p,
+                                        csize.p, part.p, noprune.p, timing ? &ms : nullptr);
+            VG_CUDA(cudaMemcpyAsync(staged, st.p, sizeof(State), cudaMemcpyDeviceToHost, ctx->stream));
+            vg_sync(ctx);
+            if (timing) {
+                timing->sweep_ms += ms;
+                timing->edges += g->ne * (its - numIters);
+            }
+            numIters = its;
+            prevMod = staged->prev_mod;
+            past = bufs[*reinterpret_cast<const int8_t *>(&staged->resbuf)];
+            break;
+        }
+        numIters++;
+        a.curr = curr;
+        a.target = target;
+        a.ident = numIters == 1 ? 1 : 0; // k_init put every vertex in its own community
         if (timing) VG_CUDA(cudaEventRecord(ev0, ctx->stream));
         for (int64_t ci = 0; ci < numColor; ci++) {
             sweep_color(ctx, a, bk, ci, hp, ordering == 0, nv);
@@ -2820,7 +2821,7 @@ void vg_phase_batch_internal(vg_ctx *ctx, vg_graph *U, int64_t J, const int64_t 
     bd.resbuf = resbuf.p;
     bd.live_count = live.p;
     int32_t *bufs[3] = {B0.p, B1.p, B2.p};
-    iterate(ctx, a, bd, bufs, bk, hp, seg, nv, cdeg.p, csize.p, part.p, noprune.p, sweep_ms);
+    iterate(ctx, a, bd, bufs, 1, bk, hp, seg, nv, cdeg.p, csize.p, part.p, noprune.p, sweep_ms);
     vg_sync(ctx);
     vg_free(ctx, U->comm, sizeof(int32_t) * nv);
     U->comm = nullptr;
