@@ -9,6 +9,7 @@ taken over."""
 import numpy as np
 import pytest
 
+from conftest import multi_hub_csr
 from oracle import vite_oracle as vo
 from test_gpu_parity import assert_graph_equal
 from test_small_phase import multigraph
@@ -86,6 +87,15 @@ def test_phase_with_hubs(ctx, et):
 @pytest.mark.parametrize("et", [0, 2])
 def test_phase_with_hubs_real_weights(ctx, et):
     check_phase(ctx, classes_graph(30000, 2, True), True, et_type=et, et_delta=0.25)
+
+
+@pytest.mark.parametrize("real", [False, True])
+@pytest.mark.parametrize("ordering,et", [(0, 0), (0, 2), (1, 0), (1, 2)])
+def test_phase_with_hubs_and_short_rows(ctx, ordering, et, real):
+    """No rows of middle length: the hubs' kernels are launched before the others'."""
+    g = vo.Graph(*multi_hub_csr(40000, 6, 9000, 21, real))
+    colors = some_colors(g.nv, 7) if ordering else None
+    check_phase(ctx, g, real, colors, 4, et_type=et, et_delta=0.25, ordering=ordering)
 
 
 @pytest.mark.parametrize("ordering", [1, 2])
