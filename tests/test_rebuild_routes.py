@@ -53,3 +53,19 @@ def test_long_segment_of_real_weights_is_sorted(ctx, members, sorted_path):
         assert_graph_equal(dev.download(), vo.rebuild(g, cv))
         dev.free()
     assert (count[True] > count[False] + 10) == sorted_path
+
+
+@pytest.mark.parametrize("n,m,one", [(3000, 40000, True), (140000, 300000, False)])
+def test_negative_zeros_stay(ctx, n, m, one):
+    """Integral weights that are -0.0: a sum of nothing else is -0.0, in a block's table too."""
+    g = multigraph(n, m, 5, False)
+    w = np.where(g.tail % 7 == 0, 2.0, np.where(g.tail % 3 == 0, 0.0, -0.0))
+    g = vo.Graph(g.rowptr, g.tail, w)
+    cv = one_long(n, n // 20, 1500)
+    dev = ctx.upload(g.rowptr, g.tail, g.weight)
+    ctx.vertex_degree(dev)
+    _, launches = launches_of(ctx, lambda: ctx.rebuild(dev, cv))
+    assert (launches <= 10) == one
+    ref = vo.rebuild(g, cv)
+    assert np.signbit(ref.weight).any() and np.diff(ref.rowptr).max() > 256
+    assert_graph_equal(dev.download(), ref)

@@ -498,7 +498,7 @@ __device__ __forceinline__ int block_segment(Table &T, int64_t s0, int64_t L, bo
     __syncthreads(); // the table of the segment before
     for (int i = tid; i <= (int)mask; i += NT) {
         T.keys[i] = H_EMPTY;
-        T.vals[i] = 0.0;
+        T.vals[i] = -0.0; // adds nothing to any weight, -0.0 included
     }
     if (tid == 0) T.used = 0;
     __syncthreads();
