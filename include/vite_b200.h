@@ -111,6 +111,12 @@ vg_status vg_ctx_reserve(vg_ctx *ctx, size_t bytes);
  * (default 2^23, some seconds) gives up; the launch then ends without a result and the step is
  * done again by a launch per step. At least 1, else VG_ERR_ARG. */
 vg_status vg_ctx_set_barrier_polls(vg_ctx *ctx, int32_t polls);
+/* Iterations after which the one launch of a small graph's phase ends without a result and the
+ * phase is done again by a launch per step (default 16,384; no reference counterpart). A phase
+ * ends when an iteration gains less than its threshold, which with a threshold of zero or less,
+ * or with weights whose squares overflow, may be never: the host can be interrupted in such a
+ * phase, a launch cannot. At least 1, else VG_ERR_ARG. */
+vg_status vg_ctx_set_phase_iterations(vg_ctx *ctx, int32_t iterations);
 /* The CUDA stream (cudaStream_t) all of the context's work runs on, so callers
  * can time it with events or order their own work after it. */
 vg_status vg_ctx_stream(vg_ctx *ctx, void **stream_out);

@@ -31,6 +31,7 @@ _STATUS_NAMES = {0: "VG_OK", 1: "VG_ERR_ARG", 2: "VG_ERR_OOM", 3: "VG_ERR_CUDA",
 EXPORTED_SYMBOLS = [
     "vg_ctx_create", "vg_ctx_destroy", "vg_last_error", "vg_ctx_bytes_in_use", "vg_ctx_profile",
     "vg_ctx_stream", "vg_ctx_reserve", "vg_ctx_set_barrier_polls",
+    "vg_ctx_set_phase_iterations",
     "vg_graph_upload", "vg_graph_info", "vg_graph_download", "vg_graph_free", "vg_vertex_degree",
     "vg_louvain_phase", "vg_color", "vg_set_colors", "vg_rebuild", "vg_louvain_run",
     "vg_generate_rgg", "vg_generate_ba", "vg_generate_er", "vg_graph_reweight",
@@ -140,6 +141,7 @@ def lib() -> C.CDLL:
         L.vg_ctx_stream.argtypes = [vp, C.POINTER(vp)]
         L.vg_ctx_reserve.argtypes = [vp, C.c_size_t]
         L.vg_ctx_set_barrier_polls.argtypes = [vp, C.c_int32]
+        L.vg_ctx_set_phase_iterations.argtypes = [vp, C.c_int32]
         L.vg_graph_upload.argtypes = [vp, C.c_int64, C.c_int64, _i64p, vp, C.POINTER(vp)]
         L.vg_graph_info.argtypes = [vp, _i64p, _i64p]
         L.vg_graph_download.argtypes = [vp, vp, _i64p, vp]
@@ -296,6 +298,11 @@ class Context:
         """Reads after which a wait inside a one-launch step of a small graph gives up and
         the step is done again by a launch per step (vg_ctx_set_barrier_polls)."""
         self._check(lib().vg_ctx_set_barrier_polls(self.handle, polls))
+
+    def set_phase_iterations(self, iterations: int) -> None:
+        """Iterations after which a one-launch phase of a small graph ends without a result and
+        is done again by a launch per step (vg_ctx_set_phase_iterations)."""
+        self._check(lib().vg_ctx_set_phase_iterations(self.handle, iterations))
 
     @property
     def stream(self) -> int:

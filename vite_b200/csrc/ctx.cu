@@ -195,6 +195,14 @@ extern "C" vg_status vg_ctx_set_barrier_polls(vg_ctx *ctx, int32_t polls) {
     });
 }
 
+extern "C" vg_status vg_ctx_set_phase_iterations(vg_ctx *ctx, int32_t iterations) {
+    if (!ctx) return VG_ERR_ARG;
+    return vg_guard(ctx, [&] {
+        VG_REQUIRE(iterations >= 1, "a phase needs at least one iteration (got %d)", iterations);
+        ctx->phase_iterations = iterations;
+    });
+}
+
 extern "C" vg_status vg_ctx_stream(vg_ctx *ctx, void **stream_out) {
     if (!ctx || !stream_out) return VG_ERR_ARG;
     *stream_out = (void *)ctx->stream;

@@ -12,9 +12,10 @@ constexpr int GS_MAX_CLUSTER = 16;
 enum : int32_t {
     GS_DONE = 0,
     GS_REFUSED = 1, // not a graph the kernel takes
-    GS_TIMEOUT = 2  // a barrier's bounded wait ran out
+    GS_TIMEOUT = 2, // a barrier's bounded wait ran out
+    GS_ENDLESS = 3  // a phase took more iterations than a launch may (vg_ctx_set_phase_iterations)
 };
-// GS_REFUSED and GS_TIMEOUT leave the graph as it was, and the general path takes it.
+// All but GS_DONE leave the graph as it was, and the general path takes it.
 
 // All blocks of the launch reach the barrier, and what they wrote before it is visible
 // after it. GRID: a counter in global memory that starts at 0 (the launch is cooperative,

@@ -2389,6 +2389,7 @@ static bool run_phase_small(vg_ctx *ctx, vg_graph *g, const vg_phase_params *p, 
     out->status = GS_DONE;
     sp.out = out;
     sp.polls = ctx->barrier_polls;
+    sp.max_iters = ctx->phase_iterations;
     vg_grid_launch(ctx, grid ? k_phase_small<true> : k_phase_small<false>, sp, grid, blocks,
                    SP_WORK_BYTES, sp.arrived);
     vg_sync(ctx);

@@ -92,6 +92,7 @@ struct SmallPhase {
     int32_t ncolors;       // uncolored (-1) vertices go with the last one
     unsigned *arrived; // (GRID) blocks that reached the grid's barriers so far (starts at 0)
     int32_t polls;     // of one wait there
+    int32_t max_iters; // then the launch ends with GS_ENDLESS
     SmallOut *out;
 };
 
@@ -371,6 +372,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) k_phase_small(SmallPhase p) {
     double prev = p.lower, sweep_ns = 0.0;
     int iters = 0;
     for (;;) {
+        if (iters == p.max_iters) { // the same in every block
+            if (rank == 0 && tid == 0) p.out->status = GS_ENDLESS;
+            return;
+        }
         iters++;
         int32_t *past = p.buf[ip], *curr = p.buf[(ip + 1) % 3], *target = p.buf[(ip + 2) % 3];
         a.curr = curr;

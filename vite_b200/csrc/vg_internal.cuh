@@ -75,6 +75,7 @@ struct vg_ctx {
     // which a wait at their barriers gives up (vg_ctx_set_barrier_polls)
     GridLimits phase_limits, rebuild_limits;
     int32_t barrier_polls = 1 << 23;
+    int32_t phase_iterations = 1 << 14; // of a one-launch phase
 };
 
 // the context's side streams: work enqueued on the first n of them between vg_side_fork and
