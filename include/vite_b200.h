@@ -91,7 +91,9 @@ typedef struct vg_level_stat {
 
 /* Create a context on `device` with a device-memory budget in bytes (0 = no
  * budget beyond the device's capacity). Replaces MPI_Init/communicator set-up
- * (main.cpp:112-118). */
+ * (main.cpp:112-118). The context's own streams have the device's highest priority (three of
+ * its side streams the lowest), so that a sweep's largest kernels start first: the blocks of
+ * work that a program puts on streams of default priority wait for them. */
 vg_status vg_ctx_create(int device, size_t mem_budget_bytes, vg_ctx **out);
 vg_status vg_ctx_destroy(vg_ctx *ctx);
 const char *vg_last_error(const vg_ctx *ctx);

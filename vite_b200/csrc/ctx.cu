@@ -120,8 +120,8 @@ extern "C" vg_status vg_ctx_create(int device, size_t mem_budget_bytes, vg_ctx *
         int least = 0, most = 0;
         VG_CUDA(cudaDeviceGetStreamPriorityRange(&least, &most));
         VG_CUDA(cudaStreamCreateWithPriority(&ctx->stream, cudaStreamNonBlocking, most));
-        // the side streams and their fork/join events exist from the start, so that a
-        // fork inside a stream capture creates nothing
+        // the side streams and their fork/join events exist from the start: a sweep forks in
+        // every iteration
         for (int k = 0; k < VG_SIDE; k++)
             VG_CUDA(cudaStreamCreateWithPriority(&ctx->side[k], cudaStreamNonBlocking,
                                                  k == 0 ? most : least));
