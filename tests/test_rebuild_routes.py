@@ -69,3 +69,20 @@ def test_negative_zeros_stay(ctx, n, m, one):
     ref = vo.rebuild(g, cv)
     assert np.signbit(ref.weight).any() and np.diff(ref.rowptr).max() > 256
     assert_graph_equal(dev.download(), ref)
+
+
+def test_integral_weights_are_known_after_a_phase(ctx):
+    """A phase in one launch does not look whether the weights are integral; the rebuild by launches
+    does, and keeps a segment of 60,000 integral entries out of the sorted path."""
+    n = 10000
+    cv = one_long(n, 5000, 1000)
+    count = {}
+    for real in (False, True):
+        g = multigraph(n, 60000, 37, real)
+        dev = ctx.upload(g.rowptr, g.tail, g.weight)
+        _, launches = launches_of(ctx, lambda: ctx.louvain_phase(dev))
+        assert launches <= 10
+        _, count[real] = launches_of(ctx, lambda: ctx.rebuild(dev, cv))
+        assert_graph_equal(dev.download(), vo.rebuild(g, cv))
+        dev.free()
+    assert 10 < count[False] < count[True] - 10

@@ -158,6 +158,8 @@ vg_graph *vg_rebuild_new(vg_ctx *ctx, const vg_graph *g, const int32_t *comm) {
         h->integral = g->integral; // sums of the same integers; else the in-order folds serve any weights
         return h;
     }
+    // a phase in one launch leaves it open, and integral weights have the faster folds
+    vg_weights_integral(ctx, const_cast<vg_graph *>(g));
     const int grid = vg_grid(ctx, nv, 256);
     if (!g->ref) {
         // reference layout: first appearance by position is first appearance by id
