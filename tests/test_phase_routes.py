@@ -43,11 +43,13 @@ def test_known_row_is_not_launched_for(n, rebuilt):
     count, iters = {}, {}
     with vite_b200.Context(0) as c:
         for entries in (8192, 8193):
+            c.set_barrier_polls(1 << 23)
             g = hub_graph(n, n // 2, entries)
             dev = c.upload(g.rowptr, g.tail, g.weight)
             if rebuilt:  # every vertex alone: equal pairs become one
                 c.rebuild(dev, np.arange(n))
-            c.set_barrier_polls(1 if entries == 8192 else 1 << 23)
+            if entries == 8192:
+                c.set_barrier_polls(1)
             (_, _, iters[entries]), count[entries] = launches_of(
                 c, lambda: c.louvain_phase(dev, threshold=10.0))
             dev.free()
